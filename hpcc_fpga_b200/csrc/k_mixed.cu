@@ -310,8 +310,9 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
         LP_CUDA(cudaGetLastError());
     }
     const TriInverses inv{winv, vinv, vlt};
+    float* dinv = block_inv(c, K * bs);
     int e = prof_begin(c, s);
-    LP_CHECK(lu_stage(c, d, lda, bs, s, beside ? &inv : nullptr));
+    LP_CHECK(lu_stage(c, d, lda, bs, dinv, s, beside ? &inv : nullptr));
     LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * b * b * b / 3.0, 8.0 * b * b));
     if (rest <= 0) return LP_OK;
     const double r = rest;
@@ -327,12 +328,18 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
         k_eye2<<<(int)((bb + 255) / 256 < 1184 ? (bb + 255) / 256 : 1184), 256, 0, s>>>(winv, vinv, bs);
         count_launch();
         LP_CUDA(cudaGetLastError());
-        LP_CUDA(cudaEventRecord(c->ev_side, s));
-        LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
-        LP_CHECK(left_blocked(d, lda, vinv, bs, bs, bs, vlt, bs, c->aux2, true));
-        LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
-        LP_CHECK(top_blocked(c, d, lda, winv, bs, bs, bs, s, true));
-        LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
+        if (bs <= 512) {
+            LP_CHECK(launch_tl(d, lda, dinv, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt,
+                               bs, c->num_sms, s));
+        } else {
+            LP_CUDA(cudaEventRecord(c->ev_side, s));
+            LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+            for (int kk = 0; kk < bs / 128; kk++)
+                LP_CHECK(left_chunk_step(c, d, lda, dinv, vinv, bs, vlt, kk, c->aux2));
+            LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
+            for (int kk = 0; kk < bs / 128; kk++) LP_CHECK(top_chunk_step(c, d, lda, dinv, winv, bs, kk, s));
+            LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
+        }
     }
     k_add_diag<<<(bs + 127) / 128, 128, 0, s>>>(vinv, bs, -1.0f);
     count_launch();
@@ -359,10 +366,7 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
     const int kq = x6 ? 6 * bs : bs;  // K of the tensor-core update
     const size_t pan = (size_t)kq * n;      // one tensor-core operand
     const int nblk = (n + 511) / 512;
-    if (bs > 128) {
-        LP_CHECK(c->lti.ensure(2 * sizeof(float) * (size_t)128 * bs));
-        LP_CHECK(c->dsub.ensure(2 * sizeof(float) * (size_t)128 * bs));
-    }
+    LP_CHECK(panel_ensure(c, n, bs));
     LP_CHECK(c->q.ensure(4 * esz * pan));
     LP_CHECK(c->qs.ensure(2 * 6 * sizeof(float) * (size_t)kseg(bs) * nblk));
     LP_CHECK(c->err.ensure(sizeof(int)));

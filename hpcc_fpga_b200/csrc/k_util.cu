@@ -1,5 +1,5 @@
 // Tiled transpose: the diagonal block's sub-blocks into the k-major operand
-// layout of the blocked top stage.
+// layout of the blocked top stage (FP64).
 #include "lp_common.cuh"
 
 namespace lp {
@@ -27,16 +27,6 @@ __global__ void __launch_bounds__(256) k_transpose(const T* __restrict__ src, in
 }
 
 }  // namespace
-
-int launch_transpose(const float* src, int lds, float* dst, int ldd, int rows, int cols, cudaStream_t st) {
-    if (rows <= 0 || cols <= 0) return LP_OK;
-    const dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-    if (grid.y > 65535) return fail(LP_E_INVALID, "transpose: too many rows");
-    k_transpose<float><<<grid, 256, 0, st>>>(src, lds, dst, ldd, rows, cols);
-    count_launch();
-    LP_CUDA(cudaGetLastError());
-    return LP_OK;
-}
 
 int launch_transpose_f64(const double* src, int lds, double* dst, int ldd, int rows, int cols, cudaStream_t st) {
     if (rows <= 0 || cols <= 0) return LP_OK;

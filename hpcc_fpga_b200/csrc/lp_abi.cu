@@ -127,40 +127,55 @@ static double trsm_flops(double b, double w) { return b * b * w; }
 static double inner_flops(double m, double n, double k) { return 2.0 * m * n * k; }
 static double inner_bytes(double m, double n, double k) { return 4.0 * (2.0 * m * n + k * (m + n)); }
 
-// lu stage of one diagonal block.  bs <= 128: one shared-memory kernel.
-// Larger blocks are factored as the same blocked algorithm with 128-wide
-// inner blocks (lu, top, left, inner on the bs x bs sub-matrix), which keeps
-// every piece on the kernels above and spreads the inner work over the GPU.
-int lu_stage(lp_ctx* c, float* d, int lda, int bs, cudaStream_t st, const TriInverses* inv) {
-    if (bs <= 128) return launch_lu_small(d, lda, bs, st);
-    const int ib = 128;
-    float* lti = static_cast<float*>(c->lti.ptr);
-    for (int kk = 0; kk < bs / ib; kk++) {
-        float* dd = d + (size_t)kk * ib * lda + (size_t)kk * ib;
-        LP_CHECK(launch_lu_small(dd, lda, ib, st));
-        const int r = bs - (kk + 1) * ib;
+// Ragged end of a matrix whose order is no multiple of 128: the last m x m
+// block (m < 128, a multiple of 16), in pieces of 64, 32 and 16 with the
+// stage kernels; nothing beside it is left to update.  lt: scratch.
+static int lu_tail(float* d, int lda, int m, float* lt, cudaStream_t st) {
+    while (m > 0) {
+        const int ib = m >= 64 ? 64 : (m >= 32 ? 32 : 16), r = m - ib;
+        LP_CHECK(launch_lu_small(d, lda, ib, st));
         if (r > 0) {
-            // top on st, left beside it on aux2 (both read only the factored block)
-            LP_CUDA(cudaEventRecord(c->ev_side, st));
-            LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
-            LP_CHECK(launch_trsm_top(dd, lda, dd + ib, lda, ib, r, st));
-            LP_CHECK(launch_trsm_left(dd, lda, dd + (size_t)ib * lda, lda, ib, r, lti, r, c->aux2));
-            LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
-            LP_CUDA(cudaStreamWaitEvent(st, c->ev_side_done, 0));
+            LP_CHECK(launch_trsm_top(d, lda, d + ib, lda, ib, r, st));
+            LP_CHECK(launch_trsm_left(d, lda, d + (size_t)ib * lda, lda, ib, r, lt, r, st));
+            LP_CHECK(launch_sgemm_update(d + (size_t)ib * lda + ib, lda, lt, r, d + ib, lda, r, r, ib, st));
         }
-        if (inv != nullptr) {
+        d += (size_t)ib * lda + ib;
+        m = r;
+    }
+    return LP_OK;
+}
+
+// lu stage of one diagonal block of any size (a multiple of 16): blocked with
+// 128-wide inner blocks.  Per inner block a chain of three launches: its LU
+// (one CTA), top and left beside it (one launch, k_panel.cu) and the rank-128
+// update of what follows.  inv: the inner blocks' 32 x 32 inverses, and dt
+// (bs x bs): the block's lower triangle transposed; both serve the top / left
+// updates with this block.
+int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, const TriInverses* tri) {
+    float* dt = static_cast<float*>(c->dt.ptr);
+    for (int k0 = 0, kk = 0; k0 < bs; k0 += 128, kk++) {
+        float* dd = d + (size_t)k0 * lda + k0;
+        float* tt = dt + (size_t)k0 * bs + k0;
+        const int ib = std::min(128, bs - k0), r = bs - k0 - ib;
+        if (ib < 128) return lu_tail(dd, lda, ib, dt, st);
+        float* vv = inv + (size_t)kk * kInvFloats;
+        LP_CHECK(launch_lu128(dd, lda, vv, tt, bs, st));
+        LP_CHECK(launch_tl(dd, lda, vv, tt, bs, ib, dd + ib, lda, r, dd + (size_t)ib * lda, lda, r, tt + ib, bs,
+                           c->num_sms, st));
+        if (tri != nullptr) {
             // block row and column kk of d are final (the trailing update below
             // touches only rows and columns after them): chunk kk of the two
             // identity recurrences, which read nothing else of d
             LP_CUDA(cudaEventRecord(c->ev_inv[kk], st));
             LP_CUDA(cudaStreamWaitEvent(c->inv_top, c->ev_inv[kk], 0));
             LP_CUDA(cudaStreamWaitEvent(c->inv_left, c->ev_inv[kk], 0));
-            LP_CHECK(top_chunk_step(c, d, lda, inv->winv, bs, bs, bs, kk, c->inv_top, true));
-            LP_CHECK(left_chunk_step(d, lda, inv->vinv, bs, bs, bs, inv->vlt, bs, kk, c->inv_left, true));
+            LP_CHECK(top_chunk_step(c, d, lda, inv, tri->winv, bs, kk, c->inv_top));
+            LP_CHECK(left_chunk_step(c, d, lda, inv, tri->vinv, bs, tri->vlt, kk, c->inv_left));
         }
-        if (r > 0) LP_CHECK(launch_sgemm_update(dd + (size_t)ib * lda + ib, lda, lti, r, dd + ib, lda, r, r, ib, st));
+        if (r > 0)
+            LP_CHECK(launch_sgemm_update(dd + (size_t)ib * lda + ib, lda, tt + ib, bs, dd + ib, lda, r, r, ib, st));
     }
-    if (inv != nullptr) {
+    if (tri != nullptr) {
         LP_CUDA(cudaEventRecord(c->ev_inv_top, c->inv_top));
         LP_CUDA(cudaEventRecord(c->ev_inv_left, c->inv_left));
         LP_CUDA(cudaStreamWaitEvent(st, c->ev_inv_top, 0));
@@ -169,91 +184,75 @@ int lu_stage(lp_ctx* c, float* d, int lda, int bs, cudaStream_t st, const TriInv
     return LP_OK;
 }
 
-// top stage for a whole block row: T (bs x ncols) <- top recurrence with the
-// factored diagonal block d.  bs <= 128: one exact-recurrence launch.  Larger
-// blocks walk 128-row diagonal chunks: exact recurrence on the chunk's rows
-// (full width, every column strip in parallel), then the chunk's
+// Chunk kk (128 rows) of the top recurrence applied to the bs x bs identity t
+// (leading dimension bs): the recurrence on the chunk's rows, then the chunk's
 // contribution to the rows below as one GEMM, T[below] += D[below][chunk] *
-// T[chunk] (D's sub-block transposed into the k-major operand first).
-// unit (T0 = identity): column j stays zero above row j, so chunk kk only
-// touches columns below (kk + 1) * 128; the skipped entries are exact zeros.
-int top_chunk_step(lp_ctx* c, const float* d, int lda, float* t, int ldt, int bs, int ncols, int kk, cudaStream_t st,
-                   bool unit) {
+// T[chunk].  Column j stays zero above row j, so chunk kk only touches columns
+// below (kk + 1) * 128; the skipped entries are exact zeros.
+int top_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* t, int bs, int kk, cudaStream_t st) {
     const int ib = 128;
-    float* dt = static_cast<float*>(c->dsub.ptr) + (st == c->aux ? (size_t)ib * bs : 0);
+    const float* dt = static_cast<const float*>(c->dt.ptr) + (size_t)kk * ib * bs + (size_t)kk * ib;
     const float* dkk = d + (size_t)kk * ib * lda + (size_t)kk * ib;
-    float* tk = t + (size_t)kk * ib * ldt;
-    const int cols = unit ? std::min(ncols, (kk + 1) * ib) : ncols;
-    LP_CHECK(launch_trsm_top(dkk, lda, tk, ldt, ib, cols, st));
+    float* tk = t + (size_t)kk * ib * bs;
+    const int cols = (kk + 1) * ib;
+    LP_CHECK(launch_tl(dkk, lda, inv + (size_t)kk * kInvFloats, dt, bs, ib, tk, bs, cols, nullptr, 4, 0, nullptr, 4,
+                       c->num_sms, st));
     const int m2 = bs - (kk + 1) * ib;
     if (m2 <= 0) return LP_OK;
-    LP_CHECK(launch_transpose(dkk + (size_t)ib * lda, lda, dt, m2, m2, ib, st));
-    return launch_sgemm_update(tk + (size_t)ib * ldt, ldt, dt, m2, tk, ldt, m2, cols, ib, st);
+    return launch_sgemm_update(tk + (size_t)ib * bs, bs, dt + ib, bs, tk, bs, m2, cols, ib, st);
 }
 
-int top_blocked(lp_ctx* c, const float* d, int lda, float* t, int ldt, int bs, int ncols, cudaStream_t st,
-                bool unit) {
-    if (bs <= 128) return launch_trsm_top(d, lda, t, ldt, bs, ncols, st);
-    for (int kk = 0; kk < bs / 128; kk++) LP_CHECK(top_chunk_step(c, d, lda, t, ldt, bs, ncols, kk, st, unit));
-    return LP_OK;
-}
-
-// left stage for a whole block column: L (nrows x bs) <- left recurrence with
-// d, and Lt = L^T.  Larger blocks walk 128-column chunks: exact recurrence on
-// the chunk's columns (which also writes the chunk's rows of Lt), then
-// L[:, after] += L[:, chunk] * D[chunk][after] as one GEMM.
-// unit (L0 = identity): row i stays zero left of column i, so chunk kk only
-// touches rows above (kk + 1) * 128 (and only those rows of lt are written).
-int left_chunk_step(const float* d, int lda, float* l, int ldl, int bs, int nrows, float* lt, int ldlt, int kk,
-                    cudaStream_t st, bool unit) {
+// Chunk kk (128 columns) of the left recurrence applied to the bs x bs
+// identity l: the recurrence on the chunk's columns (which also writes the
+// chunk's rows of lt), then L[:, after] += L[:, chunk] * D[chunk][after].
+// Row i stays zero left of column i, so chunk kk only touches rows above
+// (kk + 1) * 128.
+int left_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* l, int bs, float* lt, int kk,
+                    cudaStream_t st) {
     const int ib = 128;
     const float* dkk = d + (size_t)kk * ib * lda + (size_t)kk * ib;
     float* lk = l + (size_t)kk * ib;
-    float* ltk = lt + (size_t)kk * ib * ldlt;
-    const int rows = unit ? std::min(nrows, (kk + 1) * ib) : nrows;
-    LP_CHECK(launch_trsm_left(dkk, lda, lk, ldl, ib, rows, ltk, ldlt, st));
+    float* ltk = lt + (size_t)kk * ib * bs;
+    const int rows = (kk + 1) * ib;
+    LP_CHECK(launch_tl(dkk, lda, inv + (size_t)kk * kInvFloats, nullptr, 4, ib, nullptr, 4, 0, lk, bs, rows, ltk, bs,
+                       c->num_sms, st));
     const int m2 = bs - (kk + 1) * ib;
     if (m2 <= 0) return LP_OK;
-    return launch_sgemm_update(lk + ib, ldl, ltk, ldlt, dkk + ib, lda, rows, m2, ib, st);
+    return launch_sgemm_update(lk + ib, bs, ltk, bs, dkk + ib, lda, rows, m2, ib, st);
 }
 
-int left_blocked(const float* d, int lda, float* l, int ldl, int bs, int nrows, float* lt, int ldlt,
-                 cudaStream_t st, bool unit) {
-    if (bs <= 128) return launch_trsm_left(d, lda, l, ldl, bs, nrows, lt, ldlt, st);
-    for (int kk = 0; kk < bs / 128; kk++) LP_CHECK(left_chunk_step(d, lda, l, ldl, bs, nrows, lt, ldlt, kk, st, unit));
-    return LP_OK;
-}
-
-// Panel work of block step K: lu on the diagonal block, then the top block
-// row and the left block column (Lt written into `lt`, leading dimension the
-// number of rows below).  The left stage covers the rows below the diagonal
-// block up to row_end (default: all n).
-int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int K, float* lt, cudaStream_t st, int row_end) {
-    float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
-    const double b = bs;
+// Panel work of the block step at row k0 with block size bs: lu on the
+// diagonal block, then the block row right of it and the block column below
+// it in one launch (Lt written into `lt`, leading dimension the number of rows
+// below).  The left stage covers the rows below the diagonal block up to
+// row_end (default: all n).
+int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end) {
+    float* d = dA + (size_t)k0 * lda + k0;
+    const int kb = std::min(bs, n - k0);
+    const double b = kb;
+    float* inv = block_inv(c, k0);
     int e = prof_begin(c, st);
-    LP_CHECK(lu_stage(c, d, lda, bs, st));
+    LP_CHECK(lu_stage(c, d, lda, kb, inv, st));
     LP_CHECK(prof_end(c, st, LP_STAGE_LU, e, lu_flops(b), 8.0 * b * b));
-    const int rest = n - (K + 1) * bs;
+    const int rest = n - k0 - kb;
     if (rest <= 0) return LP_OK;
-    const int below = (row_end < 0 ? n : row_end) - (K + 1) * bs;
-    // top on st and left on aux2 run concurrently: both read only the factored
-    // diagonal block and write disjoint blocks (top uses st's dsub slot, left Lt)
-    if (below > 0) {
-        const double r = below;
-        LP_CUDA(cudaEventRecord(c->ev_side, st));
-        LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
-        e = prof_begin(c, c->aux2);
-        LP_CHECK(left_blocked(d, lda, d + (size_t)bs * lda, lda, bs, below, lt, below, c->aux2));
-        LP_CHECK(prof_end(c, c->aux2, LP_STAGE_LEFT, e, trsm_flops(b, r), 12.0 * b * r));
-        LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
-    }
-    const double r = rest;
+    const int below = (row_end < 0 ? n : row_end) - k0 - kb;
+    const double r = rest, w = below;
     e = prof_begin(c, st);
-    LP_CHECK(top_blocked(c, d, lda, d + bs, lda, bs, rest, st));
-    LP_CHECK(prof_end(c, st, LP_STAGE_TOP, e, trsm_flops(b, r), 8.0 * b * r));
-    if (below > 0) LP_CUDA(cudaStreamWaitEvent(st, c->ev_side_done, 0));
-    return LP_OK;
+    LP_CHECK(launch_tl(d, lda, inv, static_cast<const float*>(c->dt.ptr), kb, kb, d + kb, lda, rest,
+                       d + (size_t)kb * lda, lda, below, lt, std::max(4, below), c->num_sms, st));
+    return prof_end(c, st, LP_STAGE_TOP, e, trsm_flops(b, r + w), 8.0 * b * r + 12.0 * b * w);
+}
+
+// Inner block of the FP32 schedule: a multiple of 128 up to 512 whatever
+// block the caller named (the blocking changes results by rounding only).
+int f32_block(int bs) { return std::max(128, bs); }
+
+// Workspaces of the FP32 panel: the inverses of every 128-wide diagonal block
+// and the transposed lower triangle of the current block.
+int panel_ensure(lp_ctx* c, int n, int bs) {
+    LP_CHECK(c->dinv.ensure(sizeof(float) * kInvFloats * (size_t)((n + 127) / 128)));
+    return c->dt.ensure(sizeof(float) * (size_t)bs * bs);
 }
 
 // Blocked right-looking LU without pivoting (the block-row loop of
@@ -263,41 +262,37 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int K, float* lt, cu
 // panel of step K+1 (lu, top, left) runs on the high-priority auxiliary
 // stream while U_b runs on the main stream; they touch disjoint blocks, and
 // Lt is double-buffered so panel K+1 never overwrites the operand U_b reads.
-// top and left give the reference recurrences' values up to rounding
-// (blocked); the exact recurrences are lp_top_update_dev/lp_left_update_dev.
-int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int bs, cudaStream_t st) {
-    const size_t pan = sizeof(float) * (size_t)bs * n;
-    LP_CHECK(c->lt.ensure(2 * pan));
-    if (bs > 128) {
-        LP_CHECK(c->lti.ensure(2 * sizeof(float) * (size_t)128 * bs));
-        LP_CHECK(c->dsub.ensure(2 * sizeof(float) * (size_t)128 * bs));
-    }
+// The stages give the reference recurrences' values up to rounding; the exact
+// recurrences are lp_lu_block_dev, lp_top_update_dev, lp_left_update_dev.
+int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
+    const int bs = f32_block(user_bs);
+    LP_CHECK(c->lt.ensure(2 * sizeof(float) * (size_t)bs * n));
+    LP_CHECK(panel_ensure(c, n, bs));
     float* ltbuf[2] = {static_cast<float*>(c->lt.ptr), static_cast<float*>(c->lt.ptr) + (size_t)bs * n};
-    const int nb = n / bs;
     const double b = bs;
     LP_CHECK(panel_f32(c, dA, n, lda, bs, 0, ltbuf[0], st));
-    for (int K = 0; K + 1 < nb; K++) {
-        const int rest = n - (K + 1) * bs;
-        const double r = rest;
+    for (int K = 0; (K + 1) * bs < n; K++) {
+        const int rest = n - (K + 1) * bs, nx = std::min(bs, rest);  // nx: the next block
+        const double r = rest, x = nx;
         float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
         float* top = d + bs;
         float* lt = ltbuf[K & 1];
         float* c11 = d + (size_t)bs * lda + bs;
         int e = prof_begin(c, st);
-        LP_CHECK(launch_sgemm_update(c11, lda, lt, rest, top, lda, bs, rest, bs, st));
-        if (rest > bs)
-            LP_CHECK(launch_sgemm_update(c11 + (size_t)bs * lda, lda, lt + bs, rest, top, lda, rest - bs, bs, bs, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(b, r, b) + inner_flops(r - b, b, b),
-                          inner_bytes(b, r, b) + inner_bytes(r - b, b, b)));
+        LP_CHECK(launch_sgemm_update(c11, lda, lt, rest, top, lda, nx, rest, bs, st));
+        if (rest > nx)
+            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda, lda, lt + nx, rest, top, lda, rest - nx, nx, bs, st));
+        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(x, r, b) + inner_flops(r - x, x, b),
+                          inner_bytes(x, r, b) + inner_bytes(r - x, x, b)));
         LP_CUDA(cudaEventRecord(c->ev_fork, st));
         LP_CUDA(cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
-        LP_CHECK(panel_f32(c, dA, n, lda, bs, K + 1, ltbuf[(K + 1) & 1], c->aux));
+        LP_CHECK(panel_f32(c, dA, n, lda, bs, (K + 1) * bs, ltbuf[(K + 1) & 1], c->aux));
         LP_CUDA(cudaEventRecord(c->ev_join, c->aux));
-        if (rest > bs) {
-            const double r2 = rest - bs;
+        if (rest > nx) {
+            const double r2 = rest - nx;
             e = prof_begin(c, st);
-            LP_CHECK(launch_sgemm_update(c11 + (size_t)bs * lda + bs, lda, lt + bs, rest, top + bs, lda, rest - bs,
-                                         rest - bs, bs, st));
+            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda + nx, lda, lt + nx, rest, top + nx, lda, rest - nx,
+                                         rest - nx, bs, st));
             LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(r2, r2, b), inner_bytes(r2, r2, b)));
         }
         LP_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
@@ -327,14 +322,15 @@ struct Lane {
 template <class Band>
 static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r1, const Lane& ln,
                      const cudaEvent_t* panel_done, Band band) {
-    const int rows = r1 - r0, k0 = r0 / bs, k1 = r1 / bs;
+    const int rows = r1 - r0, k0 = r0 / bs, k1 = (r1 + bs - 1) / bs;
     const double b = bs, m = rows;
     float* slab = dA + (size_t)r0 * lda;
     cudaStream_t st = ln.st, aux = ln.aux;
     if (k0 > 0) {
         LP_CUDA(cudaStreamWaitEvent(st, panel_done[0], 0));
         int e = prof_begin(c, st);
-        LP_CHECK(left_blocked(dA, lda, slab, lda, bs, rows, ln.lt[0], rows, st));
+        LP_CHECK(launch_tl(dA, lda, block_inv(c, 0), nullptr, 4, bs, nullptr, 4, 0, slab, lda, rows, ln.lt[0], rows,
+                           c->num_sms, st));
         LP_CHECK(prof_end(c, st, LP_STAGE_LEFT, e, trsm_flops(b, m), 12.0 * b * m));
         for (int K = 0; K < k0; K++) {
             // block row K and D_K are final here: panel_done[K] was waited for
@@ -352,8 +348,8 @@ static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r
                 LP_CUDA(cudaStreamWaitEvent(aux, ln.fork, 0));
                 LP_CUDA(cudaStreamWaitEvent(aux, panel_done[K + 1], 0));
                 e = prof_begin(c, aux);
-                LP_CHECK(left_blocked(dA + (size_t)c1 * lda + c1, lda, cs, lda, bs, rows, ln.lt[(K + 1) & 1], rows,
-                                      aux));
+                LP_CHECK(launch_tl(dA + (size_t)c1 * lda + c1, lda, block_inv(c, c1), nullptr, 4, bs, nullptr, 4, 0, cs,
+                                   lda, rows, ln.lt[(K + 1) & 1], rows, c->num_sms, aux));
                 LP_CHECK(prof_end(c, aux, LP_STAGE_LEFT, e, trsm_flops(b, m), 12.0 * b * m));
                 LP_CUDA(cudaEventRecord(ln.join, aux));
                 const double nc = ncols - bs;  // > 0: the slab's own columns lie beyond c1 + bs
@@ -369,32 +365,33 @@ static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r
             }
         }
     }
-    LP_CHECK(panel_f32(c, dA, n, lda, bs, k0, ln.lt[k0 & 1], st, r1));
+    LP_CHECK(panel_f32(c, dA, n, lda, bs, r0, ln.lt[k0 & 1], st, r1));
     LP_CHECK(band(k0, st));
     for (int K = k0; K + 1 < k1; K++) {
-        const int below = r1 - (K + 1) * bs;  // >= bs
+        const int below = r1 - (K + 1) * bs;  // > 0; at least bs unless the slab ends the matrix
         const int rest = n - (K + 1) * bs;    // >= below
-        const double rb = below, rc = rest;
+        const int nx = std::min(bs, below);   // the next block
+        const double rb = below, rc = rest, x = nx;
         float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
         float* top = d + bs;
         float* c11 = d + (size_t)bs * lda + bs;
         const float* l = ln.lt[K & 1];
         int e = prof_begin(c, st);
-        LP_CHECK(launch_sgemm_update(c11, lda, l, below, top, lda, bs, rest, bs, st));
-        if (below > bs)
-            LP_CHECK(launch_sgemm_update(c11 + (size_t)bs * lda, lda, l + bs, below, top, lda, below - bs, bs, bs, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(b, rc, b) + inner_flops(rb - b, b, b),
-                          inner_bytes(b, rc, b) + inner_bytes(rb - b, b, b)));
+        LP_CHECK(launch_sgemm_update(c11, lda, l, below, top, lda, nx, rest, bs, st));
+        if (below > nx)
+            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda, lda, l + nx, below, top, lda, below - nx, nx, bs, st));
+        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(x, rc, b) + inner_flops(rb - x, x, b),
+                          inner_bytes(x, rc, b) + inner_bytes(rb - x, x, b)));
         LP_CUDA(cudaEventRecord(ln.fork, st));
         LP_CUDA(cudaStreamWaitEvent(aux, ln.fork, 0));
-        LP_CHECK(panel_f32(c, dA, n, lda, bs, K + 1, ln.lt[(K + 1) & 1], aux, r1));
+        LP_CHECK(panel_f32(c, dA, n, lda, bs, (K + 1) * bs, ln.lt[(K + 1) & 1], aux, r1));
         LP_CHECK(band(K + 1, aux));
         LP_CUDA(cudaEventRecord(ln.join, aux));
-        if (below > bs) {
-            const double r2 = below - bs, c2 = rest - bs;
+        if (below > nx) {
+            const double r2 = below - nx, c2 = rest - nx;
             e = prof_begin(c, st);
-            LP_CHECK(launch_sgemm_update(c11 + (size_t)bs * lda + bs, lda, l + bs, below, top + bs, lda, below - bs,
-                                         rest - bs, bs, st));
+            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda + nx, lda, l + nx, below, top + nx, lda, below - nx,
+                                         rest - nx, bs, st));
             LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(r2, c2, b), inner_bytes(r2, c2, b)));
         }
         LP_CUDA(cudaStreamWaitEvent(st, ln.join, 0));
@@ -424,20 +421,18 @@ static std::vector<int> slab_cuts(int n, int bs) {
 // lanes at once (a slab's own steps start after the other lane's last panel),
 // so the panel's scratch is shared.  With host_out, every block row goes back
 // to host_out (leading dimension lda) on the copy stream as soon as it is
-// final.  ev: at least 2 n / bs + 2 events.
-int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int bs, cudaStream_t st,
+// final.  ev: at least 2 ceil(n / bs) + 2 events.
+int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int user_bs, cudaStream_t st,
                       float* host_out, const std::vector<cudaEvent_t>& ev) {
+    const int bs = f32_block(user_bs);
     const std::vector<int> cuts = slab_cuts(n, bs);
-    const int ns = (int)cuts.size() - 1, nb = n / bs;
+    const int ns = (int)cuts.size() - 1, nb = (n + bs - 1) / bs;
     if ((int)ev.size() < nb + ns + 2) return fail(LP_E_INVALID, "streamed factorization: too few events");
     int hmax = 0;
     for (int s = 0; s < ns; s++) hmax = std::max(hmax, cuts[s + 1] - cuts[s]);
     const size_t ltf = (size_t)bs * hmax;
     LP_CHECK(c->lt.ensure(4 * sizeof(float) * ltf));
-    if (bs > 128) {
-        LP_CHECK(c->lti.ensure(2 * sizeof(float) * (size_t)128 * bs));
-        LP_CHECK(c->dsub.ensure(2 * sizeof(float) * (size_t)128 * bs));
-    }
+    LP_CHECK(panel_ensure(c, n, bs));
     if (c->copy_in == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
     if (host_out != nullptr && c->copy == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
     float* lt = static_cast<float*>(c->lt.ptr);
@@ -460,8 +455,8 @@ int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int
         if (host_out == nullptr) return LP_OK;
         LP_CUDA(cudaStreamWaitEvent(c->copy, ev[K], 0));
         const size_t r = (size_t)K * bs;
-        LP_CUDA(cudaMemcpy2DAsync(host_out + r * lda, pitch, dA + r * lda, pitch, sizeof(float) * n, bs,
-                                  cudaMemcpyDeviceToHost, c->copy));
+        LP_CUDA(cudaMemcpy2DAsync(host_out + r * lda, pitch, dA + r * lda, pitch, sizeof(float) * n,
+                                  std::min(bs, n - (int)r), cudaMemcpyDeviceToHost, c->copy));
         return LP_OK;
     };
     // the second lane starts after the work queued on st so far
@@ -566,6 +561,7 @@ int lp_ctx_create(int device, lp_ctx** out) {
         return fail(LP_E_NODEVICE, std::string("lp_ctx_create: device '") + prop.name +
                                        "' is not sm_100 (this library is built for sm_100a only)");
     LP_CHECK(lu_init_attrs());
+    LP_CHECK(panel_init_attrs());
     LP_CHECK(trsm_init_attrs());
     LP_CHECK(sgemm_init_attrs());
     LP_CHECK(gesl_inv_init_attrs());
@@ -728,8 +724,9 @@ int lp_lu_block_dev(lp_ctx* c, float* dA, int lda, int bs) {
     if (!is_pow2(bs) || bs < 16 || bs > 512 || lda < bs || lda % 4 != 0)
         return fail(LP_E_INVALID, "lp_lu_block_dev: bs must be a power of two in [16, 512], lda >= bs, lda % 4 == 0");
     LP_CUDA(cudaSetDevice(c->device));
-    if (bs > 128) LP_CHECK(c->lti.ensure(sizeof(float) * (size_t)128 * bs));
-    return lu_stage(c, dA, lda, bs, c->stream);
+    if (bs <= 128) return launch_lu_small(dA, lda, bs, c->stream);
+    LP_CHECK(panel_ensure(c, bs, bs));
+    return lu_stage(c, dA, lda, bs, block_inv(c, 0), c->stream);
 }
 
 int lp_top_update_dev(lp_ctx* c, const float* dLU, int ldlu, float* dT, int ldt, int bs, int ncols) {

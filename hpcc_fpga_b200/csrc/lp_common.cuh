@@ -34,6 +34,28 @@ long long launch_count();
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 #ifdef __CUDACC__
+// Launches a kernel that begins with pdl_wait(): its blocks may be set up while
+// the kernel before it on the stream still runs (programmatic dependent
+// launch); pdl_wait() returns once that kernel has finished and its writes are
+// visible.  pdl_start() lets the next such kernel's blocks come; every block
+// of this one is resident by then.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // 4-byte asynchronous global -> shared copy (any float address), and the wait
 // for all of the calling thread's outstanding copies.
 __device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
@@ -108,7 +130,6 @@ int launch_sgemm_update(float* c, int ldc, const float* lt, int ldlt, const floa
 int launch_dgemm_update(double* c, int ldc, const double* lt, int ldlt, const double* t, int ldt, int m, int n, int k,
                         cudaStream_t s);
 int dgemm_init_attrs();
-int launch_transpose(const float* src, int lds, float* dst, int ldd, int rows, int cols, cudaStream_t s);
 int launch_transpose_f64(const double* src, int lds, double* dst, int ldd, int rows, int cols, cudaStream_t s);
 // Forward + back substitution for nrhs rows of b with the encoded factors:
 // two persistent sweeps per 16 right-hand sides, each finisher CTA inverting

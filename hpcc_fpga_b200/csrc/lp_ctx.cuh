@@ -34,9 +34,20 @@ int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int bs, cudaStream_t st);
 int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int bs, cudaStream_t st,
                       float* host_out, const std::vector<cudaEvent_t>& ev);
 int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cudaStream_t st);
-// Panel work of block step K (lu, top, left; Lt into lt), on stream st; the
-// left stage covers the rows below the diagonal block up to row_end (-1: n).
-int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int K, float* lt, cudaStream_t st, int row_end = -1);
+// Panel work of the block step at row k0 (lu, top, left; Lt into lt), on
+// stream st; the left stage covers the rows below the diagonal block up to
+// row_end (-1: n).
+int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end = -1);
+// Workspaces of the panel stages for order n and (inner) block bs.
+int panel_ensure(lp_ctx* c, int n, int bs);
+// k_panel.cu: LU of a 128 x 128 diagonal block, its 32 x 32 inverses into inv
+// (kInvFloats floats) and its lower triangle transposed into dt; top and left
+// beside a factored block of 128 .. 512.
+constexpr size_t kInvFloats = 8 * 1024;
+int panel_init_attrs();
+int launch_lu128(float* a, int lda, float* inv, float* dt, int lddt, cudaStream_t st);
+int launch_tl(const float* d, int ldd, const float* inv, const float* dt, int lddt, int bs, float* t, int ldt,
+              int ncols, float* l, int ldl, int nrows, float* lt, int ldlt, int sms, cudaStream_t st);
 // E4M3: one absmax scale per 512 x 512 block (512 rows of L / columns of T by
 // a 512-wide K segment); sc holds 6 arrays of kseg(k) * nblk floats.
 int quantize_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, bool fp8,
@@ -45,11 +56,6 @@ inline int kseg(int k) { return (k + 511) / 512; }
 // Split-BF16 operands (exact three-term split; 6 or 3 K-segments) of a block step.
 int split_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, uint8_t* aq,
                 uint8_t* bq, cudaStream_t st, int nseg = 6);
-// The stages of panel_f32 (lp_abi.cu): lu of a diagonal block, and the top /
-// left recurrences over a block row / column (Lt written into lt).  With
-// `unit` the operand is the bs x bs identity: top then yields a lower and left
-// an upper triangle, and each 128-wide chunk skips the columns (top) or rows
-// (left) that stay exactly zero.
 // Inverses of the diagonal block's two triangles for the tensor-core panel:
 // top applied to the bs x bs identity (winv) and left applied to it (vinv;
 // vlt: scratch for its transposed chunks), both starting from the identity.
@@ -58,19 +64,16 @@ struct TriInverses {
     float* vinv;
     float* vlt;
 };
-// With inv (bs > 128), chunk kk of both identity recurrences runs on the
-// context's inv_top / inv_left streams as soon as step kk of the lu stage has
-// made block row and column kk of d final; st waits for both at the end.
-int lu_stage(lp_ctx* c, float* d, int lda, int bs, cudaStream_t st, const TriInverses* inv = nullptr);
-int top_blocked(lp_ctx* c, const float* d, int lda, float* t, int ldt, int bs, int ncols, cudaStream_t st,
-                bool unit = false);
-int left_blocked(const float* d, int lda, float* l, int ldl, int bs, int nrows, float* lt, int ldlt, cudaStream_t st,
-                 bool unit = false);
-// Step kk (128-wide chunk) of top_blocked / left_blocked, for bs > 128.
-int top_chunk_step(lp_ctx* c, const float* d, int lda, float* t, int ldt, int bs, int ncols, int kk, cudaStream_t st,
-                   bool unit);
-int left_chunk_step(const float* d, int lda, float* l, int ldl, int bs, int nrows, float* lt, int ldlt, int kk,
-                    cudaStream_t st, bool unit);
+// lu stage (lp_abi.cu) of a bs x bs diagonal block; inv: kInvFloats floats per
+// 128 rows.  With tri (bs > 128), chunk kk of both identity recurrences runs
+// on the context's inv_top / inv_left streams as soon as step kk of the lu
+// stage has made block row and column kk of d final; st waits for both at the
+// end.
+int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, const TriInverses* tri = nullptr);
+// Step kk (128-wide chunk) of the identity recurrences, for bs > 128.
+int top_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* t, int bs, int kk, cudaStream_t st);
+int left_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* l, int bs, float* lt, int kk,
+                    cudaStream_t st);
 // E4M3 scales: scale_x[seg * sstride + block] per 512-wide K segment and
 // 512-row (A) / 512-column (B) block (k_umma.cu).
 int launch_umma_update(float* c, int ldc, const void* aq, int aq_rows, const void* bq, int bq_rows, int m_off,
@@ -163,8 +166,8 @@ struct lp_ctx {
     cudaEvent_t ev_inv[lp::kMixedMaxBlock / 128] = {nullptr};
     cudaEvent_t ev_inv_top = nullptr, ev_inv_left = nullptr;
     lp::Workspace lt;    // transposed left panels (2 x bs x n, alternating by block step)
-    lp::Workspace dsub;  // transposed diagonal sub-blocks of the blocked top stage (per stream)
-    lp::Workspace lti;   // transposed inner left panel of the recursive lu stage (per stream)
+    lp::Workspace dt;    // transposed lower triangle of the current diagonal block (bs x bs)
+    lp::Workspace dinv;  // 32 x 32 inverses of every 128-wide diagonal block (kInvFloats floats each)
     lp::Workspace q;     // tensor-core operands: 2 x (Lq, Tq), BF16 or E4M3, n x bs each
     lp::Workspace qs;    // E4M3 block scales (absmax, scale, 1/scale for L and T), 2 buffers
     lp::Workspace err;   // device error word of the tensor-core update (bounded waits)
@@ -207,7 +210,7 @@ struct lp_ctx {
     double prof_s[LP_NSTAGES] = {0}, prof_flops[LP_NSTAGES] = {0}, prof_bytes[LP_NSTAGES] = {0};
     long long prof_calls[LP_NSTAGES] = {0};
     void release_all() {
-        lp::Workspace* all[] = {&lt, &dsub, &lti, &q, &qs, &err, &tri, &tq, &gw, &gerr, &dA, &dA0, &dB, &dB64, &dX, &dR, &dCol,
+        lp::Workspace* all[] = {&lt, &dt, &dinv, &q, &qs, &err, &tri, &tq, &gw, &gerr, &dA, &dA0, &dB, &dB64, &dX, &dR, &dCol,
                                 &dnorm, &gmw, &f64a, &f64b, &f64lt, &f64w, &psync, &pat, &pdesc, &pw, &pipvt, &bsys, &bnext, &tA, &tB, &bA0, &bB32, &bout, &bsys_ir, &hA, &hB, &hX};
         for (auto* w : all) w->release();
         if (bgraph != nullptr) cudaGraphExecDestroy(bgraph);
@@ -228,3 +231,10 @@ struct lp_ctx {
         hstat = nullptr;
     }
 };
+
+namespace lp {
+// The inverses of the diagonal block that starts at row k0 (a multiple of 128).
+inline float* block_inv(lp_ctx* c, int k0) {
+    return static_cast<float*>(c->dinv.ptr) + kInvFloats * (size_t)(k0 / 128);
+}
+}  // namespace lp

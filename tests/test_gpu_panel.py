@@ -1,0 +1,39 @@
+"""The FP32 factorization at the edges of its inner blocking: 128-wide inner
+blocks whatever block the caller names, a ragged last block in pieces of 64,
+32 and 16, strips of 32 / 64 beside a block, and trailing updates on each side
+of the tile forms' borders.  Bound as for the whole factorization elsewhere:
+|got - want| <= 256 eps max(1, |want|) against the oracle's factors."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+FLT_EPS = float(np.finfo(np.float32).eps)
+
+
+@pytest.mark.parametrize("n,bs,pad", [(16, 16, 0), (112, 16, 0), (144, 16, 4), (208, 16, 0), (224, 32, 0), (320, 64, 8),
+                                      (384, 128, 0), (1088, 64, 0), (1280, 256, 0), (1536, 512, 4), (2304, 256, 0)])
+def test_gefa_blocking_edges(ctx, dev, n, bs, pad):
+    A, _, _, _ = oracle.gen_reference(n)
+    store = np.full((n, n + pad), 7.0, np.float32)
+    store[:, :n] = A
+    d = dev.put(store)
+    ctx.gefa(d.data_ptr(), n, n + pad, bs)
+    got = dev.get(d)
+    assert np.all(got[:, n:] == 7.0)  # the padding is not touched
+    want = oracle.gefa_nopvt(A).astype(np.float64)
+    err = np.abs(got[:, :n].astype(np.float64) - want) / np.maximum(1.0, np.abs(want))
+    assert err.max() < 256 * FLT_EPS
+
+
+@pytest.mark.parametrize("n,bs", [(1088, 64), (2096, 16), (1536, 128)])
+def test_streamed_ragged_blocks(ctx, lp, n, bs):
+    """Page-locked buffers (factored in row slabs while copied in) give the pageable path's bits."""
+    A, b, _, _ = oracle.gen_reference(n)
+    A1, b1 = A.copy(), b.copy()
+    ctx.calculate(A1, b1, bs)
+    pa, pb = lp.Pinned((n, n)), lp.Pinned((n,))
+    pa.array[...], pb.array[...] = A, b
+    ctx.calculate(pa.array, pb.array, bs)
+    assert np.array_equal(pa.array, A1) and np.array_equal(pb.array, b1)
