@@ -15,12 +15,12 @@
 // panel of the tallest column does not fit the SMs' shared memory):
 //   k_piv_panel  the PB columns of M (PB storage rows x the trailing length),
 //                one cooperative launch: each CTA holds a slice of rows in
-//                shared memory; per step a bounded grid barrier publishes
-//                every CTA's best candidate and its row, all CTAs agree on
-//                the pivot (largest |v|, then smallest index), the two rows
-//                are exchanged across CTAs and each CTA scales and updates
-//                its rows with the reference's rounding (multiplier in
-//                double, product and sum rounded to float separately).
+//                shared memory; per step it publishes its best candidate and
+//                that row, all CTAs agree on the pivot (largest |v|, then
+//                smallest index), the two rows are exchanged across CTAs and
+//                each CTA scales and updates its rows with the reference's
+//                rounding (multiplier in double, product and sum rounded to
+//                float separately).
 //                Inside the panel whole panel rows are exchanged ("block
 //                form"); the earlier multipliers of the same panel are put
 //                back into LINPACK order by k_piv_convert at the end.
@@ -35,8 +35,8 @@
 //                substitution, one cooperative launch with one bounded grid
 //                barrier per panel and direction.
 //
-// Every spin-wait is bounded: a barrier that does not complete within the
-// iteration limit sets the error word and every CTA returns; the host
+// Every spin-wait is bounded: a message or barrier that does not arrive within
+// the iteration limit sets the error word and every CTA returns; the host
 // reports LP_E_TIMEOUT.
 #include "lp_ctx.cuh"
 
@@ -48,11 +48,14 @@ constexpr int GMAX = 256;                // CTAs of one panel launch, at most
 constexpr int PBMAX = 128;               // panel width, at most
 constexpr unsigned kSpinLimit = 1u << 21;
 
-// Device scratch of one factorization or solve.
-constexpr size_t kKeysOff = 16;                                          // u64 [2][GMAX]
-constexpr size_t kRowsOff = kKeysOff + 2 * GMAX * sizeof(unsigned long long);  // float [2][GMAX][PBMAX]
-constexpr size_t kKrowOff = kRowsOff + 2 * (size_t)GMAX * PBMAX * sizeof(float);  // float [2][PBMAX]
-constexpr size_t kSyncBytes = kKrowOff + 2 * PBMAX * sizeof(float);
+// Device scratch of one factorization or solve: a barrier counter, an error
+// word, then the panel's messages, 64-bit words (tag << 32 | 32-bit value)
+// that are valid on their own, alternating by pivot step.
+constexpr int RW = PBMAX + 2;                                                          // a row and its reciprocal
+constexpr size_t kKeysOff = 16;                                                        // u64 [2][GMAX]
+constexpr size_t kRowsOff = kKeysOff + 2 * (size_t)GMAX * sizeof(unsigned long long);  // u64 [2][GMAX][RW]
+constexpr size_t kKrowOff = kRowsOff + 2 * (size_t)GMAX * RW * sizeof(unsigned long long);  // u64 [2][PBMAX]
+constexpr size_t kSyncBytes = kKrowOff + 2 * (size_t)PBMAX * sizeof(unsigned long long);
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     unsigned v;
@@ -87,38 +90,85 @@ __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target, int* e
     return s_ok != 0;
 }
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
-    }
+// Rank of M row value v in the pivot search: larger magnitudes rank higher
+// (the bit pattern of a non-negative float orders like the value), equal ones
+// are told apart by the index (the smaller wins, as the reference's strict "<"
+// scan keeps the first).  NaN never wins, except at the diagonal itself, which
+// the reference's scan then never leaves.
+__device__ __forceinline__ unsigned pivot_rank(float v, bool diag) {
+    const float a = fabsf(v);
+    if (a != a) return diag ? 0xFFFFFFFFu : 0u;
+    return __float_as_uint(a) + 1u;
+}
+
+__device__ __forceinline__ void st_word(unsigned long long* p, unsigned tag, unsigned v) {
+    const unsigned long long w = ((unsigned long long)tag << 32) | v;
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
-// Candidate key of M row i in the pivot search: |v| in the high word (the
-// bit pattern of a non-negative float orders like the value), the index
-// complemented in the low word (equal magnitudes: the smaller index wins, as
-// the reference's strict "<" scan keeps the first).  NaN never wins, except
-// at the diagonal itself, which the reference's scan then never leaves.
-__device__ __forceinline__ unsigned long long pivot_key(float v, unsigned i, bool diag) {
-    const float a = fabsf(v);
-    if (a != a) return diag ? ~0ull : 0ull;
-    return (static_cast<unsigned long long>(__float_as_uint(a)) << 32) | (0xFFFFFFFFu - i);
+// A CTA's candidate in one word: its rank, its row within the CTA and the
+// step (20 bits: a matrix of that order would take 4 TB).
+constexpr int kKeyTagBits = 20, kKeyRowBits = 12;
+__device__ __forceinline__ unsigned long long key_word(unsigned rank, unsigned row, unsigned tag) {
+    return ((unsigned long long)rank << 32) | (row << kKeyTagBits) | tag;
 }
 
+// One more unsuccessful poll: false (and the error word set) past the limit or
+// when another CTA gave up.
+__device__ __forceinline__ bool keep_polling(unsigned& spins, int* err) {
+    if ((++spins & 255u) != 0) return true;
+    if (*reinterpret_cast<volatile int*>(err) != 0) return false;
+    if (spins > kSpinLimit) {
+        atomicExch(err, 1);
+        return false;
+    }
+    return true;
+}
+
+// The value of the message word at p once it carries `tag`.
+__device__ __forceinline__ unsigned poll_word(const unsigned long long* p, unsigned tag, int* err, bool& ok) {
+    unsigned spins = 0;
+    unsigned long long w = ld_word(p);
+    while ((unsigned)(w >> 32) != tag) {
+        if (!keep_polling(spins, err)) {
+            ok = false;
+            break;
+        }
+        w = ld_word(p);
+    }
+    return (unsigned)w;
+}
+
+// One panel.  A pivot step is a chain through all CTAs, so what counts is its
+// latency.  Each CTA brings only the next column up to date, finds its
+// candidate there and publishes it with its row (the row's other columns
+// brought up to date on the way out); the rank-1 update of everything else
+// runs while the messages travel.  Messages are words that carry their step,
+// so a consumer needs one L2 round trip for the candidates and one for the
+// winner's row, without barrier or fence.  The winner's reciprocal, a double
+// division, travels with its row: it is formed while the candidates do.  Two
+// buffers suffice: a CTA publishes step s + 2 only after every CTA published
+// s + 1, and so had read all it needs of s.  Measured on one B200, 128 steps:
+// m = 4500 855 -> 330 us (a grid barrier, then keys and row, each an L2 round
+// trip, before), m = 900 280 us.
+// R is a multiple of 4.
 __global__ void __launch_bounds__(PT, 1)
     k_piv_panel(float* __restrict__ a, int lda, int n, int k0, int kb, int R, int* __restrict__ ipvt,
-                unsigned char* __restrict__ sync, unsigned bar_base) {
-    extern __shared__ float slab[];  // kb columns of M x R rows: slab[c * R + r]
-    __shared__ float newk[PBMAX];
-    __shared__ unsigned long long red[PT / 32];
-    __shared__ int s_p, s_wg;
-    unsigned* bar = reinterpret_cast<unsigned*>(sync);
+                unsigned char* __restrict__ sync) {
+    extern __shared__ __align__(16) float slab[];  // kb columns of M x R rows: slab[c * R + r]
+    __shared__ float newk[PBMAX];    // the pivot row of the last step
+    __shared__ unsigned red_v[PT / 32], red_i[PT / 32];
+    __shared__ int s_p, s_ok;
+    __shared__ double s_rcp;         // its -1 / pivot
     int* err = reinterpret_cast<int*>(sync + 4);
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(sync + kKeysOff);
-    float* rows = reinterpret_cast<float*>(sync + kRowsOff);
-    float* krow = reinterpret_cast<float*>(sync + kKrowOff);
+    unsigned long long* rows = reinterpret_cast<unsigned long long*>(sync + kRowsOff);
+    unsigned long long* krow = reinterpret_cast<unsigned long long*>(sync + kKrowOff);
     const int G = gridDim.x, g = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row0 = g * R;                       // M rows k0 + row0 ... belong to this CTA
     const int nr = max(0, min(R, n - k0 - row0));
@@ -130,86 +180,144 @@ __global__ void __launch_bounds__(PT, 1)
     cp_async_wait_all();
     __syncthreads();
     for (int kk = 0; kk < kb; kk++) {
-        const int k = k0 + kk, par = kk & 1;
+        const int k = k0 + kk, par = k & 1;
+        const unsigned tag = (unsigned)k + 1u;
         const int rk = kk - row0;  // local index of M row k (in range only in its owner)
         const bool own_k = rk >= 0 && rk < nr;
-        const float* colk = slab + kk * R;
-        unsigned long long best = 0;
-        for (int r = max(0, rk) + tid; r < nr; r += PT) {
-            const unsigned long long key = pivot_key(colk[r], (unsigned)(cbase + r), r == rk);
-            best = key > best ? key : best;
-        }
-        best = warp_max_u64(best);
-        if (lane == 0) red[warp] = best;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long v = lane < PT / 32 ? red[lane] : 0ull;
-            v = warp_max_u64(v);
-            if (lane == 0) red[0] = v;
-        }
-        __syncthreads();
-        const unsigned long long mine = red[0];
-        // publish this CTA's candidate (its whole panel row) and, from the owner, row k
-        if (mine != 0ull) {
-            const int rc = mine == ~0ull ? rk : (int)(0xFFFFFFFFu - (unsigned)mine) - (int)cbase;
-            float* dst = rows + ((size_t)par * GMAX + g) * PBMAX;
-            for (int c = tid; c < kb; c += PT) dst[c] = slab[c * R + rc];
-        }
-        if (own_k)
-            for (int c = tid; c < kb; c += PT) krow[par * PBMAX + c] = slab[c * R + rk];
-        if (tid == 0) keys[par * GMAX + g] = mine;
-        if (!grid_sync(bar, bar_base + (unsigned)(kk + 1) * (unsigned)G, err)) return;
-        if (warp == 0) {
-            unsigned long long v = 0;
-            int wg = 0;
-            for (int q = lane; q < G; q += 32) {
-                const unsigned long long x = __ldcg(keys + par * GMAX + q);
-                if (x > v) v = x, wg = q;
+        const int lo = max(0, rk);  // this CTA's rows from k on
+        float* colm = slab + (kk - 1) * R;  // (kk > 0) the last step's column: its multipliers
+        // the last step's multipliers (the reciprocal in double, the product rounded to float), column k up to date
+        // (product and sum rounded separately), and the best row of it
+        unsigned best = 0, bi = 0xFFFFFFFFu;
+        {
+            const double s = s_rcp;
+            const float u = newk[kk];
+            float* colk = slab + kk * R;
+            for (int r = lo + tid; r < nr; r += PT) {
+                float v = colk[r];
+                if (kk > 0) {
+                    const float m = (float)((double)colm[r] * s);
+                    colm[r] = m;
+                    v = __fadd_rn(v, __fmul_rn(m, u));
+                    colk[r] = v;
+                }
+                const unsigned q = pivot_rank(v, r == rk);
+                if (q > best) best = q, bi = (unsigned)r;  // rows in ascending order: the first stays
             }
+        }
+        {
+            const unsigned m = __reduce_max_sync(0xffffffffu, best);
+            const unsigned i = __reduce_min_sync(0xffffffffu, best == m ? bi : 0xFFFFFFFFu);
+            if (lane == 0) red_v[warp] = m, red_i[warp] = i;
+        }
+        __syncthreads();
+        {
+            const unsigned v = lane < PT / 32 ? red_v[lane] : 0u, i = lane < PT / 32 ? red_i[lane] : 0xFFFFFFFFu;
+            best = __reduce_max_sync(0xffffffffu, v);
+            bi = __reduce_min_sync(0xffffffffu, v == best ? i : 0xFFFFFFFFu);
+        }
+        // publish the candidate, its panel row and, from the owner, row k
+        if (tid == PT - 1) {
+            const unsigned long long w = key_word(best, bi & ((1u << kKeyRowBits) - 1u), tag);
+            asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(keys + par * GMAX + g), "l"(w) : "memory");
+        }
+        const int half = tid >> 7, c0 = tid & 127;
+        unsigned long long* mine = rows + ((size_t)par * GMAX + g) * RW;
+        if (c0 < kb && (half == 0 ? best != 0u : own_k)) {
+            const int r = half == 0 ? (int)bi : rk;
+            float v = slab[c0 * R + r];
+            if (kk > 0 && c0 > kk) v = __fadd_rn(v, __fmul_rn(colm[r], newk[c0]));
+            st_word(half == 0 ? mine + c0 : krow + par * PBMAX + c0, tag, __float_as_uint(v));
+        }
+        if (warp == 1 && best != 0u && lane == 0) {
+            const double s = -1.0 / (double)slab[kk * R + (int)bi];
+            st_word(mine + PBMAX, tag, (unsigned)__double2loint(s));
+            st_word(mine + PBMAX + 1, tag, (unsigned)__double2hiint(s));
+        }
+        __syncthreads();  // the rows above are read before the update below changes them
+        if (warp == 0) {
+            constexpr int KQ = GMAX / 32;
+            bool ok = true;
+            unsigned long long w[KQ];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long ov = __shfl_xor_sync(0xffffffffu, v, o);
-                const int ow = __shfl_xor_sync(0xffffffffu, wg, o);
-                if (ov > v || (ov == v && ow < wg)) v = ov, wg = ow;
+            for (int j = 0; j < KQ; j++)  // every candidate's word in flight at once
+                w[j] = lane + 32 * j < G ? ld_word(keys + par * GMAX + lane + 32 * j) : tag;
+            unsigned v = 0, i = 0xFFFFFFFFu;
+#pragma unroll
+            for (int j = 0; j < KQ; j++) {
+                const int q = lane + 32 * j;
+                if (q < G) {
+                    unsigned spins = 0;
+                    while (((unsigned)w[j] & ((1u << kKeyTagBits) - 1u)) != tag && ok) {
+                        ok = keep_polling(spins, err);
+                        w[j] = ld_word(keys + par * GMAX + q);
+                    }
+                    const unsigned x = (unsigned)(w[j] >> 32), y = (unsigned)(k0 + q * R) + ((unsigned)w[j] >> kKeyTagBits);
+                    if (x > v || (x == v && y < i)) v = x, i = y;
+                }
             }
-            if (lane == 0) {
-                s_p = v == ~0ull ? k : (int)(0xFFFFFFFFu - (unsigned)v);
-                s_wg = wg;
+            const unsigned m = __reduce_max_sync(0xffffffffu, v);
+            const unsigned im = __reduce_min_sync(0xffffffffu, v == m ? i : 0xFFFFFFFFu);
+            const int all = __all_sync(0xffffffffu, ok);
+            if (lane == 0) s_p = (int)im, s_ok = all;
+        } else if (kk > 0) {
+            // rank-1 update of the panel's later columns (product and sum rounded separately): a warp takes every
+            // seventh column, a lane four rows, four columns' loads in flight
+            constexpr int CB = 4, CS = PT / 32 - 1;
+            for (int r = 4 * lane; r < nr; r += 128) {
+                if (r + 3 < lo) continue;
+                const float4 m = *reinterpret_cast<const float4*>(colm + r);
+                for (int c = kk + warp; c < kb; c += CB * CS) {
+                    float4 x[CB];
+                    float u[CB];
+#pragma unroll
+                    for (int j = 0; j < CB; j++)
+                        if (c + j * CS < kb) {
+                            x[j] = *reinterpret_cast<const float4*>(slab + (c + j * CS) * R + r);
+                            u[j] = newk[c + j * CS];
+                        }
+#pragma unroll
+                    for (int j = 0; j < CB; j++)
+                        if (c + j * CS < kb) {
+                            if (r >= lo) x[j].x = __fadd_rn(x[j].x, __fmul_rn(m.x, u[j]));
+                            if (r + 1 >= lo) x[j].y = __fadd_rn(x[j].y, __fmul_rn(m.y, u[j]));
+                            if (r + 2 >= lo) x[j].z = __fadd_rn(x[j].z, __fmul_rn(m.z, u[j]));
+                            x[j].w = __fadd_rn(x[j].w, __fmul_rn(m.w, u[j]));
+                            *reinterpret_cast<float4*>(slab + (c + j * CS) * R + r) = x[j];
+                        }
+                }
             }
         }
         __syncthreads();
-        const int p = s_p, wg = s_wg;
-        for (int c = tid; c < kb; c += PT) newk[c] = __ldcg(rows + ((size_t)par * GMAX + wg) * PBMAX + c);
-        __syncthreads();
-        if (p != k) {  // exchange M rows k and p over the whole panel
-            const int rp = p - (int)cbase;
-            if (rp >= 0 && rp < nr)
-                for (int c = tid; c < kb; c += PT) slab[c * R + rp] = __ldcg(krow + par * PBMAX + c);
-            if (own_k)
-                for (int c = tid; c < kb; c += PT) slab[c * R + rk] = newk[c];
+        if (!s_ok) return;
+        const int p = s_p, wg = (p - k0) / R, rp = p - (int)cbase;
+        const bool own_p = p != k && rp >= 0 && rp < nr;
+        bool ok = true;
+        const unsigned long long* won = rows + ((size_t)par * GMAX + wg) * RW;
+        if (c0 < kb) {
+            if (half == 0) {
+                const float v = __uint_as_float(poll_word(won + c0, tag, err, ok));
+                newk[c0] = v;
+                if (p != k && own_k) slab[c0 * R + rk] = v;  // exchange M rows k and p over the whole panel
+            } else if (own_p) {
+                slab[c0 * R + rp] = __uint_as_float(poll_word(krow + par * PBMAX + c0, tag, err, ok));
+            }
+        }
+        if (warp == PT / 32 - 1) {  // the reciprocal, by two lanes
+            const unsigned h = lane < 2 ? poll_word(won + PBMAX + lane, tag, err, ok) : 0u;
+            const unsigned hi = __shfl_sync(0xffffffffu, h, 1);
+            if (lane == 0) s_rcp = __hiloint2double((int)hi, (int)h);
         }
         if (g == 0 && tid == 0) ipvt[k] = p;
-        __syncthreads();
-        // multipliers: the reciprocal in double, the product rounded to float
-        const double s = -1.0 / (double)newk[kk];
-        const int rs = max(0, kk + 1 - row0);  // local rows below the pivot
-        float* colm = slab + kk * R;
-        for (int r = rs + tid; r < nr; r += PT) colm[r] = (float)((double)colm[r] * s);
-        __syncthreads();
-        // rank-1 update of the panel's later columns: product and sum rounded separately
-        const int nrows = nr - rs;
-        if (kk + 1 < kb && nrows > 0) {
-            int rw = 32;
-            while (rw < nrows && rw < PT) rw <<= 1;
-            const int cg = PT / rw, rl = tid & (rw - 1);
-            for (int c = kk + 1 + tid / rw; c < kb; c += cg) {
-                const float u = newk[c];
-                float* colc = slab + c * R;
-                for (int r = rs + rl; r < nr; r += rw) colc[r] = __fadd_rn(colc[r], __fmul_rn(colm[r], u));
-            }
-        }
-        __syncthreads();
+        if (!__syncthreads_and(ok)) return;
     }
+    // the last column's multipliers
+    {
+        const double s = s_rcp;
+        for (int r = max(0, kb - row0) + tid; r < nr; r += PT)
+            slab[(kb - 1) * R + r] = (float)((double)slab[(kb - 1) * R + r] * s);
+    }
+    __syncthreads();
     for (int c = 0; c < kb; c++) {
         float* dst = a + (size_t)(k0 + c) * lda + cbase;
         for (int r = tid; r < nr; r += PT) dst[r] = slab[c * R + r];
@@ -217,54 +325,44 @@ __global__ void __launch_bounds__(PT, 1)
 }
 
 // The interchanges of one panel (M rows k0 .. k0+kb-1 with ipvt) as one
-// composite permutation, by warp 0: after it, panel position k0+t holds the
-// value that was at psrc[t], and outside position odst[e] (>= r0) the value
-// that was at osrc[e] (a panel position, or odst[e] itself when the value went
-// out and came back).  pv: the panel's ipvt entries in shared memory.
+// composite permutation: after it, panel position k0+t holds the value that
+// was at psrc[t], and outside position odst[e] (>= r0) the value that was at
+// osrc[e].  Every position is traced back through the interchanges by a thread
+// of its own, the outside ones (distinct ipvt values beyond the panel) by the
+// first step that names them.  pv: the panel's ipvt entries in shared memory;
+// all threads of the block.
 __device__ void build_perm(const int* pv, int k0, int kb, int r0, int* psrc, int* odst, int* osrc, int* s_nout) {
-    const int lane = threadIdx.x & 31;
-    for (int t = lane; t < kb; t += 32) psrc[t] = k0 + t;
-    __syncwarp();
-    int nout = 0;
-    for (int kk = 0; kk < kb; kk++) {
-        const int p = pv[kk];
-        if (p == k0 + kk) continue;
-        if (p < r0) {
-            if (lane == 0) {
-                const int t = psrc[kk];
-                psrc[kk] = psrc[p - k0];
-                psrc[p - k0] = t;
-            }
-        } else {
-            int found = nout;
-            for (int e0 = 0; e0 < nout; e0 += 32) {
-                const int e = e0 + lane;
-                const unsigned hit = __ballot_sync(0xffffffffu, e < nout && odst[e] == p);
-                if (hit != 0u) {
-                    found = e0 + __ffs(hit) - 1;
-                    break;
-                }
-            }
-            if (lane == 0) {
-                if (found == nout) odst[found] = p, osrc[found] = p;
-                const int t = psrc[kk];
-                psrc[kk] = osrc[found];
-                osrc[found] = t;
-            }
-            if (found == nout) nout++;
+    auto trace = [&](int pos) {
+        for (int kk = kb - 1; kk >= 0; kk--) {
+            const int p = pv[kk], q = k0 + kk;
+            pos = pos == q ? p : (pos == p ? q : pos);
         }
-        __syncwarp();
+        return pos;
+    };
+    for (int t = threadIdx.x; t < kb; t += blockDim.x) psrc[t] = trace(k0 + t);
+    if (threadIdx.x < 32) {
+        int nout = 0;
+        for (int b = 0; b < kb; b += 32) {
+            const int t = b + threadIdx.x;
+            bool first = t < kb && pv[t] >= r0;
+            for (int u = 0; first && u < t; u++) first = pv[u] != pv[t];
+            const unsigned who = __ballot_sync(0xffffffffu, first);
+            if (first) odst[nout + __popc(who & ((1u << threadIdx.x) - 1u))] = pv[t];
+            nout += __popc(who);
+        }
+        if (threadIdx.x == 0) *s_nout = nout;
     }
-    if (lane == 0) *s_nout = nout;
+    __syncthreads();
+    for (int e = threadIdx.x; e < *s_nout; e += blockDim.x) osrc[e] = trace(odst[e]);
 }
 
-// Trailing storage rows c >= r0 (M's trailing columns): interchanges, then
+// Trailing storage rows [r0 + first, r0 + last) (M's trailing columns): interchanges, then
 // x_t += L[k][t] x_k (t > k) with the panel's unit lower block, written in
 // place and transposed into at (at[t * ldat + c - r0]).  One warp per row.
 template <int PB>
 __global__ void __launch_bounds__(PT)
-    k_piv_rows(float* __restrict__ a, int lda, int n, int k0, const int* __restrict__ ipvt, float* __restrict__ at,
-               int ldat) {
+    k_piv_rows(float* __restrict__ a, int lda, int k0, int first, int last, const int* __restrict__ ipvt,
+               float* __restrict__ at, int ldat) {
     constexpr int Q = PB / 32, SS = PB + 4;
     extern __shared__ float sm[];
     float* L = sm;               // L[k * PB + t] = S[k0 + k][k0 + t]
@@ -272,7 +370,7 @@ __global__ void __launch_bounds__(PT)
     __shared__ int pv[PB], psrc[PB], odst[PB], osrc[PB];
     __shared__ int s_nout;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int r0 = k0 + PB, m = n - r0;
+    const int r0 = k0 + PB;
     for (int t = tid; t < PB; t += PT) pv[t] = ipvt[k0 + t];
     for (int idx = tid; idx < PB * PB; idx += PT) {
         const int k = idx / PB, t = idx - k * PB;
@@ -280,12 +378,12 @@ __global__ void __launch_bounds__(PT)
     }
     cp_async_wait_all();
     __syncthreads();
-    if (warp == 0) build_perm(pv, k0, PB, r0, psrc, odst, osrc, &s_nout);
+    build_perm(pv, k0, PB, r0, psrc, odst, osrc, &s_nout);
     __syncthreads();
     const int nout = s_nout;
-    for (int base = blockIdx.x * 8; base < m; base += gridDim.x * 8) {
+    for (int base = first + blockIdx.x * 8; base < last; base += gridDim.x * 8) {
         const int c = r0 + base + warp;
-        if (c < n) {
+        if (base + warp < last) {
             float* row = a + (size_t)c * lda;
             float x[Q], ov[Q];
 #pragma unroll
@@ -318,30 +416,30 @@ __global__ void __launch_bounds__(PT)
         __syncthreads();
         for (int idx = tid; idx < PB * 8; idx += PT) {
             const int t = idx >> 3, j = idx & 7;
-            if (base + j < m) at[(size_t)t * ldat + base + j] = stage[j * SS + t];
+            if (base + j < last) at[(size_t)t * ldat + base + j] = stage[j * SS + t];
         }
         __syncthreads();
     }
 }
 
 // One composite permutation per panel (layout: psrc[PB], odst[PB], osrc[PB],
-// count at [3 PB]), one warp per panel.
+// count at [3 PB]), one block per panel.
 template <int PB>
 __global__ void k_piv_desc(const int* __restrict__ ipvt, int n, int* __restrict__ desc) {
     __shared__ int pv[PB], psrc[PB], odst[PB], osrc[PB];
     __shared__ int s_nout;
-    const int j = blockIdx.x, k0 = j * PB, kb = min(PB, n - k0), lane = threadIdx.x;
-    for (int t = lane; t < kb; t += 32) pv[t] = ipvt[k0 + t];
-    __syncwarp();
+    const int j = blockIdx.x, k0 = j * PB, kb = min(PB, n - k0);
+    for (int t = threadIdx.x; t < kb; t += blockDim.x) pv[t] = ipvt[k0 + t];
+    __syncthreads();
     build_perm(pv, k0, kb, k0 + kb, psrc, odst, osrc, &s_nout);
-    __syncwarp();
+    __syncthreads();
     int* d = desc + (size_t)j * 4 * PB;
-    for (int t = lane; t < PB; t += 32) {
+    for (int t = threadIdx.x; t < PB; t += blockDim.x) {
         d[t] = t < kb ? psrc[t] : k0 + t;
         d[PB + t] = odst[t];
         d[2 * PB + t] = osrc[t];
     }
-    if (lane == 0) d[3 * PB] = s_nout;
+    if (threadIdx.x == 0) d[3 * PB] = s_nout;
 }
 
 // Between block form (whole panel rows exchanged inside a panel) and the
@@ -376,20 +474,40 @@ __global__ void k_piv_convert(float* __restrict__ a, int lda, int n, int pb, con
     }
 }
 
-// acc + sgn * sum_{t < kb} ys[t] * S[k0 + t][i] in ascending t, the column
-// read 16 rows at a time with all 16 loads in flight before they are used.
-__device__ __forceinline__ float panel_dot(const float* __restrict__ a, int lda, int k0, int kb, int i,
-                                           const float* ys, float sgn, float acc) {
-    const float* col = a + (size_t)k0 * lda + i;
-    for (int t0 = 0; t0 < kb; t0 += 16) {
-        float v[16];
+// One warp's share of the products with a block's rows: the sums over rows
+// [16 part, +16) of ys[t] S[k0 + t][i], lane = column; all 16 loads in flight
+// before they are used.
+struct DotRows {
+    float v[16];
+    __device__ __forceinline__ void load(const float* __restrict__ a, int lda, int k0, int kb, int part, int i, bool in) {
+        const float* col = a + (size_t)(k0 + 16 * part) * lda + i;
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = t0 + j < kb ? __ldg(col + (size_t)(t0 + j) * lda) : 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; j++)
-            if (t0 + j < kb) acc = fmaf(sgn * ys[t0 + j], v[j], acc);
+        for (int j = 0; j < 16; j++) v[j] = in && 16 * part + j < kb ? __ldg(col + (size_t)j * lda) : 0.0f;
     }
-    return acc;
+    __device__ __forceinline__ float dot(const float* ys) const {
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; j++) s = fmaf(ys[j], v[j], s);
+        return s;
+    }
+};
+
+// The block's diagonal block into D (row stride PB), 16-byte copies where the
+// rows allow them (k0 is a multiple of PB).
+template <int PB>
+__device__ __forceinline__ void stage_diag(float* D, const float* __restrict__ a, int lda, int k0, int kb, bool vec) {
+    const float* src = a + (size_t)k0 * lda + k0;
+    if (vec && kb == PB) {
+        for (int idx = threadIdx.x; idx < PB * PB / 4; idx += PT) {
+            const int k = idx / (PB / 4), t = (idx % (PB / 4)) * 4;
+            cp_async_vec16(D + k * PB + t, src + (size_t)k * lda + t);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < kb * kb; idx += PT) {
+            const int k = idx / kb, t = idx - k * kb;
+            cp_async4(D + k * PB + t, src + (size_t)k * lda + t);
+        }
+    }
 }
 
 // Forward and back substitution on block-form factors, nrhs right-hand
@@ -397,16 +515,20 @@ __device__ __forceinline__ float panel_dot(const float* __restrict__ a, int lda,
 // values y, two alternating trailing vectors).  Per panel every CTA computes
 // the block's values itself (warp 0, from the diagonal block staged in
 // shared memory), then updates its share of the positions after (forward) or
-// before (backward) the block; one grid barrier per panel.
+// before (backward) the block; one grid barrier per panel.  A chain of two
+// panels' work per barrier, so latency counts: the next diagonal block is
+// copied in and the first products' rows are loaded before the barrier, and
+// the 128 terms of a position are split over eight warps (n = 5000: 2.46 ms ->
+// 1.02; one thread per position and 40 CTAs before).
 template <int PB>
 __global__ void __launch_bounds__(PT, 1)
     k_piv_gesl(const float* __restrict__ a, int lda, int n, const int* __restrict__ desc, float* b, int ldb, int nrhs,
                float* w, unsigned char* __restrict__ sync) {
-    constexpr int Q = PB / 32;
-    extern __shared__ float sm[];
-    float* D = sm;                                      // D[k * PB + t] = S[k0 + k][k0 + t]
-    int* ovr = reinterpret_cast<int*>(D + PB * PB);     // this CTA's positions: override source or -1
-    __shared__ float ys[PB];
+    constexpr int Q = PB / 32, NP = PB / 16;  // NP warps share the terms of a position (the others idle there)
+    extern __shared__ __align__(16) float sm[];
+    float* Dbuf = sm;                                     // 2 x PB x PB diagonal blocks, alternating
+    int* ovr = reinterpret_cast<int*>(Dbuf + 2 * PB * PB);  // this CTA's positions: override source or -1
+    __shared__ float ys[PB], part[NP][32], rd[PB];
     __shared__ int od[PB], os[PB];
     __shared__ int ps[PB];
     __shared__ int s_nout;
@@ -414,33 +536,66 @@ __global__ void __launch_bounds__(PT, 1)
     int* err = reinterpret_cast<int*>(sync + 4);
     const int G = gridDim.x, g = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int np = (n + PB - 1) / PB;
+    const bool vec = (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0;
     unsigned nbar = 0;
     float* y = w;
     float* buf0 = w + n;
     float* buf1 = w + 2 * (size_t)n;
+    // this CTA's positions of panel j: [i0, i1) after (forward) or before (backward) the block
+    auto range = [&](int j, bool fwd, int& i0, int& i1) {
+        const int k0 = j * PB, lo = fwd ? min(n, k0 + PB) : 0, hi = fwd ? n : k0, ch = (hi - lo + G - 1) / G;
+        i0 = min(hi, lo + g * ch);
+        i1 = min(hi, i0 + ch);
+    };
+    // dst[i] = src[i] (or its override) + sgn * sum_t ys[t] S[k0 + t][i] over [i0, i1); pre: the first group's rows
+    auto products = [&](int j, int i0, int i1, float sgn, DotRows& pre, const float* src, const int* over, float* dst) {
+        const int k0 = j * PB, kb = min(PB, n - k0);
+        for (int ib = i0; ib < i1; ib += 32) {
+            const int i = ib + lane;
+            if (warp < NP) {
+                if (ib != i0) pre.load(a, lda, k0, kb, warp, i, i < i1);
+                part[warp][lane] = pre.dot(ys + 16 * warp);
+            }
+            __syncthreads();
+            if (warp == 0 && i < i1) {
+                float s = 0.0f;
+#pragma unroll
+                for (int q = 0; q < NP; q++) s += part[q][lane];
+                const int o = over != nullptr ? over[i - i0] : -1;
+                dst[i] = __ldcg(src + (o >= 0 ? o : i)) + sgn * s;
+            }
+            __syncthreads();
+        }
+    };
     for (int q = 0; q < nrhs; q++) {
         float* bq = b + (size_t)q * ldb;
-        // forward: phase j reads cur, writes nxt (positions >= r0) and y (the block)
+        DotRows pre;
+        int i0, i1;
+        // forward: phase j reads cur, writes nxt (positions after the block) and y (the block)
+        stage_diag<PB>(Dbuf, a, lda, 0, min(PB, n), vec);
+        range(0, true, i0, i1);
+        if (warp < NP) pre.load(a, lda, 0, min(PB, n), warp, i0 + lane, i0 + lane < i1);
         for (int j = 0; j < np; j++) {
-            const int k0 = j * PB, kb = min(PB, n - k0), r0 = k0 + kb;
+            const int k0 = j * PB, kb = min(PB, n - k0);
             const float* cur = j == 0 ? bq : ((j & 1) ? buf0 : buf1);
             float* nxt = (j & 1) ? buf1 : buf0;
+            const float* D = Dbuf + (j & 1) * PB * PB;
             const int* dj = desc + (size_t)j * 4 * PB;
-            for (int t = tid; t < PB; t += PT) ps[t] = dj[t], od[t] = dj[PB + t], os[t] = dj[2 * PB + t];
-            if (tid == 0) s_nout = dj[3 * PB];
-            for (int idx = tid; idx < kb * kb; idx += PT) {
-                const int k = idx / kb, t = idx - k * kb;
-                cp_async4(D + k * PB + t, a + (size_t)(k0 + k) * lda + k0 + t);
+            for (int t = tid; t < PB; t += PT) {
+                ps[t] = dj[t], od[t] = dj[PB + t], os[t] = dj[2 * PB + t];
+                ys[t] = 0.0f;
             }
+            if (tid == 0) s_nout = dj[3 * PB];
             cp_async_wait_all();
-            const int mrest = n - r0, ch = (mrest + G - 1) / G, i0 = r0 + g * ch, i1 = min(n, i0 + ch);
-            for (int i = tid; i < ch; i += PT) ovr[i] = -1;
+            for (int i = tid; i < i1 - i0; i += PT) ovr[i] = -1;
             __syncthreads();
             const int nout = s_nout;
             for (int e = tid; e < nout; e += PT) {
                 const int d = od[e];
                 if (d >= i0 && d < i1) ovr[d - i0] = os[e];
             }
+            // the next diagonal block on its way: the forward sweep's, or the backward sweep's first (this last one)
+            if (j + 1 < np) stage_diag<PB>(Dbuf + ((j + 1) & 1) * PB * PB, a, lda, k0 + PB, min(PB, n - k0 - PB), vec);
             if (warp == 0) {
                 float x[Q];
 #pragma unroll
@@ -467,20 +622,28 @@ __global__ void __launch_bounds__(PT, 1)
                 }
             }
             __syncthreads();
-            for (int i = i0 + tid; i < i1; i += PT) {
-                const int o = ovr[i - i0];
-                nxt[i] = panel_dot(a, lda, k0, kb, i, ys, 1.0f, __ldcg(cur + (o >= 0 ? o : i)));
+            products(j, i0, i1, 1.0f, pre, cur, ovr, nxt);
+            if (j + 1 < np) {
+                range(j + 1, true, i0, i1);
+                if (warp < NP) pre.load(a, lda, k0 + PB, min(PB, n - k0 - PB), warp, i0 + lane, i0 + lane < i1);
+            } else {
+                range(np - 1, false, i0, i1);
+                if (warp < NP) pre.load(a, lda, k0, kb, warp, i0 + lane, i0 + lane < i1);
             }
             if (!grid_sync(bar, (++nbar) * (unsigned)G, err)) return;
         }
-        // backward: x_k = y_k / u_kk; y_t -= x_k u_tk (t < k)
+        // backward: x_k = y_k / u_kk; y_t -= x_k u_tk (t < k).  Block j's diagonal block is in buffer j & 1, as in
+        // the forward sweep; the last one is still there.
         for (int j = np - 1; j >= 0; j--) {
             const int k0 = j * PB, kb = min(PB, n - k0);
-            for (int idx = tid; idx < kb * kb; idx += PT) {
-                const int k = idx / kb, t = idx - k * kb;
-                cp_async4(D + k * PB + t, a + (size_t)(k0 + k) * lda + k0 + t);
-            }
+            const float* D = Dbuf + (j & 1) * PB * PB;
             cp_async_wait_all();
+            __syncthreads();
+            for (int t = tid; t < PB; t += PT) {
+                ys[t] = 0.0f;
+                rd[t] = t < kb ? __frcp_rn(D[t * PB + t]) : 0.0f;
+            }
+            if (j > 0) stage_diag<PB>(Dbuf + ((j - 1) & 1) * PB * PB, a, lda, k0 - PB, PB, vec);
             __syncthreads();
             if (warp == 0) {
                 float x[Q];
@@ -492,7 +655,12 @@ __global__ void __launch_bounds__(PT, 1)
 #pragma unroll
                 for (int k = PB - 1; k >= 0; k--) {
                     if (k < kb) {
-                        const float xk = __shfl_sync(0xffffffffu, x[k >> 5], k & 31) / D[k * PB + k];
+                        // the quotient: the product with the reciprocal and one correction; where that is not finite
+                        // (a zero or infinite pivot, overflow) the division itself
+                        const float v = __shfl_sync(0xffffffffu, x[k >> 5], k & 31), d = D[k * PB + k], r = rd[k];
+                        const float q0 = v * r;
+                        float xk = fmaf(fmaf(-q0, d, v), r, q0);
+                        if (!(fabsf(xk) < 3.0e38f)) xk = v / d;
                         if (lane == (k & 31)) x[k >> 5] = xk;
 #pragma unroll
                         for (int qq = 0; qq < Q; qq++) {
@@ -511,8 +679,11 @@ __global__ void __launch_bounds__(PT, 1)
                 }
             }
             __syncthreads();
-            const int ch = (k0 + G - 1) / G, i0 = g * ch, i1 = min(k0, i0 + ch);
-            for (int i = i0 + tid; i < i1; i += PT) y[i] = panel_dot(a, lda, k0, kb, i, ys, -1.0f, __ldcg(y + i));
+            products(j, i0, i1, -1.0f, pre, y, nullptr, y);
+            if (j > 0) {
+                range(j - 1, false, i0, i1);
+                if (warp < NP) pre.load(a, lda, k0 - PB, PB, warp, i0 + lane, i0 + lane < i1);
+            }
             if (!grid_sync(bar, (++nbar) * (unsigned)G, err)) return;
         }
     }
@@ -550,7 +721,7 @@ int piv_init_attrs() {
 size_t piv_sync_bytes() { return kSyncBytes; }
 
 int piv_panel_width(int n, int sms) {
-    const long long rows = (n + sms - 1) / sms;
+    const long long rows = ((n + sms - 1) / sms + 3) / 4 * 4;
     return rows * 128 * (long long)sizeof(float) <= g_panel_smem_max ? 128 : 64;
 }
 
@@ -558,40 +729,35 @@ int piv_panel_width(int n, int sms) {
 // rows per CTA, at most one CTA per SM, the slice within shared memory.
 static void panel_grid(int m, int kb, int sms, int* G, int* R) {
     int g = std::min(sms, std::max(1, (m + 127) / 128));
-    int r = (m + g - 1) / g;
-    while ((long long)r * kb * (long long)sizeof(float) > g_panel_smem_max && g < sms) {
-        g = std::min(sms, g * 2);
-        r = (m + g - 1) / g;
-    }
-    *G = g;
-    *R = r;
+    auto rows = [&]() { return ((m + g - 1) / g + 3) / 4 * 4; };
+    while ((long long)rows() * kb * (long long)sizeof(float) > g_panel_smem_max && g < sms) g = std::min(sms, g * 2);
+    *R = rows();
+    *G = (m + *R - 1) / *R;
 }
 
-int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, unsigned* bar_base,
-                     int sms, cudaStream_t st) {
+int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, int sms,
+                     cudaStream_t st) {
     const int m = n - k0;
     int G = 0, R = 0;
     panel_grid(m, kb, sms, &G, &R);
     const size_t smem = (size_t)kb * R * sizeof(float);
-    if (kb > PBMAX || G > GMAX || (long long)smem > g_panel_smem_max)
+    if (kb > PBMAX || G > GMAX || R >= 1 << kKeyRowBits || n >= 1 << kKeyTagBits || (long long)smem > g_panel_smem_max)
         return fail(LP_E_INVALID, "pivoting panel: matrix too large for the panel width");
-    unsigned base = *bar_base;
-    void* args[] = {&a, &lda, &n, &k0, &kb, &R, &ipvt, &sync, &base};
+    void* args[] = {&a, &lda, &n, &k0, &kb, &R, &ipvt, &sync};
     LP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_piv_panel), dim3(G), dim3(PT), args, smem, st));
     count_launch();
-    *bar_base = base + (unsigned)G * (unsigned)kb;
     return LP_OK;
 }
 
-int launch_piv_rows(float* a, int lda, int n, int k0, int pb, const int* ipvt, float* at, int ldat, int sms,
-                    cudaStream_t st) {
-    const int m = n - k0 - pb;
-    if (m <= 0) return LP_OK;
-    const int grid = std::max(1, std::min(2 * sms, (m + 7) / 8));
+// Storage rows [r0 + first, r0 + last) of the trailing matrix, r0 = k0 + pb.
+int launch_piv_rows(float* a, int lda, int k0, int pb, int first, int last, const int* ipvt, float* at, int ldat,
+                    int sms, cudaStream_t st) {
+    if (last <= first) return LP_OK;
+    const int grid = std::max(1, std::min(2 * sms, (last - first + 7) / 8));
     if (pb == 128)
-        k_piv_rows<128><<<grid, PT, rows_smem<128>(), st>>>(a, lda, n, k0, ipvt, at, ldat);
+        k_piv_rows<128><<<grid, PT, rows_smem<128>(), st>>>(a, lda, k0, first, last, ipvt, at, ldat);
     else
-        k_piv_rows<64><<<grid, PT, rows_smem<64>(), st>>>(a, lda, n, k0, ipvt, at, ldat);
+        k_piv_rows<64><<<grid, PT, rows_smem<64>(), st>>>(a, lda, k0, first, last, ipvt, at, ldat);
     count_launch();
     LP_CUDA(cudaGetLastError());
     return LP_OK;
@@ -600,9 +766,9 @@ int launch_piv_rows(float* a, int lda, int n, int k0, int pb, const int* ipvt, f
 int launch_piv_desc(const int* ipvt, int n, int pb, int* desc, cudaStream_t st) {
     const int np = (n + pb - 1) / pb;
     if (pb == 128)
-        k_piv_desc<128><<<np, 32, 0, st>>>(ipvt, n, desc);
+        k_piv_desc<128><<<np, 128, 0, st>>>(ipvt, n, desc);
     else
-        k_piv_desc<64><<<np, 32, 0, st>>>(ipvt, n, desc);
+        k_piv_desc<64><<<np, 128, 0, st>>>(ipvt, n, desc);
     count_launch();
     LP_CUDA(cudaGetLastError());
     return LP_OK;
@@ -617,8 +783,8 @@ int launch_piv_convert(float* a, int lda, int n, int pb, const int* ipvt, bool t
 
 int launch_piv_gesl(const float* a, int lda, int n, int pb, const int* desc, float* b, int ldb, int nrhs, float* w,
                     unsigned char* sync, int sms, cudaStream_t st) {
-    const int G = std::max(1, std::min(sms, (n + 127) / 128));
-    const size_t smem = sizeof(float) * (size_t)pb * pb + sizeof(int) * (size_t)((n + G - 1) / G);
+    const int G = std::max(1, std::min(sms, (n + 31) / 32));
+    const size_t smem = sizeof(float) * 2 * (size_t)pb * pb + sizeof(int) * (size_t)((n + G - 1) / G);
     if ((long long)smem > g_gesl_smem_max) return fail(LP_E_INVALID, "pivoting solve: matrix too large");
     void* args[] = {&a, &lda, &n, &desc, &b, &ldb, &nrhs, &w, &sync};
     const void* fn = pb == 128 ? reinterpret_cast<const void*>(k_piv_gesl<128>)

@@ -115,10 +115,10 @@ int gesl_f64_on_f32(lp_ctx* c, const float* a, int n, int lda, double* b, int nr
 int piv_init_attrs();
 size_t piv_sync_bytes();
 int piv_panel_width(int n, int sms);
-int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, unsigned* bar_base,
-                     int sms, cudaStream_t st);
-int launch_piv_rows(float* a, int lda, int n, int k0, int pb, const int* ipvt, float* at, int ldat, int sms,
-                    cudaStream_t st);
+int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, int sms,
+                     cudaStream_t st);
+int launch_piv_rows(float* a, int lda, int k0, int pb, int first, int last, const int* ipvt, float* at, int ldat,
+                    int sms, cudaStream_t st);
 int launch_piv_desc(const int* ipvt, int n, int pb, int* desc, cudaStream_t st);
 int launch_piv_convert(float* a, int lda, int n, int pb, const int* ipvt, bool to_reference, cudaStream_t st);
 int launch_piv_gesl(const float* a, int lda, int n, int pb, const int* desc, float* b, int ldb, int nrhs, float* w,

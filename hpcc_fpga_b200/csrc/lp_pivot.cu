@@ -34,7 +34,10 @@ int piv_validate(const void* a, int n, int lda, const char* who) {
 }  // namespace
 
 // Factorization in block form (interchanges applied to whole panel rows
-// inside each panel); ipvt receives the pivots.  pb: the panel width.
+// inside each panel); ipvt receives the pivots.  pb: the panel width.  One step
+// of look-ahead: the next panel's storage rows are updated first, then that
+// panel, a latency-bound chain on at most one CTA per 128 rows, runs on the
+// high-priority auxiliary stream beside the update of the rest.
 int gefa_pvt_block(lp_ctx* c, float* a, int n, int lda, int* ipvt, int pb, cudaStream_t st) {
     if (n > 128 && !aligned16(a)) return fail(LP_E_INVALID, "pivoting LU: matrix must be 16-byte aligned");
     const int ldat = (n + 3) / 4 * 4;
@@ -42,21 +45,34 @@ int gefa_pvt_block(lp_ctx* c, float* a, int n, int lda, int* ipvt, int pb, cudaS
     LP_CHECK(c->pat.ensure(sizeof(float) * (size_t)pb * ldat));
     unsigned char* sync = static_cast<unsigned char*>(c->psync.ptr);
     float* at = static_cast<float*>(c->pat.ptr);
-    LP_CUDA(cudaMemsetAsync(sync, 0, 16, st));
-    unsigned bar_base = 0;
-    for (int k0 = 0; k0 < n; k0 += pb) {
-        const int kb = std::min(pb, n - k0), r0 = k0 + kb, m = n - k0, rest = n - r0;
+    LP_CUDA(cudaMemsetAsync(sync, 0, piv_sync_bytes(), st));
+    auto panel = [&](int k0, cudaStream_t s) -> int {
+        const int m = n - k0, kb = std::min(pb, m);
+        const int e = prof_begin(c, s);
+        LP_CHECK(launch_piv_panel(a, lda, n, k0, kb, ipvt, sync, c->num_sms, s));
+        return prof_end(c, s, LP_STAGE_LU, e, (double)m * kb * kb, 8.0 * m * kb);
+    };
+    // storage rows [r0 + first, r0 + last): interchanges, block row, trailing update
+    auto update = [&](int k0, int first, int last) -> int {
+        const int r0 = k0 + pb, rest = n - r0, m = last - first;
         int e = prof_begin(c, st);
-        LP_CHECK(launch_piv_panel(a, lda, n, k0, kb, ipvt, sync, &bar_base, c->num_sms, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_LU, e, (double)m * kb * kb, 8.0 * m * kb));
-        if (rest <= 0) break;
+        LP_CHECK(launch_piv_rows(a, lda, k0, pb, first, last, ipvt, at, rest, c->num_sms, st));
+        LP_CHECK(prof_end(c, st, LP_STAGE_LEFT, e, (double)m * pb * pb, 12.0 * m * pb));
         e = prof_begin(c, st);
-        LP_CHECK(launch_piv_rows(a, lda, n, k0, pb, ipvt, at, rest, c->num_sms, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_LEFT, e, (double)rest * pb * pb, 12.0 * rest * pb));
-        e = prof_begin(c, st);
-        LP_CHECK(launch_sgemm_update(a + (size_t)r0 * lda + r0, lda, at, rest, a + (size_t)k0 * lda + r0, lda, rest,
-                                     rest, pb, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * rest * rest * pb, 8.0 * rest * rest));
+        LP_CHECK(launch_sgemm_update(a + (size_t)(r0 + first) * lda + r0, lda, at + first, rest,
+                                     a + (size_t)k0 * lda + r0, lda, m, rest, pb, st));
+        return prof_end(c, st, LP_STAGE_INNER, e, 2.0 * m * rest * pb, 8.0 * m * rest);
+    };
+    LP_CHECK(panel(0, st));
+    for (int k0 = 0; n - k0 > pb; k0 += pb) {
+        const int rest = n - k0 - pb, nx = std::min(pb, rest);
+        LP_CHECK(update(k0, 0, nx));
+        LP_CUDA(cudaEventRecord(c->ev_fork, st));
+        LP_CUDA(cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
+        LP_CHECK(panel(k0 + pb, c->aux));
+        LP_CUDA(cudaEventRecord(c->ev_join, c->aux));
+        if (rest > nx) LP_CHECK(update(k0, nx, rest));
+        LP_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
     }
     return piv_error(c, st, "pivoting LU");
 }

@@ -37,3 +37,22 @@ def test_streamed_ragged_blocks(ctx, lp, n, bs):
     pa.array[...], pb.array[...] = A, b
     ctx.calculate(pa.array, pb.array, bs)
     assert np.array_equal(pa.array, A1) and np.array_equal(pb.array, b1)
+
+
+@pytest.mark.parametrize("n,nrhs", [(132, 1), (160, 2), (388, 1), (644, 3), (1156, 1)])
+def test_pivoting_panel_edges(ctx, dev, torch_cuda, n, nrhs):
+    """Panels whose last rows or columns do not fill a CTA's slice (its rows are held by fours), on matrices whose
+    every step exchanges rows: the oracle's pivots, and solutions within 8 n eps max|x| of the FP64 ones (the matrix
+    is a scaled permutation plus a perturbation of a third of its norm, so its condition is small)."""
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-0.5, 0.5, (n, n)).astype(np.float32)
+    A[np.arange(n), rng.permutation(n)] += np.float32(np.sqrt(n))
+    B = rng.uniform(-1.0, 1.0, (nrhs, n)).astype(np.float32)
+    dA, dB = dev.put(A), dev.put(B)
+    piv = torch_cuda.empty(n, dtype=torch_cuda.int32, device="cuda")
+    ctx.gefa_pvt(dA.data_ptr(), n, n, piv.data_ptr())
+    ctx.gesl_pvt(dA.data_ptr(), n, n, piv.data_ptr(), dB.data_ptr(), nrhs)
+    ctx.sync()
+    assert np.array_equal(piv.cpu().numpy(), oracle.gefa_pvt(A)[1])
+    want = np.linalg.solve(A.T.astype(np.float64), B.T.astype(np.float64)).T
+    assert np.abs(dev.get(dB) - want).max() <= 8 * n * FLT_EPS * np.abs(want).max()
