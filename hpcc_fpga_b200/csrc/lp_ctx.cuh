@@ -108,6 +108,7 @@ int gesl_clear(lp_ctx* c, cudaStream_t st);
 int gesl_status(lp_ctx* c, cudaStream_t st, const char* who);
 // FP64 form (lp_fp64.cu): factorization and substitution in double.
 int gefa_f64(lp_ctx* c, double* a, int n, int lda, int bs, cudaStream_t st);
+int gesl64_init_attrs();
 int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st);
 // The same substitution in FP64 arithmetic on FP32 factors (widened exactly).
 int gesl_f64_on_f32(lp_ctx* c, const float* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st);

@@ -6,10 +6,10 @@
 // lu, top and left are the float kernels instantiated for double
 // (k_lu.cu, k_trsm.cu: reference operation order, bit-identical on one
 // block); inner is k_dgemm_update.  The substitution below is blocked by 64
-// unknowns, one launch per block and direction: every CTA stages the diagonal
-// block, solves it redundantly (one warp per right-hand side), then updates
-// its share of the other unknowns with the block's rows (a GEMV over
-// contiguous rows, each factor element read once per sweep).
+// unknowns, one launch for both sweeps: every CTA forms a block's values with
+// the inverse of its diagonal block, then updates its share of the other
+// unknowns with the block's rows (a GEMV over contiguous rows, each factor
+// element read once per sweep).
 #include <string>
 
 #include "lp_ctx.cuh"
@@ -18,137 +18,230 @@ namespace lp {
 namespace {
 
 constexpr int SB = 64;       // substitution block
-constexpr int GT = 256;      // threads per CTA; one unknown per thread in the update
+constexpr int GT = 256;      // threads per CTA
 constexpr int RMAX = 16;     // right-hand sides per pass
+constexpr int NW = GT / 32;  // warps; in the updates each takes SB / NW rows of the block
+constexpr int RPW = SB / NW;
+constexpr unsigned kSpinLimit64 = 1u << 22;
 
-// The kb x kb diagonal block into shared memory, every copy in flight before
-// the wait; entries outside it are zero.  FP32 factors (the substitution in
-// FP64 arithmetic on FP32 factors, used by the GMRES refinement) are widened
-// exactly as they are read.
-__device__ __forceinline__ void stage_block(double (*dg)[SB + 1], const double* __restrict__ a, int lda, int k0,
-                                            int kb) {
-    for (int idx = threadIdx.x; idx < SB * SB; idx += GT) {
-        const int r = idx / SB, c = idx - r * SB;
-        if (r < kb && c < kb)
-            cp_async8(&dg[r][c], a + (size_t)(k0 + r) * lda + k0 + c);
-        else
-            dg[r][c] = 0.0;
-    }
-    cp_async_wait_all();
-}
-__device__ __forceinline__ void stage_block(double (*dg)[SB + 1], const float* __restrict__ a, int lda, int k0,
-                                            int kb) {
-    float v[SB * SB / GT];
-#pragma unroll
-    for (int q = 0; q < SB * SB / GT; q++) {  // all loads in flight before the first store
-        const int idx = threadIdx.x + q * GT, r = idx / SB, c = idx - r * SB;
-        v[q] = (r < kb && c < kb) ? __ldg(a + (size_t)(k0 + r) * lda + k0 + c) : 0.0f;
-    }
-#pragma unroll
-    for (int q = 0; q < SB * SB / GT; q++) {
-        const int idx = threadIdx.x + q * GT, r = idx / SB, c = idx - r * SB;
-        dg[r][c] = (double)v[q];
-    }
-}
-
-// acc[r] = sum_{k < kb} coef[r][k] * S[k0 + k][c]: the block's column c, read
-// 16 rows at a time with all 16 loads in flight before they are used.
+// The inverses of both triangles of every SB x SB diagonal block D (encoded
+// factors, read as double; a ragged last block padded with the identity):
+// op[2j] = (I - strict-upper(D))^-1, op[2j + 1] = (diag(D_kk)^-1 -
+// strict-lower(D))^-1, so that the block's 64 dependent steps become one
+// product.  One CTA per block: the four 32 x 32 triangles by one warp each
+// (lane = column), then the 32 x 32 blocks joining them.
 template <typename FT>
-__device__ __forceinline__ void block_gemv(const FT* __restrict__ a, int lda, int k0, int kb, int c,
-                                           const double (*coef)[SB], int nrhs, double (&acc)[RMAX]) {
-#pragma unroll
-    for (int r = 0; r < RMAX; r++) acc[r] = 0.0;
-    const FT* col = a + (size_t)k0 * lda + c;
-    for (int kc = 0; kc < kb; kc += 16) {
-        double v[16];
-#pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = kc + j < kb ? (double)__ldg(col + (size_t)(kc + j) * lda) : 0.0;
-#pragma unroll
-        for (int r = 0; r < RMAX; r++)
-            if (r < nrhs)
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (kc + j < kb) acc[r] = fma(coef[r][kc + j], v[j], acc[r]);
+__global__ void __launch_bounds__(128) k_inv64(const FT* __restrict__ a, int lda, int n, double* __restrict__ op) {
+    extern __shared__ __align__(16) double ism[];
+    double(*D)[SB + 1] = reinterpret_cast<double(*)[SB + 1]>(ism);
+    double(*T)[33] = reinterpret_cast<double(*)[33]>(ism + SB * (SB + 1));  // two 32 x 32 products
+    const int j = blockIdx.x, k0 = j * SB, kb = min(SB, n - k0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int idx = tid; idx < SB * SB; idx += 128) {
+        const int r = idx / SB, c = idx % SB;
+        D[r][c] = r < kb && c < kb ? (double)a[(size_t)(k0 + r) * lda + k0 + c] : (r == c ? 1.0 : 0.0);
     }
-}
-
-// forward: y_i += y_k S[k][i] (i > k).  w1: accumulating values (all
-// unknowns), w2: solved values of the block.
-template <typename FT>
-__global__ void __launch_bounds__(GT) k_gesl64_fwd(const FT* __restrict__ a, int lda, int n, double* w1,
-                                                   double* w2, int ldw, int nrhs, int k0) {
-    __shared__ double dg[SB][SB + 1];
-    __shared__ double ys[RMAX][SB];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kb = min(SB, n - k0);
-    stage_block(dg, a, lda, k0, kb);
     __syncthreads();
-    for (int r = warp; r < nrhs; r += GT / 32) {
-        double v0 = lane < kb ? w1[(size_t)r * ldw + k0 + lane] : 0.0;
-        double v1 = lane + 32 < kb ? w1[(size_t)r * ldw + k0 + lane + 32] : 0.0;
-        for (int k = 0; k < kb; k++) {
-            const double yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
-            if (lane > k) v0 = fma(yk, dg[k][lane], v0);
-            if (lane + 32 > k) v1 = fma(yk, dg[k][lane + 32], v1);
-        }
-        ys[r][lane] = v0;
-        ys[r][lane + 32] = v1;
-        if (blockIdx.x == 0) {
-            if (lane < kb) w2[(size_t)r * ldw + k0 + lane] = v0;
-            if (lane + 32 < kb) w2[(size_t)r * ldw + k0 + lane + 32] = v1;
+    double* Y = op + (size_t)(2 * j) * SB * SB;
+    double* X = Y + SB * SB;
+    const int o = 32 * (warp & 1);  // warps 0, 1: Y's diagonal blocks, 2, 3: X's
+    double x[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) x[r] = r == lane ? 1.0 : 0.0;
+    if (warp < 2) {
+#pragma unroll
+        for (int k = 31; k > 0; k--)
+#pragma unroll
+            for (int r = 0; r < k; r++) x[r] = fma(D[o + r][o + k], x[k], x[r]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 32; k++) {
+            x[k] *= D[o + k][o + k];
+#pragma unroll
+            for (int r = k + 1; r < 32; r++) x[r] = fma(D[o + r][o + k], x[k], x[r]);
         }
     }
-    __syncthreads();
-    const int c = k0 + kb + blockIdx.x * GT + threadIdx.x;
-    if (c >= n) return;
-    double acc[RMAX];
-    block_gemv(a, lda, k0, kb, c, ys, nrhs, acc);
+    double* out = warp < 2 ? Y : X;
 #pragma unroll
-    for (int r = 0; r < RMAX; r++)
-        if (r < nrhs) w1[(size_t)r * ldw + c] += acc[r];
-}
-
-// backward: s = y_k S[k][k]; x_k = -s; y_i += s S[k][i] (i < k).  w2: values
-// (updated in place for the unknowns before the block), out: solutions.
-template <typename FT>
-__global__ void __launch_bounds__(GT) k_gesl64_bwd(const FT* __restrict__ a, int lda, int n, double* w2, int ldw,
-                                                   double* out, int ldo, int nrhs, int k0) {
-    __shared__ double dg[SB][SB + 1];
-    __shared__ double ss[RMAX][SB];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kb = min(SB, n - k0);
-    stage_block(dg, a, lda, k0, kb);
+    for (int r = 0; r < 32; r++) out[(o + r) * SB + o + lane] = x[r];
+    // the blocks beside them: Y01 = Y00 U01 Y11 and X10 = X11 L10 X00, Y10 = X01 = 0; both read back (this CTA's
+    // writes) after the barrier, 64 threads each, 16 outputs per thread
     __syncthreads();
-    for (int r = warp; r < nrhs; r += GT / 32) {
-        double v0 = lane < kb ? w2[(size_t)r * ldw + k0 + lane] : 0.0;
-        double v1 = lane + 32 < kb ? w2[(size_t)r * ldw + k0 + lane + 32] : 0.0;
-        for (int k = kb - 1; k >= 0; k--) {
-            const double yk = __shfl_sync(0xffffffffu, k < 32 ? v0 : v1, k & 31);
-            const double s = yk * dg[k][k];
-            if (lane == (k & 31)) {
-                if (k < 32)
-                    v0 = -s;
-                else
-                    v1 = -s;
-                ss[r][k] = s;
+    const bool up = tid < 64;
+    const int t = tid & 63, c = t & 31, r0 = 16 * (t >> 5);
+    const int lo = up ? 0 : 32, hi = up ? 32 : 0;  // block (lo, hi) of D and of the inverse
+    const double* in = up ? Y : X;
+    double s[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) s[q] = 0.0;
+    for (int k = 0; k < 32; k++) {
+        const double v = in[(hi + k) * SB + hi + c];
+#pragma unroll
+        for (int q = 0; q < 16; q++) s[q] = fma(D[lo + r0 + q][hi + k], v, s[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) T[(up ? 0 : 32) + r0 + q][c] = s[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; q++) s[q] = 0.0;
+    for (int k = 0; k < 32; k++) {
+        const double v = T[(up ? 0 : 32) + k][c];
+#pragma unroll
+        for (int q = 0; q < 16; q++) s[q] = fma(in[(lo + r0 + q) * SB + lo + k], v, s[q]);
+    }
+    double* w = up ? Y : X;
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+        w[(lo + r0 + q) * SB + hi + c] = s[q];
+        w[(hi + r0 + q) * SB + lo + c] = 0.0;
+    }
+}
+constexpr size_t kInv64Smem = sizeof(double) * (SB * (SB + 1) + 64 * 33);
+
+// Bounded grid barrier of a cooperative launch; the counter only grows.
+__device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, int* err) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        int ok = 1;
+        unsigned spins = 0, v;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if (v >= target) break;
+            if ((++spins & 255u) == 0 && (*reinterpret_cast<volatile int*>(err) != 0 || spins > kSpinLimit64)) {
+                atomicExch(err, 1);
+                ok = 0;
+                break;
             }
-            if (lane < k) v0 = fma(s, dg[k][lane], v0);
-            if (lane + 32 < k) v1 = fma(s, dg[k][lane + 32], v1);
         }
-        if (blockIdx.x == 0) {
-            if (lane < kb) out[(size_t)r * ldo + k0 + lane] = v0;
-            if (lane + 32 < kb) out[(size_t)r * ldo + k0 + lane + 32] = v1;
-        }
+        __threadfence();
+        s_ok = ok;
     }
     __syncthreads();
-    const int c = blockIdx.x * GT + threadIdx.x;
-    if (c >= k0) return;
-    double acc[RMAX];
-    block_gemv(a, lda, k0, kb, c, ss, nrhs, acc);
-#pragma unroll
-    for (int r = 0; r < RMAX; r++)
-        if (r < nrhs) w2[(size_t)r * ldw + c] += acc[r];
+    return s_ok != 0;
 }
+
+// Forward and back substitution of one group of right-hand sides (rows of b,
+// overwritten by the solutions), one cooperative launch.  Per block of SB
+// unknowns every CTA forms the block's values itself (one product with the
+// block's inverse, copied in before the barrier), then updates its share of
+// the unknowns after (forward) or before (backward) it with rows loaded before
+// the barrier; one barrier per block.  w1, w2: n x nrhs accumulating values of
+// the two sweeps (the forward sweep's results are the second's input).  A
+// chain of 2 n / 64 short steps, where one launch per block and direction took
+// 15 us each (n = 6144: 192 launches, 2.9 ms).  A barrier that gives up leaves
+// NaN in the solutions.
+template <typename FT>
+__global__ void __launch_bounds__(GT, 1)
+    k_gesl64(const FT* __restrict__ a, int lda, int n, const double* __restrict__ op, double* w1, double* w2, double* b,
+             int ldb, int nrhs, unsigned* sync) {
+    extern __shared__ __align__(16) double sm[];
+    double* Ob = sm;                          // 2 x SB x SB: the block's inverse, alternating
+    double* in = Ob + 2 * SB * SB;            // RMAX x SB: the block's accumulated values
+    double* ys = in + RMAX * SB;              // RMAX x SB: its solved values
+    double* part = ys + RMAX * SB;            // NW x 32 x RMAX partial sums
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, g = blockIdx.x;
+    int* err = reinterpret_cast<int*>(sync + 1);
+    const int nblk = (n + SB - 1) / SB, steps = 2 * nblk;
+    // step s: forward block s, then backward blocks nblk - 1 .. 0
+    auto block_of = [&](int s) { return s < nblk ? s : steps - 1 - s; };
+    auto range = [&](int s, int& i0, int& i1) {
+        const int k0 = block_of(s) * SB, lo = s < nblk ? min(n, k0 + SB) : 0, hi = s < nblk ? n : k0;
+        const int ch = (hi - lo + G - 1) / G;
+        i0 = min(hi, lo + g * ch);
+        i1 = min(hi, i0 + ch);
+    };
+    auto stage = [&](int s) {
+        const double* src = op + (size_t)(2 * block_of(s) + (s < nblk ? 0 : 1)) * SB * SB;
+        double* dst = Ob + (s & 1) * SB * SB;
+        for (int idx = tid * 2; idx < SB * SB; idx += GT * 2) cp_async_vec16(dst + idx, src + idx);
+    };
+    double v[RPW];
+    auto load_rows = [&](int s, int i, bool ok) {
+        const int k0 = block_of(s) * SB + RPW * warp;
+#pragma unroll
+        for (int q = 0; q < RPW; q++) v[q] = ok && k0 + q < n ? (double)__ldg(a + (size_t)(k0 + q) * lda + i) : 0.0;
+    };
+    int i0, i1;
+    stage(0);
+    range(0, i0, i1);
+    load_rows(0, i0 + lane, i0 + lane < i1);
+    for (int s = 0; s < steps; s++) {
+        const bool fwd = s < nblk;
+        const int k0 = block_of(s) * SB, kb = min(SB, n - k0);
+        double* w = fwd ? w1 : w2;
+        for (int idx = tid; idx < nrhs * SB; idx += GT) {
+            const int r = idx / SB, i = idx % SB;
+            in[idx] = i < kb ? __ldcg(w + (size_t)r * n + k0 + i) : 0.0;
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        if (s + 1 < steps) stage(s + 1);
+        {  // y_i = sum_k op[k][i] in_k: column i by a quarter of the threads per quarter of k
+            const double* o = Ob + (s & 1) * SB * SB;
+            const int i = tid & (SB - 1), kq = (tid >> 6) * (SB / 4);
+            for (int r = 0; r < nrhs; r++) {
+                double y0 = 0.0, y1 = 0.0;
+#pragma unroll
+                for (int k = 0; k < SB / 4; k += 2) {
+                    y0 = fma(o[(kq + k) * SB + i], in[r * SB + kq + k], y0);
+                    y1 = fma(o[(kq + k + 1) * SB + i], in[r * SB + kq + k + 1], y1);
+                }
+                part[(r * 4 + (tid >> 6)) * SB + i] = y0 + y1;
+            }
+        }
+        __syncthreads();
+        for (int idx = tid; idx < nrhs * SB; idx += GT) {
+            const int r = idx / SB, i = idx % SB;
+            const double* q = part + r * 4 * SB + i;
+            const double y = (q[0] + q[SB]) + (q[2 * SB] + q[3 * SB]);
+            ys[idx] = y;
+            if (g == 0 && i < kb) {
+                if (fwd)
+                    w2[(size_t)r * n + k0 + i] = y;  // (w1's block is still being read by other CTAs)
+                else
+                    b[(size_t)r * ldb + k0 + i] = -y;
+            }
+        }
+        __syncthreads();
+        // unknowns after (forward) or before (backward) the block: += y^T S[block][i]
+        for (int ib = i0; ib < i1; ib += 32) {
+            if (ib != i0) load_rows(s, ib + lane, ib + lane < i1);
+            for (int r = 0; r < nrhs; r++) {
+                const double* y = ys + r * SB + RPW * warp;
+                double t = 0.0;
+#pragma unroll
+                for (int q = 0; q < RPW; q++) t = fma(y[q], v[q], t);
+                part[(r * NW + warp) * 32 + lane] = t;
+            }
+            __syncthreads();
+            for (int idx = tid; idx < nrhs * 32; idx += GT) {
+                const int r = idx >> 5, i = ib + (idx & 31);
+                if (i < i1) {
+                    const double* q = part + r * NW * 32 + (idx & 31);
+                    double t = 0.0;
+#pragma unroll
+                    for (int e = 0; e < NW; e++) t += q[32 * e];
+                    double* p = w + (size_t)r * n + i;
+                    *p = __ldcg(p) + t;
+                }
+            }
+            __syncthreads();
+        }
+        if (s + 1 == steps) break;
+        range(s + 1, i0, i1);
+        load_rows(s + 1, i0 + lane, i0 + lane < i1);
+        if (!grid_sync64(sync, (unsigned)(s + 1) * (unsigned)G, err)) {
+            for (int idx = g * GT + tid; idx < nrhs * n; idx += G * GT)
+                b[(size_t)(idx / n) * ldb + idx % n] = __longlong_as_double(0x7ff8000000000000ll);
+            return;
+        }
+    }
+}
+constexpr size_t kGesl64Smem = sizeof(double) * (2 * SB * SB + 2 * RMAX * SB + (size_t)NW * 32 * RMAX);
+static_assert(4 * SB <= NW * 32, "the block's partial sums share the updates' space");
 
 double event_s64(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0.0f;
@@ -223,60 +316,93 @@ static int left_blocked64(const double* d, int lda, double* l, int ldl, int bs, 
     return LP_OK;
 }
 
+// One step of look-ahead, as gefa_f32: the next block row and column first,
+// then the panel of the next step (a latency-bound chain, top on its stream and
+// left beside it) on the auxiliary stream beside the update of the rest.
 int gefa_f64(lp_ctx* c, double* a, int n, int lda, int bs, cudaStream_t st) {
-    LP_CHECK(c->f64lt.ensure(sizeof(double) * ((size_t)bs * n + (bs > 128 ? 2 * (size_t)128 * bs : 0))));
-    double* lt = static_cast<double*>(c->f64lt.ptr);
-    double* scratch = lt + (size_t)bs * n;  // bs > 128: inner Lt of the lu stage, then transposed D sub-blocks
-    for (int k0 = 0; k0 < n; k0 += bs) {
+    const size_t pan = (size_t)bs * n;
+    LP_CHECK(c->f64lt.ensure(sizeof(double) * (2 * pan + (bs > 128 ? 2 * (size_t)128 * bs : 0))));
+    double* lts[2] = {static_cast<double*>(c->f64lt.ptr), static_cast<double*>(c->f64lt.ptr) + pan};
+    double* scratch = lts[1] + pan;  // bs > 128: inner Lt of the lu stage, then transposed D sub-blocks
+    auto panel = [&](int k0, double* lt, cudaStream_t s) -> int {
         double* d = a + (size_t)k0 * lda + k0;
         const int rest = n - k0 - bs;
-        int e = prof_begin(c, st);
-        LP_CHECK(lu_stage64(d, lda, bs, scratch, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_LU, e, 2.0 * bs * bs * bs / 3.0, 16.0 * bs * bs));
-        if (rest <= 0) break;
-        e = prof_begin(c, st);
-        LP_CHECK(top_blocked64(d, lda, d + bs, lda, bs, rest, scratch, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_TOP, e, (double)bs * bs * rest, 16.0 * bs * rest));
-        e = prof_begin(c, st);
-        LP_CHECK(left_blocked64(d, lda, d + (size_t)bs * lda, lda, bs, rest, lt, rest, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_LEFT, e, (double)bs * bs * rest, 24.0 * bs * rest));
-        e = prof_begin(c, st);
-        LP_CHECK(launch_dgemm_update(d + (size_t)bs * lda + bs, lda, lt, rest, d + bs, lda, rest, rest, bs, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * rest * rest * bs,
-                          8.0 * (2.0 * rest * rest + 2.0 * bs * rest)));
+        int e = prof_begin(c, s);
+        LP_CHECK(lu_stage64(d, lda, bs, scratch, s));
+        LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * bs * bs * bs / 3.0, 16.0 * bs * bs));
+        if (rest <= 0) return LP_OK;
+        LP_CUDA(cudaEventRecord(c->ev_side, s));
+        LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+        e = prof_begin(c, c->aux2);
+        LP_CHECK(left_blocked64(d, lda, d + (size_t)bs * lda, lda, bs, rest, lt, rest, c->aux2));
+        LP_CHECK(prof_end(c, c->aux2, LP_STAGE_LEFT, e, (double)bs * bs * rest, 24.0 * bs * rest));
+        LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
+        e = prof_begin(c, s);
+        LP_CHECK(top_blocked64(d, lda, d + bs, lda, bs, rest, scratch, s));
+        LP_CHECK(prof_end(c, s, LP_STAGE_TOP, e, (double)bs * bs * rest, 16.0 * bs * rest));
+        LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
+        return LP_OK;
+    };
+    auto update = [&](double* cc, const double* lt, const double* t, int rest, int m, int nn) -> int {
+        const int e = prof_begin(c, st);
+        LP_CHECK(launch_dgemm_update(cc, lda, lt, rest, t, lda, m, nn, bs, st));
+        return prof_end(c, st, LP_STAGE_INNER, e, 2.0 * m * nn * bs, 8.0 * (2.0 * m * nn + (double)bs * (m + nn)));
+    };
+    LP_CHECK(panel(0, lts[0], st));
+    for (int k0 = 0, K = 0; k0 + bs < n; k0 += bs, K++) {
+        const int rest = n - k0 - bs;
+        double* top = a + (size_t)k0 * lda + k0 + bs;
+        double* c11 = a + (size_t)(k0 + bs) * lda + k0 + bs;
+        const double* lt = lts[K & 1];
+        LP_CHECK(update(c11, lt, top, rest, bs, rest));
+        if (rest > bs) LP_CHECK(update(c11 + (size_t)bs * lda, lt + bs, top, rest, rest - bs, bs));
+        LP_CUDA(cudaEventRecord(c->ev_fork, st));
+        LP_CUDA(cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
+        LP_CHECK(panel(k0 + bs, lts[(K + 1) & 1], c->aux));
+        LP_CUDA(cudaEventRecord(c->ev_join, c->aux));
+        if (rest > bs)
+            LP_CHECK(update(c11 + (size_t)bs * lda + bs, lt + bs, top + bs, rest, rest - bs, rest - bs));
+        LP_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
     }
     return LP_OK;
 }
 
 template <typename FT>
 static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st) {
-    const int g0 = nrhs < RMAX ? nrhs : RMAX;
-    LP_CHECK(c->f64w.ensure(sizeof(double) * 2 * (size_t)n * g0));
-    double* w1 = static_cast<double*>(c->f64w.ptr);
+    const int g0 = nrhs < RMAX ? nrhs : RMAX, nblk = (n + SB - 1) / SB;
+    const size_t ops = 2 * (size_t)nblk * SB * SB;
+    LP_CHECK(c->f64w.ensure(sizeof(double) * (2 * (size_t)n * g0 + ops + 2)));
+    double* op = static_cast<double*>(c->f64w.ptr);
+    unsigned* sync = reinterpret_cast<unsigned*>(op + ops);  // barrier counter, error word
+    double* w1 = op + ops + 2;
     double* w2 = w1 + (size_t)n * g0;
     const int e = prof_begin(c, st);
-    const int nblk = (n + SB - 1) / SB;
+    k_inv64<FT><<<nblk, 128, kInv64Smem, st>>>(a, lda, n, op);
+    LP_CUDA(cudaGetLastError());
+    count_launch();
+    // enough CTAs that a step's products are one pass of 32 unknowns each, at most one per SM
+    const int grid = std::max(1, std::min(c->num_sms, (n + 31) / 32));
     for (int r0 = 0; r0 < nrhs; r0 += RMAX) {
-        const int g = nrhs - r0 < RMAX ? nrhs - r0 : RMAX;
+        int g = nrhs - r0 < RMAX ? nrhs - r0 : RMAX;
         double* bb = b + (size_t)r0 * ldb;
         LP_CUDA(cudaMemcpy2DAsync(w1, sizeof(double) * n, bb, sizeof(double) * ldb, sizeof(double) * n, g,
                                   cudaMemcpyDeviceToDevice, st));
-        for (int K = 0; K < nblk; K++) {
-            const int k0 = K * SB, rest = n - k0 - std::min(SB, n - k0);
-            const int grid = rest > 0 ? (rest + GT - 1) / GT : 1;
-            k_gesl64_fwd<FT><<<grid, GT, 0, st>>>(a, lda, n, w1, w2, n, g, k0);
-            count_launch();
-        }
-        for (int K = nblk - 1; K >= 0; K--) {
-            const int k0 = K * SB;
-            const int grid = k0 > 0 ? (k0 + GT - 1) / GT : 1;
-            k_gesl64_bwd<FT><<<grid, GT, 0, st>>>(a, lda, n, w2, n, bb, ldb, g, k0);
-            count_launch();
-        }
-        LP_CUDA(cudaGetLastError());
+        LP_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st));
+        void* args[] = {&a, &lda, &n, &op, &w1, &w2, &bb, &ldb, &g, &sync};
+        LP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_gesl64<FT>), dim3(grid), dim3(GT), args,
+                                            kGesl64Smem, st));
+        count_launch();
     }
     return prof_end(c, st, LP_STAGE_GESL, e, 2.0 * n * n * nrhs,
                     (double)sizeof(FT) * n * n * ((nrhs + RMAX - 1) / RMAX));
+}
+
+int gesl64_init_attrs() {
+    LP_CUDA(cudaFuncSetAttribute(k_inv64<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInv64Smem));
+    LP_CUDA(cudaFuncSetAttribute(k_inv64<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInv64Smem));
+    LP_CUDA(cudaFuncSetAttribute(k_gesl64<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGesl64Smem));
+    LP_CUDA(cudaFuncSetAttribute(k_gesl64<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGesl64Smem));
+    return LP_OK;
 }
 
 int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st) {

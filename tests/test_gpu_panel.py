@@ -56,3 +56,22 @@ def test_pivoting_panel_edges(ctx, dev, torch_cuda, n, nrhs):
     assert np.array_equal(piv.cpu().numpy(), oracle.gefa_pvt(A)[1])
     want = np.linalg.solve(A.T.astype(np.float64), B.T.astype(np.float64)).T
     assert np.abs(dev.get(dB) - want).max() <= 8 * n * FLT_EPS * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n,nrhs,pad", [(1, 1, 0), (31, 2, 1), (63, 1, 0), (64, 16, 0), (65, 17, 1), (200, 3, 0),
+                                        (1000, 1, 0), (4801, 2, 3)])
+def test_gesl_f64_edges(ctx, dev, n, nrhs, pad):
+    """The FP64 substitution for orders that are no multiple of its 64 blocks, one to several groups of 16 right-hand
+    sides, padded rows: against numpy's triangular products with the same bound as for the factored systems,
+    1e3 n eps max(1, |x|)."""
+    rng = np.random.default_rng(n)
+    E = np.full((n, n + pad), 3.0)
+    E[:, :n] = rng.uniform(-0.5, 0.5, (n, n))
+    u = n / 4 * rng.uniform(0.99, 1.01, n) + 1.0
+    E[:, :n] = np.tril(E[:, :n], -1) + np.triu(E[:, :n], 1) / u[:, None] - np.diag(1.0 / u)
+    M = (np.eye(n) - np.triu(E[:, :n], 1)).T @ (np.tril(E[:, :n], -1) + np.diag(u)).T  # L U of the encoding
+    want = rng.uniform(-1.0, 1.0, (nrhs, n))
+    dE, dB = dev.put(E), dev.put(np.ascontiguousarray(want @ M.T))
+    ctx.gesl_f64(dE.data_ptr(), n, n + pad, dB.data_ptr(), nrhs)
+    ctx.sync()
+    assert np.abs(dev.get(dB) - want).max() <= 1e3 * n * np.finfo(np.float64).eps
