@@ -17,8 +17,9 @@
 // lanes of a load share addresses or not, and the FMA pipe takes 128 products
 // a clock: R x C outputs per thread cost R + C clocks of loads against R C / 4
 // of products per warp and k.  At 8 x 8 the two are level (and the kernel
-// reached 75 % of the pipe); the wide form takes 8 x 16, 24 against 32.  The
-// small forms trade that for more CTAs (launch_sgemm_update).  Every element
+// reached 75 % of the pipe); the large form takes 8 x 16, 24 against 32
+// (7680^2 x 512 1093 -> 993 us, 60.8 TFLOP/s; x 128 313 -> 274).  The small
+// forms trade that for more CTAs (launch_sgemm_update).  Every element
 // gets the same sum in the same order in each form, so they agree bit for
 // bit.
 #include "lp_common.cuh"
@@ -127,30 +128,33 @@ __global__ void __launch_bounds__(32 * WR * WC, MINB)
     }
     cp_async_wait<0>();
 
+    // four rows' loads in flight before their first store (the compiler keeps a load behind a store to the same array)
 #pragma unroll
-    for (int i = 0; i < R; i++) {
-        const int r = m0 + row + 16 * WR * (i >> 2) + (i & 3);
-        if (r >= M) continue;
+    for (int i0 = 0; i0 < R; i0 += 4) {
+        float4 v[4][CG];
 #pragma unroll
-        for (int j = 0; j < CG; j++) {
-            const int c = n0 + col + 32 * WC * j;
-            if (c >= N) continue;
-            float4* p = reinterpret_cast<float4*>(C + (size_t)r * ldc + c);
-            float4 v = *p;
-            v.x += acc[i][2 * j].x;
-            v.y += acc[i][2 * j].y;
-            v.z += acc[i][2 * j + 1].x;
-            v.w += acc[i][2 * j + 1].y;
-            *p = v;
-        }
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < CG; j++) {
+                const int r = m0 + row + 4 * WR * i0 + i, c = n0 + col + 32 * WC * j;
+                if (r < M && c < N) v[i][j] = *reinterpret_cast<const float4*>(C + (size_t)r * ldc + c);
+            }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < CG; j++) {
+                const int r = m0 + row + 4 * WR * i0 + i, c = n0 + col + 32 * WC * j;
+                if (r < M && c < N)
+                    *reinterpret_cast<float4*>(C + (size_t)r * ldc + c) =
+                        make_float4(v[i][j].x + acc[i0 + i][2 * j].x, v[i][j].y + acc[i0 + i][2 * j].y,
+                                    v[i][j].z + acc[i0 + i][2 * j + 1].x, v[i][j].w + acc[i0 + i][2 * j + 1].y);
+            }
     }
 }
 
-#define LP_WIDE 4, 1, 2, 4, 16, 4    // 128 x 128 tiles, 8 x 16 outputs per thread
-#define LP_LARGE 4, 2, 2, 2, 16, 4   // 128 x 128, 8 x 8
+#define LP_LARGE 4, 1, 2, 4, 16, 4   // 128 x 128 tiles, 8 x 16 outputs per thread
 #define LP_MIDDLE 2, 2, 2, 1, 32, 3  // 64 x 64, 8 x 4
 #define LP_SMALL 2, 1, 1, 1, 32, 4   // 32 x 32, 4 x 4
-using Wide = Form<LP_WIDE>;
 using Large = Form<LP_LARGE>;
 using Middle = Form<LP_MIDDLE>;
 using Small = Form<LP_SMALL>;
@@ -160,8 +164,6 @@ constexpr int kSms = 148;
 }  // namespace
 
 int sgemm_init_attrs() {
-    LP_CUDA(cudaFuncSetAttribute(k_sgemm_update<LP_WIDE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)Wide::smem));
     LP_CUDA(cudaFuncSetAttribute(k_sgemm_update<LP_LARGE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)Large::smem));
     LP_CUDA(cudaFuncSetAttribute(k_sgemm_update<LP_MIDDLE, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -181,9 +183,7 @@ int launch_sgemm_update(float* c, int ldc, const float* lt, int ldlt, const floa
     if ((m + Large::TM - 1) / Large::TM > 65535) return fail(LP_E_INVALID, "inner_update: m too large");
     auto grid = [&](int tm, int tn) { return dim3((n + tn - 1) / tn, (m + tm - 1) / tm); };
     // The form whose busiest SM has the least to do: tiles per SM x clocks per k of a tile (products or loads,
-    // whichever is more: 128, 48, 16).  Of the two 128 x 128 forms the one with 8 x 16 outputs per thread where K
-    // is long enough for its longer epilogue: 7680^2 x 512 1078 -> 1022 us, x 256 559 -> 541, but x 128 297 -> 318,
-    // and below eight waves no gain at 256.
+    // whichever is more: 128, 48, 16).
     auto cost = [&](int tm, int tn, long long clocks) {
         const dim3 g = grid(tm, tn);
         return ((long long)g.x * g.y + kSms - 1) / kSms * clocks;
@@ -191,11 +191,8 @@ int launch_sgemm_update(float* c, int ldc, const float* lt, int ldlt, const floa
     const long long large = cost(Large::TM, Large::TN, 128), middle = cost(Middle::TM, Middle::TN, 48),
                     small = cost(Small::TM, Small::TN, 16);
     if (large <= middle && large <= small) {
-        const dim3 g = grid(Large::TM, Large::TN);
-        if (k >= 512 || (k >= 256 && large >= 8 * 128))
-            k_sgemm_update<LP_WIDE, 2><<<g, Wide::NT, Wide::smem, st>>>(c, ldc, lt, ldlt, t, ldt, m, n, k);
-        else
-            k_sgemm_update<LP_LARGE, 2><<<g, Large::NT, Large::smem, st>>>(c, ldc, lt, ldlt, t, ldt, m, n, k);
+        k_sgemm_update<LP_LARGE, 2><<<grid(Large::TM, Large::TN), Large::NT, Large::smem, st>>>(c, ldc, lt, ldlt, t, ldt, m,
+                                                                                              n, k);
     } else if (middle <= small) {
         LP_CUDA(launch_pdl(k_sgemm_update<LP_MIDDLE, 4>, grid(Middle::TM, Middle::TN), dim3(Middle::NT), Middle::smem, st,
                            c, ldc, lt, ldlt, t, ldt, m, n, k));

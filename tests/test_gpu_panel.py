@@ -75,3 +75,33 @@ def test_gesl_f64_edges(ctx, dev, n, nrhs, pad):
     ctx.gesl_f64(dE.data_ptr(), n, n + pad, dB.data_ptr(), nrhs)
     ctx.sync()
     assert np.abs(dev.get(dB) - want).max() <= 1e3 * n * np.finfo(np.float64).eps
+
+
+@pytest.mark.parametrize("sizes,pad", [([129, 160, 161, 255], 0), ([257, 384, 385, 530], 3), ([641, 1024], 0),
+                                       ([31, 33, 64, 95, 127, 128], 1)])
+def test_batch_tile_edges(ctx, dev, lp, sizes, pad):
+    """Batched systems at the edges of the outer blocks (128), inner panels (32) and unknowns per thread, with rows
+    that allow 16-byte copies and rows that do not, 1 to 16 right-hand sides: factors within 256 eps max(1, |want|)
+    of the oracle's, solutions within 8 n eps max|x| of the FP64 ones (diagonally dominant: condition below 8)."""
+    rhs = [1, 2, 5, 8, 9, 16]
+    systems, mats, a_off, b_off = [], [], 0, 0
+    for k, n in enumerate(sizes):
+        lda = (n + 3) // 4 * 4 + pad
+        systems.append(lp.LpSystem(n, rhs[k % 6], lda, n, a_off, b_off))
+        mats.append(oracle.gen_reference(n)[0])
+        a_off += (n * lda + 3) // 4 * 4
+        b_off += rhs[k % 6] * n
+    A, B = np.zeros(a_off, np.float32), np.random.default_rng(len(sizes)).uniform(-1, 1, b_off).astype(np.float32)
+    for s, m in zip(systems, mats):
+        A[s.a_off:s.a_off + s.n * s.lda].reshape(s.n, s.lda)[:, :s.n] = m
+    dA, dB = dev.put(A), dev.put(B)
+    ctx.batch_solve(systems, dA.data_ptr(), dB.data_ptr())
+    gotA, gotB = dev.get(dA), dev.get(dB)
+    for s, m in zip(systems, mats):
+        f = gotA[s.a_off:s.a_off + s.n * s.lda].reshape(s.n, s.lda)[:, :s.n].astype(np.float64)
+        want = oracle.gefa_nopvt(m).astype(np.float64)
+        assert (np.abs(f - want) / np.maximum(1.0, np.abs(want))).max() < 256 * FLT_EPS, s.n
+        b = B[s.b_off:s.b_off + s.nrhs * s.n].reshape(s.nrhs, s.n).astype(np.float64)
+        x = np.linalg.solve(m.T.astype(np.float64), b.T).T
+        got = gotB[s.b_off:s.b_off + s.nrhs * s.n].reshape(s.nrhs, s.n)
+        assert np.abs(got - x).max() <= 8 * s.n * FLT_EPS * np.abs(x).max(), s.n
