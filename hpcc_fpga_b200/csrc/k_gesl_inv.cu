@@ -50,8 +50,8 @@
 // consumer needs one L2 round trip (no flag, then data).  The forward sweep
 // tags with 1, the backward sweep with 2 into the same array (cleared before
 // the forward sweep); the backward sweep reads its input y_j there.  The
-// summation order is fixed (sources in order, rows in order, chunks in order,
-// fixed two-way reductions), so results are deterministic whichever CTA runs
+// summation order is fixed (sources in order, rows in order within a warp,
+// warps in order, chunks in order), so results are deterministic whichever CTA runs
 // an item.
 #include <algorithm>
 
@@ -372,6 +372,59 @@ __device__ bool resolve_tile(Pending<NR>& pd, const unsigned long long* __restri
     return __syncthreads_and(ok) != 0;
 }
 
+// A thread's sums for four neighbouring columns and NR right-hand sides.
+// Shared memory delivers 128 bytes a clock to the registers, broadcast or not,
+// so the four columns share every value read of the right-hand sides: 4 + NR
+// clocks of loads per row and warp (one column per thread took 4 (1 + NR)).
+template <int NR>
+struct Sums {
+    float2 s[4][NR / 2];  // pairs of right-hand sides
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int q = 0; q < NR / 2; q++) s[c][q] = make_float2(0.0f, 0.0f);
+    }
+    // += v (a row's four columns) * y (its NR values)
+    __device__ __forceinline__ void add(float4 v, const float* y) {
+        const float vc[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int q = 0; q < NR; q += 4) {
+            const float4 u = *reinterpret_cast<const float4*>(y + q);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const float2 vv = make_float2(vc[c], vc[c]);
+                s[c][q / 2] = __ffma2_rn(vv, make_float2(u.x, u.y), s[c][q / 2]);
+                s[c][q / 2 + 1] = __ffma2_rn(vv, make_float2(u.z, u.w), s[c][q / 2 + 1]);
+            }
+        }
+    }
+    // to dst[q * SB + column]
+    __device__ __forceinline__ void store(float* dst, int lane) const {
+#pragma unroll
+        for (int q = 0; q < NR / 2; q++) {
+            *reinterpret_cast<float4*>(dst + 2 * q * SB + 4 * lane) =
+                make_float4(s[0][q].x, s[1][q].x, s[2][q].x, s[3][q].x);
+            *reinterpret_cast<float4*>(dst + (2 * q + 1) * SB + 4 * lane) =
+                make_float4(s[0][q].y, s[1][q].y, s[2][q].y, s[3][q].y);
+        }
+    }
+};
+template <>
+struct Sums<1> {
+    float4 s;
+    __device__ __forceinline__ void clear() { s = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    __device__ __forceinline__ void add(float4 v, const float* y) {
+        const float u = *y;
+        s.x = fmaf(v.x, u, s.x);
+        s.y = fmaf(v.y, u, s.y);
+        s.z = fmaf(v.z, u, s.z);
+        s.w = fmaf(v.w, u, s.w);
+    }
+    __device__ __forceinline__ void store(float* dst, int lane) const { *reinterpret_cast<float4*>(dst + 4 * lane) = s; }
+};
+constexpr int NWARP = GT / 32;
+
 // One sweep (see the file comment).  FWD: in = b (rows of ldb), out: the
 // published y.  Backward: in = the forward sweep's published y, out: x = -s
 // into xout (rows of ldb) and the published s.  g = right-hand sides of this
@@ -385,9 +438,6 @@ __global__ void __launch_bounds__(GT, 1)
                  int ldb, unsigned long long* __restrict__ pub, int g, int q, int* __restrict__ ticket,
                  int* __restrict__ err, int stall) {
     constexpr int STG = stages<NR>();
-    // PS partial sums per right-hand side (rows round-robin) so that one right-hand side's
-    // FMAs form independent chains; combined in a fixed order
-    constexpr int PS = NR == 1 ? 4 : 1;
     extern __shared__ __align__(16) float smem[];
     float* op = smem;                         // 128 x 128 operator of the tile (row stride LDY)
     float* ring = op + kOpFloats;             // STG x 32 x 128 factor rows
@@ -399,7 +449,7 @@ __global__ void __launch_bounds__(GT, 1)
     const int nblk = (n + SB - 1) / SB;
     const long long nitems = items_before(nblk, q);
     const unsigned tag = FWD ? kTagFwd : kTagBwd;
-    const int c = tid & (SB - 1), h = tid >> 7;  // compute mapping: column c, rows 16h..16h+15 of a stage
+    const int warp = tid >> 5, lane = tid & 31;  // in the products: rows by warps, columns 4 lane .. 4 lane + 3
     for (;;) {
         __syncthreads();  // the previous item's shared data is consumed
         if (tid == 0) {
@@ -468,9 +518,8 @@ __global__ void __launch_bounds__(GT, 1)
             if (s < total) issue(s);
             cp_commit();
         }
-        float p[NR * PS];
-#pragma unroll
-        for (int r = 0; r < NR * PS; r++) p[r] = 0.0f;
+        Sums<NR> p;
+        p.clear();
         bool ok = *(volatile int*)err == 0;
         ok = __syncthreads_and(ok) != 0;
         const bool never = FWD && stall != 0 && t == 1;  // tile 1's only source is tile 0
@@ -483,24 +532,24 @@ __global__ void __launch_bounds__(GT, 1)
         auto consume = [&](int s, int sr) {
             const float* stg = ring + (s % STG) * STAGE_FLOATS;
 #pragma unroll
-            for (int r = 0; r < RS / 2; r++) {
-                const int row = h * (RS / 2) + r;
-                const float v = stg[row * SB + c];
-                const float* y = ybuf + (sr * RS + row) * NR;
-                if constexpr (NR % 4 == 0) {
-#pragma unroll
-                    for (int qq = 0; qq < NR; qq += 4) {
-                        const float4 y4 = *reinterpret_cast<const float4*>(y + qq);
-                        p[qq] = fmaf(y4.x, v, p[qq]);
-                        p[qq + 1] = fmaf(y4.y, v, p[qq + 1]);
-                        p[qq + 2] = fmaf(y4.z, v, p[qq + 2]);
-                        p[qq + 3] = fmaf(y4.w, v, p[qq + 3]);
-                    }
-                } else {
-#pragma unroll
-                    for (int qq = 0; qq < NR; qq++) p[qq * PS + r % PS] = fmaf(y[qq], v, p[qq * PS + r % PS]);
-                }
+            for (int r = 0; r < RS / NWARP; r++) {
+                const int row = warp * (RS / NWARP) + r;
+                p.add(*reinterpret_cast<const float4*>(stg + row * SB + 4 * lane), ybuf + (sr * RS + row) * NR);
             }
+        };
+        // The warps' sums meet in the ring slots of consumed stages (the finisher's last source occupies the four
+        // slots before them): SB x NR floats per warp from slot total % STG on, four slots at most, and the tile's
+        // accumulated input in the one after those.
+        auto wsum = [&](int w) {
+            constexpr int PER = STAGE_FLOATS / (SB * NR) < NWARP ? STAGE_FLOATS / (SB * NR) : NWARP;
+            return ring + ((total + w / PER) % STG) * STAGE_FLOATS + (w % PER) * (SB * NR);
+        };
+        float* acc = ring + ((total + SPT) % STG) * STAGE_FLOATS;  // 128 x NR (i * NR + q)
+        auto warp_sums = [&](int idx) {  // entry (q, i) = (idx / 128, idx % 128), the warps in order
+            float v = 0.0f;
+#pragma unroll
+            for (int w = 0; w < NWARP; w++) v += wsum(w)[idx];
+            return v;
         };
         const unsigned want = never ? kTagNever : tag;
         for (int s = 0; s < total && ok; s++) {
@@ -523,46 +572,28 @@ __global__ void __launch_bounds__(GT, 1)
             consume(s, sr);
         }
         if (!fin) cp_wait<0>();  // (a finisher's last source may still be in flight)
-        // this thread's sums of the sources added so far; the upper half's go to red.  The sums
-        // use two ring slots whose stages were consumed (the finisher's last source occupies
-        // the four slots before them)
-        float* red = ring + (total % STG) * STAGE_FLOATS;  // NR x 128
-        float* acc = red + NR * SB;                         // 128 x NR (i * NR + q): the tile's accumulated input
-        float* part = ring + ((total + 1) % STG) * STAGE_FLOATS;  // 2 x NR x 128
-        if constexpr (PS > 1) {
-#pragma unroll
-            for (int qq = 0; qq < NR; qq++)
-                p[qq * PS] = (p[qq * PS] + p[qq * PS + 1]) + (p[qq * PS + 2] + p[qq * PS + 3]);
-        }
-        if (h == 1) {
-#pragma unroll
-            for (int qq = 0; qq < NR; qq++) red[qq * SB + c] = p[qq * PS];
-        }
-        ok = __syncthreads_and(ok) != 0;
+        ok = __syncthreads_and(ok) != 0;  // every stage added so far is consumed
+        p.store(wsum(warp), lane);
+        __syncthreads();
+        constexpr int M = Pending<NR>::M;  // entries idx = tid + mm * GT of the tile's values per thread
         if (!fin) {  // a chunk: publish its sums
-            if (h == 0) {
-                unsigned long long* dst = pub + (size_t)(nblk + chunks_before(t, q) + mi) * g * SB;
+            unsigned long long* dst = pub + (size_t)(nblk + chunks_before(t, q) + mi) * g * SB;
 #pragma unroll
-                for (int qq = 0; qq < NR; qq++)
-                    if (qq < g && c < kb)
-                        st_pair(dst + (size_t)qq * SB + c, tag,
-                                ok ? p[qq * PS] + red[qq * SB + c] : __int_as_float(0x7fc00000));  // NaN: aborted
+            for (int mm = 0; mm < M; mm++) {
+                const int idx = tid + mm * GT, qq = idx / SB, i = idx - qq * SB;
+                if (idx < NR * SB && qq < g && i < kb)
+                    st_pair(dst + (size_t)qq * SB + i, tag, ok ? warp_sums(idx) : __int_as_float(0x7fc00000));  // NaN: aborted
             }
             continue;
         }
         // the finisher: acc = (in + the chunks' sums) + its own sources but the last
-        float own[NR];
+        float psum[M];
 #pragma unroll
-        for (int qq = 0; qq < NR; qq++) own[qq] = p[qq * PS] + red[qq * SB + c];
+        for (int mm = 0; mm < M; mm++) psum[mm] = 0.0f;
         if (nch > 0 && ok) {
-            // the chunks' sums: each thread adds up its entries over the chunks in chunk order
-            // (CG chunks' loads in flight at a time), then one barrier
+            // the chunks' sums, in chunk order, CG chunks' loads in flight at a time
             constexpr int CG = NR == 1 ? 8 : (NR <= 4 ? 4 : 1);
-            constexpr int M = Pending<NR>::M;
             const long long base = nblk + chunks_before(t, q);
-            float psum[M];
-#pragma unroll
-            for (int mm = 0; mm < M; mm++) psum[mm] = 0.0f;
             bool okp = true;
             for (int m0 = 0; m0 < nch; m0 += CG) {
                 Pending<NR> pc[CG];
@@ -584,75 +615,50 @@ __global__ void __launch_bounds__(GT, 1)
                     }
                 }
             }
-            __syncthreads();  // ybuf is free
-#pragma unroll
-            for (int mm = 0; mm < M; mm++) {
-                const int idx = tid + mm * GT;
-                if (idx < NR * SB) ybuf[(idx - (idx / SB) * SB) * NR + idx / SB] = psum[mm];
-            }
-            ok = __syncthreads_and(ok && okp) != 0;
+            ok = __syncthreads_and(okp) != 0;
         }
-        if (h == 0) {
 #pragma unroll
-            for (int qq = 0; qq < NR; qq++)
-                acc[c * NR + qq] = (inb[qq * SB + c] + (nch > 0 ? ybuf[c * NR + qq] : 0.0f)) + own[qq];
+        for (int mm = 0; mm < M; mm++) {
+            const int idx = tid + mm * GT, qq = idx / SB, i = idx - qq * SB;
+            if (idx < NR * SB) psum[mm] = (inb[idx] + psum[mm]) + warp_sums(idx);
+            if (idx < NR * SB && nsrc == 0) acc[i * NR + qq] = psum[mm];
         }
         // the last source: its values, then its four stages (all in the ring: STG > SPT)
         if (nsrc > 0 && ok) {
-            __syncthreads();  // ybuf is free
             ok = resolve_tile<NR>(pd, pub, src_tile(nloop), g, want, ybuf, err);
             cp_wait<0>();
             __syncthreads();
             if (ok) {
-#pragma unroll
-                for (int r = 0; r < NR * PS; r++) p[r] = 0.0f;
+                p.clear();
 #pragma unroll
                 for (int r4 = 0; r4 < SPT; r4++) consume(nloop * SPT + r4, r4);
-                if constexpr (PS > 1) {
-#pragma unroll
-                    for (int qq = 0; qq < NR; qq++)
-                        p[qq * PS] = (p[qq * PS] + p[qq * PS + 1]) + (p[qq * PS + 2] + p[qq * PS + 3]);
-                }
-                if (h == 1) {
-#pragma unroll
-                    for (int qq = 0; qq < NR; qq++) red[qq * SB + c] = p[qq * PS];
-                }
+                p.store(wsum(warp), lane);
                 __syncthreads();
-                if (h == 0) {
 #pragma unroll
-                    for (int qq = 0; qq < NR; qq++) acc[c * NR + qq] += p[qq * PS] + red[qq * SB + c];
+                for (int mm = 0; mm < M; mm++) {
+                    const int idx = tid + mm * GT, qq = idx / SB, i = idx - qq * SB;
+                    if (idx < NR * SB) acc[i * NR + qq] = psum[mm] + warp_sums(idx);
                 }
             }
         }
         cp_wait<0>();  // nothing of this item stays in flight (also after a wait that gave up)
         ok = __syncthreads_and(ok) != 0;
-        {  // res = operator^T acc, from the two halves of the product
-            const int i = tid & (SB - 1), hh = tid >> 7;
-            float pr[NR * PS];
+        // res = operator^T acc, rows by warps again
+        p.clear();
 #pragma unroll
-            for (int r = 0; r < NR * PS; r++) pr[r] = 0.0f;
-#pragma unroll 16
-            for (int kk = 0; kk < SB / 2; kk++) {
-                const int k = hh * (SB / 2) + kk;
-                const float m = op[k * LDY + i];
-#pragma unroll
-                for (int r = 0; r < NR; r++) pr[r * PS + kk % PS] = fmaf(m, acc[k * NR + r], pr[r * PS + kk % PS]);
-            }
-#pragma unroll
-            for (int r = 0; r < NR; r++) {
-                float v = pr[r * PS];
-                if constexpr (PS > 1) v = (pr[r * PS] + pr[r * PS + 1]) + (pr[r * PS + 2] + pr[r * PS + 3]);
-                part[(hh * NR + r) * SB + i] = v;
-            }
+        for (int r = 0; r < SB / NWARP; r++) {
+            const int k = warp * (SB / NWARP) + r;
+            p.add(*reinterpret_cast<const float4*>(op + k * LDY + 4 * lane), acc + k * NR);
         }
+        p.store(wsum(warp), lane);
         __syncthreads();
-        for (int idx = tid; idx < NR * SB; idx += GT) {
-            const int qq = idx / SB, i = idx - qq * SB;
-            if (qq < g && i < kb) {
-                const float v = ok ? part[qq * SB + i] + part[(NR + qq) * SB + i]
-                                   : __int_as_float(0x7fc00000);  // NaN marks an aborted solve
-                if (!FWD) xout[(size_t)qq * ldb + c0 + i] = -v;
+#pragma unroll
+        for (int mm = 0; mm < M; mm++) {
+            const int idx = tid + mm * GT, qq = idx / SB, i = idx - qq * SB;
+            if (idx < NR * SB && qq < g && i < kb) {
+                const float v = ok ? warp_sums(idx) : __int_as_float(0x7fc00000);  // NaN marks an aborted solve
                 st_pair(pub + ((size_t)j * g + qq) * SB + i, tag, v);
+                if (!FWD) xout[(size_t)qq * ldb + c0 + i] = -v;
             }
         }
     }
@@ -664,8 +670,10 @@ constexpr size_t sweep_smem() {
 }
 // the pieces fit in the ring; the tile's sums fit in two slots beside the last source's four
 static_assert(kScrFloats <= 9 * STAGE_FLOATS && 64 * L64 <= kMidOff, "scratch");
-static_assert(2 * 16 * SB <= STAGE_FLOATS && stages<1>() >= 2 * SPT + 1, "ring");
-static_assert(sweep_smem<1>() <= 227 * 1024 && sweep_smem<4>() <= 227 * 1024 && sweep_smem<16>() <= 227 * 1024,
+static_assert(NWARP * 16 * SB <= SPT * STAGE_FLOATS && 16 * SB <= STAGE_FLOATS && stages<1>() >= 2 * SPT + 1, "ring");
+static_assert(RS % NWARP == 0 && (GT & 31) == 0, "rows per warp");
+static_assert(sweep_smem<1>() <= 227 * 1024 && sweep_smem<4>() <= 227 * 1024 && sweep_smem<8>() <= 227 * 1024 &&
+                  sweep_smem<16>() <= 227 * 1024,
               "sweep shared memory");
 
 template <int NR>
@@ -699,6 +707,7 @@ int sweep_attrs() {
 int gesl_inv_init_attrs() {
     LP_CHECK(sweep_attrs<1>());
     LP_CHECK(sweep_attrs<4>());
+    LP_CHECK(sweep_attrs<8>());
     LP_CHECK(sweep_attrs<16>());
     return LP_OK;
 }
@@ -733,6 +742,8 @@ int launch_gesl_inv(const float* a, int lda, int n, float* b, int ldb, int nrhs,
             LP_CHECK(sweeps<1>(a, lda, n, bb, ldb, g, chunk, pub, tickets, err, stall_here, sms, st));
         else if (g <= 4)
             LP_CHECK(sweeps<4>(a, lda, n, bb, ldb, g, chunk, pub, tickets, err, stall_here, sms, st));
+        else if (g <= 8)
+            LP_CHECK(sweeps<8>(a, lda, n, bb, ldb, g, chunk, pub, tickets, err, stall_here, sms, st));
         else
             LP_CHECK(sweeps<16>(a, lda, n, bb, ldb, g, chunk, pub, tickets, err, stall_here, sms, st));
     }

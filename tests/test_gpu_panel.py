@@ -105,3 +105,22 @@ def test_batch_tile_edges(ctx, dev, lp, sizes, pad):
         x = np.linalg.solve(m.T.astype(np.float64), b.T).T
         got = gotB[s.b_off:s.b_off + s.nrhs * s.n].reshape(s.nrhs, s.n)
         assert np.abs(got - x).max() <= 8 * s.n * FLT_EPS * np.abs(x).max(), s.n
+
+
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (127, 5), (128, 8), (129, 9), (257, 3), (1000, 6), (4229, 8), (4229, 24)])
+def test_gesl_rhs_forms(ctx, dev, n, nrhs):
+    """The FP32 sweeps' forms for 1, 4, 8 and 16 right-hand sides on whole and ragged tiles, without and with chunk
+    items (tile 33 on): |x - want| <= 8 n eps max|x| on encoded factors of a dominant matrix."""
+    rng = np.random.default_rng(n + nrhs)
+    lda = (n + 3) // 4 * 4
+    u = n / 4 * rng.uniform(0.99, 1.01, n) + 1.0
+    S = rng.uniform(-0.5, 0.5, (n, n))
+    E = np.zeros((n, lda), np.float32)
+    E[:, :n] = np.tril(S, -1) + np.triu(S, 1) / u[:, None] - np.diag(1.0 / u)
+    want = rng.uniform(-1.0, 1.0, (nrhs, n))
+    F = E[:, :n].astype(np.float64)
+    y = want @ (np.tril(F, -1) - np.diag(1.0 / np.diag(F)))  # U x, U the transposed lower triangle
+    B = y @ (np.eye(n) - np.triu(F, 1))                      # L y
+    dE, dB = dev.put(E), dev.put(B.astype(np.float32))
+    ctx.gesl(dE.data_ptr(), n, lda, dB.data_ptr(), nrhs)
+    assert np.abs(dev.get(dB) - want).max() <= 8 * max(n, 16) * FLT_EPS
