@@ -3,10 +3,12 @@
 // host entry points that stand in for the reference's execution backend.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "lp_common.cuh"
@@ -50,8 +52,25 @@ void Workspace::release() {
     cap = 0;
 }
 
+// A blocking wait costs 100 to 400 us from the event's completion until the
+// thread runs again, more than a small solve takes on the device; so a caller's
+// own context polls the event, for 2 ms without pause, then every 50 us.  The
+// serving loop's worker threads share the cores and block.
 int wait_stream(lp_ctx* c, cudaStream_t st) {
     LP_CUDA(cudaEventRecord(c->ev_block, st));
+    if (!c->blocking_waits) {
+        using clock = std::chrono::steady_clock;
+        const auto spin_until = clock::now() + std::chrono::milliseconds(2);
+        for (;;) {
+            const cudaError_t e = cudaEventQuery(c->ev_block);
+            if (e == cudaSuccess) return LP_OK;
+            if (e != cudaErrorNotReady) return cuda_fail(e, "cudaEventQuery", __FILE__, __LINE__);
+            if (clock::now() < spin_until)
+                std::this_thread::yield();
+            else
+                std::this_thread::sleep_for(std::chrono::microseconds(50));
+        }
+    }
     LP_CUDA(cudaEventSynchronize(c->ev_block));
     return LP_OK;
 }
@@ -492,13 +511,20 @@ int gesl_clear(lp_ctx* c, cudaStream_t st) {
     return LP_OK;
 }
 
-int gesl_status(lp_ctx* c, cudaStream_t st, const char* who) {
+int read_status(lp_ctx* c, const void* word, cudaStream_t st, int* value) {
     if (c->hstat == nullptr) LP_CUDA(cudaMallocHost(&c->hstat, sizeof(int)));
-    LP_CHECK(c->gerr.ensure(sizeof(int)));
     *c->hstat = 0;
-    LP_CUDA(cudaMemcpyAsync(c->hstat, c->gerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    LP_CUDA(cudaMemcpyAsync(c->hstat, word, sizeof(int), cudaMemcpyDeviceToHost, st));
     LP_CHECK(wait_stream(c, st));
-    if (*c->hstat != 0)
+    *value = *c->hstat;
+    return LP_OK;
+}
+
+int gesl_status(lp_ctx* c, cudaStream_t st, const char* who) {
+    LP_CHECK(c->gerr.ensure(sizeof(int)));
+    int gave_up = 0;
+    LP_CHECK(read_status(c, c->gerr.ptr, st, &gave_up));
+    if (gave_up != 0)
         return fail(LP_E_TIMEOUT, std::string(who) + ": a bounded wait of the substitution sweeps expired "
                                                      "(the affected solution entries are NaN)");
     return LP_OK;

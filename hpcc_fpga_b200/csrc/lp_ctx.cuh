@@ -127,8 +127,10 @@ int launch_piv_gesl(const float* a, int lda, int n, int pb, const int* desc, flo
 // Restarted left-preconditioned GMRES in FP64 (lp_gmres.cu).
 int gmres_core(lp_ctx* c, const float* a0, int lda, const float* lu, int n, const double* b, double* x, int restart,
                int max_it, double tol, int* steps_out, double* resid_out, cudaStream_t st);
-// Waits for the work queued on st so far without spinning a CPU core.
+// Waits for the work queued on st so far.
 int wait_stream(lp_ctx* c, cudaStream_t st);
+// Copies a device error word back (through pinned memory) and waits for st.
+int read_status(lp_ctx* c, const void* word, cudaStream_t st, int* value);
 int solve_host_impl(lp_ctx* c, int precision, int n, int bs, float* A, int lda, const double* b64, int nrhs,
                     double* x, int max_iters, lp_timing* t);
 // lp_factor / lp_solve: factors of a host matrix kept resident in the context
@@ -158,7 +160,8 @@ struct lp_ctx {
     cudaStream_t lane_st = nullptr, lane_aux = nullptr;  // second lane of the row-slab schedule
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr;
     cudaEvent_t ev_side = nullptr, ev_side_done = nullptr;
-    cudaEvent_t ev_block = nullptr;           // blocking-sync event: waits yield the CPU instead of spinning
+    cudaEvent_t ev_block = nullptr;           // the event wait_stream waits for (blocking-sync)
+    bool blocking_waits = false;              // wait_stream blocks instead of polling (serving loop)
     cudaEvent_t ev[8] = {nullptr};
     // tensor-core panel: the identity recurrences (inverses of the diagonal
     // block's triangles) run on these two streams beside the lu stage, 128

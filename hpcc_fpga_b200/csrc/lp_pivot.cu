@@ -10,9 +10,7 @@ namespace {
 
 int piv_error(lp_ctx* c, cudaStream_t st, const char* who) {
     int herr = 0;
-    LP_CUDA(cudaMemcpyAsync(&herr, static_cast<unsigned char*>(c->psync.ptr) + 4, sizeof(int),
-                            cudaMemcpyDeviceToHost, st));
-    LP_CHECK(wait_stream(c, st));
+    LP_CHECK(read_status(c, static_cast<unsigned char*>(c->psync.ptr) + 4, st, &herr));
     if (herr != 0) return fail(LP_E_TIMEOUT, std::string(who) + ": a grid barrier did not complete in time");
     return LP_OK;
 }

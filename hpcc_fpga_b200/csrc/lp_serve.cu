@@ -814,6 +814,7 @@ int lp_server_start(int device, const lp_server_config* cfg, lp_server** out) {
         s->workers.push_back(w);
         const int st = lp_ctx_create(device, &w->c);
         if (st != LP_OK) return undo(st);
+        w->c->blocking_waits = true;
         w->base = w->c->stream;
         if (!w->wave && !per_request) {
             e = cudaStreamCreateWithPriority(&w->high, cudaStreamNonBlocking, prio_large);
