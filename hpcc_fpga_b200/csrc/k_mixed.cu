@@ -33,29 +33,49 @@ __device__ __forceinline__ void atomic_max_nonneg(float* addr, float v) {
 }
 
 // amax[seg * nblk + r / 512] = max |L[r][512 seg .. 512 seg + 512)| over each
-// 512-row block (blockIdx.y = seg).
-__global__ void k_absmax_rows(const float* __restrict__ L, int ldl, int rows, int k, int nblk,
-                              float* __restrict__ amax) {
-    const int r = blockIdx.x, seg = blockIdx.y;
+// 512-row block (blockIdx.y = seg), a warp per row, eight rows per warp; rows a
+// multiple of 128 and k of 128.
+__global__ void __launch_bounds__(256) k_absmax_rows(const float* __restrict__ L, int ldl, int rows, int k, int nblk,
+                                                     float* __restrict__ amax) {
+    const int seg = blockIdx.y, lane = threadIdx.x & 31, r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 8;
+    if (r0 >= rows) return;
     const int c1 = min(k, 512 * (seg + 1));
     float m = 0.0f;
-    for (int c = 512 * seg + threadIdx.x; c < c1; c += blockDim.x) m = fmaxf(m, fabsf(L[(size_t)r * ldl + c]));
+    for (int c = 512 * seg + 4 * lane; c < c1; c += 128) {
+        float4 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) v[r] = *reinterpret_cast<const float4*>(L + (size_t)(r0 + r) * ldl + c);
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[r].x), fabsf(v[r].y)), fmaxf(fabsf(v[r].z), fabsf(v[r].w))));
+    }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomic_max_nonneg(&amax[seg * nblk + (r >> 9)], m);
+    if (lane == 0) atomic_max_nonneg(&amax[seg * nblk + (r0 >> 9)], m);
 }
 
 // amax[seg * nblk + c / 512] = max |T[512 seg .. 512 seg + 512)[c]| over each
-// 512-column block.
-__global__ void k_absmax_cols(const float* __restrict__ T, int ldt, int k, int cols, int nblk,
-                              float* __restrict__ amax) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    for (int seg = 0; 512 * seg < k; seg++) {
-        float m = 0.0f;
-        const int r1 = min(k, 512 * (seg + 1));
-        for (int r = 512 * seg; r < r1; r++) m = fmaxf(m, fabsf(T[(size_t)r * ldt + c]));
-        atomic_max_nonneg(&amax[seg * nblk + (c >> 9)], m);
+// 512-column block: 128 columns x 64 rows per block (blockIdx.y: 64-row
+// chunks, which lie in one segment), so that the 512 rows of a column are not
+// one thread's chain.  cols a multiple of 4, k of 64; vec: rows allow 16-byte
+// loads.
+__global__ void __launch_bounds__(256) k_absmax_cols(const float* __restrict__ T, int ldt, int k, int cols, int nblk,
+                                                     bool vec, float* __restrict__ amax) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 128 + 4 * lane;
+    const int r0 = blockIdx.y * 64 + warp * 8;
+    float m = 0.0f;
+    if (c < cols && r0 < k) {
+        float4 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const float* p = T + (size_t)(r0 + r) * ldt + c;
+            v[r] = vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[r].x), fabsf(v[r].y)), fmaxf(fabsf(v[r].z), fabsf(v[r].w))));
     }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0 && c < cols) atomic_max_nonneg(&amax[((blockIdx.y * 64) >> 9) * nblk + (c >> 9)], m);
 }
 
 // scale = amax / 448 (1 for an all-zero block); inv = 1 / scale.
@@ -155,9 +175,9 @@ __global__ void k_split_rows(const float* __restrict__ L, int ldl, __nv_bfloat16
     }
 }
 
-// out[c][s*k + r] = term tterm(s) of T[r][c]: cols x (NSEG k) BF16, through a
-// 32 x 32 shared-memory transpose.
-template <int NSEG>
+// out[c][s*k + r] = term tterm(s) of T[r][c] (EYE: of T - I): cols x (NSEG k)
+// BF16, through a 32 x 32 shared-memory transpose.
+template <int NSEG, bool EYE>
 __global__ void __launch_bounds__(256) k_split_trans(const float* __restrict__ T, int ldt,
                                                      __nv_bfloat16* __restrict__ out, int k, int cols) {
     __shared__ float tile[32][33];
@@ -175,18 +195,12 @@ __global__ void __launch_bounds__(256) k_split_trans(const float* __restrict__ T
         const int c = c0 + ty + j, r = r0 + tx;
         if (r < k && c < cols) {
             __nv_bfloat16 t[3];
-            split3(tile[tx][ty + j], t[0], t[1], t[2]);
+            split3(EYE && r == c ? tile[tx][ty + j] - 1.0f : tile[tx][ty + j], t[0], t[1], t[2]);
             __nv_bfloat16* o = out + (size_t)c * kq + r;
 #pragma unroll
             for (int s = 0; s < NSEG; s++) o[(size_t)s * k] = t[tterm<NSEG>(s)];
         }
     }
-}
-
-// x[i][i] += v for i < n (an n x n block, leading dimension n).
-__global__ void k_add_diag(float* __restrict__ x, int n, float v) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[(size_t)i * n + i] += v;
 }
 
 // x = identity (two n x n blocks, leading dimension n).
@@ -201,67 +215,101 @@ __global__ void k_eye2(float* __restrict__ x, float* __restrict__ y, int n) {
 
 }  // namespace
 
-// The split-BF16 operands of a block step (nseg 6, 3 or 1 K-segments):
-// aq: rows_l x nseg k, bq: cols_t x nseg k.
-int split_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, uint8_t* aq,
-                uint8_t* bq, cudaStream_t st, int nseg) {
-    if (rows_l <= 0 || cols_t <= 0) return LP_OK;
-    if (nseg != 6 && nseg != 3 && nseg != 1) return fail(LP_E_INVALID, "split_panel: 1, 3 or 6 segments");
-    const size_t total = (size_t)rows_l * k;
+// The split-BF16 operands of a product (nseg 6, 3 or 1 K-segments): aq, rows x
+// nseg k, from L (rows x k).
+static int split_rows(const float* L, int ldl, int rows, int k, __nv_bfloat16* a, cudaStream_t st, int nseg) {
+    if (rows <= 0) return LP_OK;
+    const size_t total = (size_t)rows * k;
     const int grid = (int)((total + 255) / 256 < 4736 ? (total + 255) / 256 : 4736);
-    const dim3 tgrid((cols_t + 31) / 32, (k + 31) / 32);
-    auto* a = reinterpret_cast<__nv_bfloat16*>(aq);
-    auto* b = reinterpret_cast<__nv_bfloat16*>(bq);
-    if (nseg == 6) {
-        k_split_rows<6><<<grid, 256, 0, st>>>(L, ldl, a, rows_l, k);
-        k_split_trans<6><<<tgrid, 256, 0, st>>>(T, ldt, b, k, cols_t);
-    } else if (nseg == 3) {
-        k_split_rows<3><<<grid, 256, 0, st>>>(L, ldl, a, rows_l, k);
-        k_split_trans<3><<<tgrid, 256, 0, st>>>(T, ldt, b, k, cols_t);
-    } else {
-        k_split_rows<1><<<grid, 256, 0, st>>>(L, ldl, a, rows_l, k);
-        k_split_trans<1><<<tgrid, 256, 0, st>>>(T, ldt, b, k, cols_t);
-    }
-    count_launch(2);
+    if (nseg == 6)
+        k_split_rows<6><<<grid, 256, 0, st>>>(L, ldl, a, rows, k);
+    else if (nseg == 3)
+        k_split_rows<3><<<grid, 256, 0, st>>>(L, ldl, a, rows, k);
+    else if (nseg == 1)
+        k_split_rows<1><<<grid, 256, 0, st>>>(L, ldl, a, rows, k);
+    else
+        return fail(LP_E_INVALID, "split operands: 1, 3 or 6 segments");
+    count_launch();
     LP_CUDA(cudaGetLastError());
     return LP_OK;
 }
 
-// Rounds the panel of a block step to the tensor-core operand type.
-// L: rows_l x k (ld ldl), T: k x cols_t (ld ldt); aq: rows_l x k, bq:
-// cols_t x k; sc: 3 arrays of kseg(k) * nblk floats (absmax, scale, 1/scale,
-// indexed seg * nblk + block) for L, then 3 for T (nblk >=
-// ceil(max(rows_l, cols_t) / 512)).
-int quantize_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, bool fp8,
-                   uint8_t* aq, uint8_t* bq, float* sc, int nblk, cudaStream_t st) {
-    if (rows_l <= 0 || cols_t <= 0) return LP_OK;
-    const size_t q4 = (size_t)rows_l * k / 4;
-    const int qgrid = (int)((q4 + 255) / 256 < 2368 ? (q4 + 255) / 256 : 2368);
-    const dim3 tgrid((cols_t + 31) / 32, (k + 31) / 32);
+// bq, cols x nseg k, from T (k x cols), or from T - I (eye).
+static int split_trans(const float* T, int ldt, int cols, int k, __nv_bfloat16* b, cudaStream_t st, int nseg,
+                       bool eye = false) {
+    if (cols <= 0) return LP_OK;
+    const dim3 grid((cols + 31) / 32, (k + 31) / 32);
+    if (nseg == 6 && eye)
+        k_split_trans<6, true><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else if (nseg == 6)
+        k_split_trans<6, false><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else if (nseg == 3 && eye)
+        k_split_trans<3, true><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else if (nseg == 3)
+        k_split_trans<3, false><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else if (nseg == 1 && eye)
+        k_split_trans<1, true><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else if (nseg == 1)
+        k_split_trans<1, false><<<grid, 256, 0, st>>>(T, ldt, b, k, cols);
+    else
+        return fail(LP_E_INVALID, "split operands: 1, 3 or 6 segments");
+    count_launch();
+    LP_CUDA(cudaGetLastError());
+    return LP_OK;
+}
+
+// The left panel L (rows x k, ld ldl) rounded to the tensor-core operand type:
+// aq, rows x k.  E4M3: sc holds kseg(k) * nblk block maxima, then the scales,
+// then their reciprocals, indexed seg * nblk + block.  rows and k multiples of
+// 128.
+static int quantize_left(const float* L, int ldl, int rows, int k, bool fp8, uint8_t* aq, float* sc, int nblk,
+                         cudaStream_t st) {
+    if (rows <= 0) return LP_OK;
+    const size_t q4 = (size_t)rows * k / 4;
+    const int grid = (int)((q4 + 255) / 256 < 2368 ? (q4 + 255) / 256 : 2368);
     if (fp8) {
         const int ns = kseg(k) * nblk;
-        float* amax_a = sc;
-        float* scale_a = sc + ns;
-        float* inv_a = sc + 2 * ns;
-        float* amax_b = sc + 3 * ns;
-        float* scale_b = sc + 4 * ns;
-        float* inv_b = sc + 5 * ns;
-        LP_CUDA(cudaMemsetAsync(amax_a, 0, sizeof(float) * ns, st));
-        LP_CUDA(cudaMemsetAsync(amax_b, 0, sizeof(float) * ns, st));
-        k_absmax_rows<<<dim3(rows_l, kseg(k)), 128, 0, st>>>(L, ldl, rows_l, k, nblk, amax_a);
-        k_absmax_cols<<<(cols_t + 255) / 256, 256, 0, st>>>(T, ldt, k, cols_t, nblk, amax_b);
-        k_scales<<<(ns + 127) / 128, 128, 0, st>>>(amax_a, scale_a, inv_a, ns);
-        k_scales<<<(ns + 127) / 128, 128, 0, st>>>(amax_b, scale_b, inv_b, ns);
-        k_quant_rows<true><<<qgrid, 256, 0, st>>>(L, ldl, aq, rows_l, k, inv_a, nblk);
-        k_quant_trans<true><<<tgrid, 256, 0, st>>>(T, ldt, bq, k, cols_t, inv_b, nblk);
-        count_launch(6);
+        LP_CUDA(cudaMemsetAsync(sc, 0, sizeof(float) * ns, st));
+        k_absmax_rows<<<dim3((rows + 63) / 64, kseg(k)), 256, 0, st>>>(L, ldl, rows, k, nblk, sc);
+        k_scales<<<(ns + 127) / 128, 128, 0, st>>>(sc, sc + ns, sc + 2 * ns, ns);
+        k_quant_rows<true><<<grid, 256, 0, st>>>(L, ldl, aq, rows, k, sc + 2 * ns, nblk);
+        count_launch(3);
     } else {
-        k_quant_rows<false><<<qgrid, 256, 0, st>>>(L, ldl, aq, rows_l, k, nullptr, nblk);
-        k_quant_trans<false><<<tgrid, 256, 0, st>>>(T, ldt, bq, k, cols_t, nullptr, nblk);
-        count_launch(2);
+        k_quant_rows<false><<<grid, 256, 0, st>>>(L, ldl, aq, rows, k, nullptr, nblk);
+        count_launch();
     }
     LP_CUDA(cudaGetLastError());
     return LP_OK;
+}
+
+// The same for the top panel T (k x cols, ld ldt), transposed: bq, cols x k.
+static int quantize_top(const float* T, int ldt, int cols, int k, bool fp8, uint8_t* bq, float* sc, int nblk,
+                        cudaStream_t st) {
+    if (cols <= 0) return LP_OK;
+    const dim3 grid((cols + 31) / 32, (k + 31) / 32);
+    if (fp8) {
+        const int ns = kseg(k) * nblk;
+        LP_CUDA(cudaMemsetAsync(sc, 0, sizeof(float) * ns, st));
+        k_absmax_cols<<<dim3((cols + 127) / 128, (k + 63) / 64), 256, 0, st>>>(T, ldt, k, cols, nblk,
+                                                                                   ldt % 4 == 0 && aligned16(T), sc);
+        k_scales<<<(ns + 127) / 128, 128, 0, st>>>(sc, sc + ns, sc + 2 * ns, ns);
+        k_quant_trans<true><<<grid, 256, 0, st>>>(T, ldt, bq, k, cols, sc + 2 * ns, nblk);
+        count_launch(3);
+    } else {
+        k_quant_trans<false><<<grid, 256, 0, st>>>(T, ldt, bq, k, cols, nullptr, nblk);
+        count_launch();
+    }
+    LP_CUDA(cudaGetLastError());
+    return LP_OK;
+}
+
+// Both panels; sc: the left panel's three arrays of kseg(k) * nblk floats, then
+// the top panel's (nblk >= ceil(max(rows_l, cols_t) / 512)).
+int quantize_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, bool fp8,
+                   uint8_t* aq, uint8_t* bq, float* sc, int nblk, cudaStream_t st) {
+    if (rows_l <= 0 || cols_t <= 0) return LP_OK;
+    LP_CHECK(quantize_left(L, ldl, rows_l, k, fp8, aq, sc, nblk, st));
+    return quantize_top(T, ldt, cols_t, k, fp8, bq, sc + 3 * (size_t)kseg(k) * nblk, nblk, st);
 }
 
 // One trailing (sub)update of the mixed schedule: rows [m_off, m_off+m) and
@@ -289,7 +337,16 @@ static int mixed_update(lp_ctx* c, float* c11, int lda, const uint8_t* aq, const
 // the n bs^2 flops of the recurrences per step leave the FMA pipe.  V is unit
 // triangular, so L keeps its exact identity part; W^-1 is not (its diagonal
 // is D_kk = -1/u_kk), and T0 + (W^-1 - I) T0 would cancel nearly all of T0.
-static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nseg, cudaStream_t s) {
+// What reads only the panel's input -- the operands T0 and L0, and clearing the
+// block row -- runs on aux2 beside the lu stage; the rounded copies q for the
+// trailing update run beside the other half's product.
+struct PanelOut {
+    int fp8, x6;         // operand type of the trailing update (neither: BF16)
+    uint8_t *aq, *bq;    // left and top operands
+    float* sc;           // E4M3 scales
+    int nblk;
+};
+static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nseg, const PanelOut& q, cudaStream_t s) {
     float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
     const double b = bs;
     const int rest = n - (K + 1) * bs;
@@ -297,6 +354,12 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     float* winv = static_cast<float*>(c->tri.ptr);
     float* vinv = winv + bb;
     float* vlt = vinv + bb;
+    float* t = d + bs;
+    float* l = d + (size_t)bs * lda;
+    __nv_bfloat16* a_top = static_cast<__nv_bfloat16*>(c->tq.ptr);  // bs x kq: W^-1
+    __nv_bfloat16* b_left = a_top + bb * nseg;                      // bs x kq: (V - I)^T
+    __nv_bfloat16* b_top = b_left + bb * nseg;                      // rest x kq: T^T
+    __nv_bfloat16* a_left = b_top + (size_t)n * kq;                 // rest x kq: L
     // bs > 128: W^-1 and V are built 128 rows / columns behind the lu stage on
     // two side streams (lu_stage), rather than after it.  Measured on one B200,
     // factorization alone, n = 32768, block 1024: BF16 55.3 -> 51.5 ms, E4M3
@@ -304,7 +367,13 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     // FP32 form (six segments), whose tensor-bound update only loses SMs to the
     // side streams (143 -> 148 ms).
     const bool beside = rest > 0 && bs > 128 && nseg < 6;
-    if (beside) {
+    if (rest > 0) {
+        LP_CUDA(cudaEventRecord(c->ev_side, s));
+        LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+        LP_CHECK(split_trans(t, lda, rest, bs, b_top, c->aux2, nseg));
+        LP_CUDA(cudaMemset2DAsync(t, sizeof(float) * (size_t)lda, 0, sizeof(float) * (size_t)rest, bs, c->aux2));
+        LP_CHECK(split_rows(l, lda, rest, bs, a_left, c->aux2, nseg));
+        LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
         k_eye2<<<(int)((bb + 255) / 256 < 1184 ? (bb + 255) / 256 : 1184), 256, 0, s>>>(winv, vinv, bs);
         count_launch();
         LP_CUDA(cudaGetLastError());
@@ -316,46 +385,48 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * b * b * b / 3.0, 8.0 * b * b));
     if (rest <= 0) return LP_OK;
     const double r = rest;
-    __nv_bfloat16* tq = static_cast<__nv_bfloat16*>(c->tq.ptr);
-    uint8_t* a_top = reinterpret_cast<uint8_t*>(tq);                    // bs x kq: W^-1
-    uint8_t* b_left = reinterpret_cast<uint8_t*>(tq + bb * nseg);       // bs x kq: (V - I)^T
-    uint8_t* b_top = reinterpret_cast<uint8_t*>(tq + 2 * bb * nseg);    // rest x kq: T^T
-    uint8_t* a_left = reinterpret_cast<uint8_t*>(tq + 2 * bb * nseg + (size_t)n * kq);  // rest x kq: L
     int* err = static_cast<int*>(c->err.ptr);
 
     e = prof_begin(c, s);
     if (!beside) {
-        k_eye2<<<(int)((bb + 255) / 256 < 1184 ? (bb + 255) / 256 : 1184), 256, 0, s>>>(winv, vinv, bs);
-        count_launch();
-        LP_CUDA(cudaGetLastError());
         if (bs <= 512) {
             LP_CHECK(launch_tl(d, lda, dinv, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt,
                                bs, c->num_sms, s));
         } else {
-            LP_CUDA(cudaEventRecord(c->ev_side, s));
-            LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+            LP_CUDA(cudaEventRecord(c->ev_inv[0], s));
+            LP_CUDA(cudaStreamWaitEvent(c->inv_left, c->ev_inv[0], 0));
             for (int kk = 0; kk < bs / 128; kk++)
-                LP_CHECK(left_chunk_step(c, d, lda, dinv, vinv, bs, vlt, kk, c->aux2));
-            LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
+                LP_CHECK(left_chunk_step(c, d, lda, dinv, vinv, bs, vlt, kk, c->inv_left));
+            LP_CUDA(cudaEventRecord(c->ev_inv_left, c->inv_left));
             for (int kk = 0; kk < bs / 128; kk++) LP_CHECK(top_chunk_step(c, d, lda, dinv, winv, bs, kk, s));
-            LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
+            LP_CUDA(cudaStreamWaitEvent(s, c->ev_inv_left, 0));
         }
     }
-    k_add_diag<<<(bs + 127) / 128, 128, 0, s>>>(vinv, bs, -1.0f);
-    count_launch();
-    LP_CUDA(cudaGetLastError());
-    float* t = d + bs;
-    float* l = d + (size_t)bs * lda;
-    LP_CHECK(split_panel(winv, bs, t, lda, bs, rest, bs, a_top, b_top, s, nseg));
-    LP_CUDA(cudaMemset2DAsync(t, sizeof(float) * (size_t)lda, 0, sizeof(float) * (size_t)rest, bs, s));
+    LP_CHECK(split_rows(winv, bs, bs, bs, a_top, s, nseg));
+    LP_CHECK(split_trans(vinv, bs, bs, bs, b_left, s, nseg, true));
+    LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
     LP_CHECK(launch_umma_update(t, lda, a_top, bs, b_top, rest, 0, 0, bs, rest, (int)kq, false, nullptr, nullptr, 0,
                                 err, s));
     LP_CHECK(prof_end(c, s, LP_STAGE_TOP, e, b * b * r, 8.0 * b * r));
+    LP_CUDA(cudaEventRecord(c->ev_side, s));
+    LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+    if (q.x6)
+        LP_CHECK(split_trans(t, lda, rest, bs, reinterpret_cast<__nv_bfloat16*>(q.bq), c->aux2, 6));
+    else
+        LP_CHECK(quantize_top(t, lda, rest, bs, q.fp8 != 0, q.bq, q.sc + 3 * (size_t)kseg(bs) * q.nblk, q.nblk, c->aux2));
+    LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
     e = prof_begin(c, s);
-    LP_CHECK(split_panel(l, lda, vinv, bs, rest, bs, bs, a_left, b_left, s, nseg));
     LP_CHECK(launch_umma_update(l, lda, a_left, rest, b_left, bs, 0, 0, rest, bs, (int)kq, false, nullptr, nullptr, 0,
                                 err, s));
-    return prof_end(c, s, LP_STAGE_LEFT, e, b * b * r, 8.0 * b * r);
+    LP_CHECK(prof_end(c, s, LP_STAGE_LEFT, e, b * b * r, 8.0 * b * r));
+    e = prof_begin(c, s);
+    if (q.x6)
+        LP_CHECK(split_rows(l, lda, rest, bs, reinterpret_cast<__nv_bfloat16*>(q.aq), s, 6));
+    else
+        LP_CHECK(quantize_left(l, lda, rest, bs, q.fp8 != 0, q.aq, q.sc, q.nblk, s));
+    LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
+    const double esz = q.fp8 ? 1.0 : 2.0;
+    return prof_end(c, s, LP_STAGE_OTHER, e, 0.0, 2.0 * 4.0 * b * rest + 2.0 * esz * b * rest);
 }
 
 int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cudaStream_t st) {
@@ -389,19 +460,8 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
     const double b = bs;
 
     auto panel_q = [&](int K, cudaStream_t s) -> int {
-        LP_CHECK(panel_tc(c, dA, n, lda, bs, K, nseg, s));
-        const int rest = n - (K + 1) * bs;
-        if (rest <= 0) return LP_OK;
-        float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
-        const int e = prof_begin(c, s);
-        if (x6)
-            LP_CHECK(split_panel(d + (size_t)bs * lda, lda, d + bs, lda, rest, rest, bs, aqb[K & 1], bqb[K & 1], s));
-        else
-            LP_CHECK(quantize_panel(d + (size_t)bs * lda, lda, d + bs, lda, rest, rest, bs, fp8, aqb[K & 1],
-                                    bqb[K & 1], scb[K & 1], nblk, s));
-        return prof_end(c, s, LP_STAGE_OTHER, e, 0.0, 2.0 * 4.0 * b * rest + 2.0 * esz * b * rest);
+        return panel_tc(c, dA, n, lda, bs, K, nseg, PanelOut{fp8, x6, aqb[K & 1], bqb[K & 1], scb[K & 1], nblk}, s);
     };
-
     LP_CHECK(panel_q(0, st));
     for (int K = 0; K + 1 < nb; K++) {
         const int rest = n - (K + 1) * bs;

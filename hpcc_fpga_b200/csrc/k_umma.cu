@@ -848,10 +848,10 @@ int launch_umma_update(float* c, int ldc, const void* aq, int aq_rows, const voi
     // of this kernel fills an SM (shared memory, registers), so a full-width
     // persistent grid would hold the panel off until the update ends.  Measured
     // on B200 (BF16 factorization alone): block 512, n = 32768: 8 free SMs +9 %
-    // over none; block 1024, n = 32768: 16 instead of 8 56.7 -> 55.3 ms (E4M3
-    // 63.9 -> 59.3 ms), 24 to 48 no further gain; block 2048, n = 65536, and the
-    // emulated FP32 form: 8 and 16 alike.
-    constexpr int kPanelSMs = 16;
+    // over none; block 1024, n = 32768: 32 instead of 16 50.1 -> 48.1 ms (E4M3
+    // 46.4 -> 47.1); block 512, n = 16384: 14.4 -> 13.8 ms (E4M3 14.9 -> 14.2);
+    // emulated FP32, n = 16384: 23.4 -> 22.4 ms; 48 no further gain.
+    constexpr int kPanelSMs = 32;
     const int usable = sms - kPanelSMs > 1 ? sms - kPanelSMs : 1;
     if (pair) {
         const int tiles_n = n / 256, tiles = tiles_n * (m / 256);

@@ -53,9 +53,6 @@ int launch_tl(const float* d, int ldd, const float* inv, const float* dt, int ld
 int quantize_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, bool fp8,
                    uint8_t* aq, uint8_t* bq, float* sc, int nblk, cudaStream_t st);
 inline int kseg(int k) { return (k + 511) / 512; }
-// Split-BF16 operands (exact three-term split; 6 or 3 K-segments) of a block step.
-int split_panel(const float* L, int ldl, const float* T, int ldt, int rows_l, int cols_t, int k, uint8_t* aq,
-                uint8_t* bq, cudaStream_t st, int nseg = 6);
 // Inverses of the diagonal block's two triangles for the tensor-core panel:
 // top applied to the bs x bs identity (winv) and left applied to it (vinv;
 // vlt: scratch for its transposed chunks), both starting from the identity.
