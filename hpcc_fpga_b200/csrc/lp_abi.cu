@@ -263,9 +263,17 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
     return prof_end(c, st, LP_STAGE_TOP, e, trsm_flops(b, r + w), 8.0 * b * r + 12.0 * b * w);
 }
 
-// Inner block of the FP32 schedule: a multiple of 128 up to 512 whatever
-// block the caller named (the blocking changes results by rounding only).
-int f32_block(int bs) { return std::max(128, bs); }
+// Inner block of the FP32 schedule, from the order alone whatever block the
+// caller named (the blocking changes results by rounding only).  A matrix of
+// one block is only the lu stage's chain.  Above that, small blocks shorten
+// the chain of a step (what bounds small orders) and large blocks read and
+// write the trailing matrix less often (what bounds large ones).  Measured on
+// one B200, factorization alone in us with blocks of 128 / 256 / 512:
+//   n =  512: 158 / 155 / 139         n =  6144: 5093 / 4784 / 5063
+//   n = 1024: 341 / 359 / 356         n =  8192: 9772 / 9104 / 9124
+//   n = 2048: 773 / 824 / 903         n = 12288: 27395 / 25235 / 24717
+//   n = 4096: 2199 / 2222 / 2435      n = 16384: 59371 / 55091 / 53552
+static int f32_block(int n) { return n <= 512 ? 512 : n < 4096 ? 128 : n < 9216 ? 256 : 512; }
 
 // Workspaces of the FP32 panel: the inverses of every 128-wide diagonal block
 // and the transposed lower triangle of the current block.
@@ -284,7 +292,13 @@ int panel_ensure(lp_ctx* c, int n, int bs) {
 // The stages give the reference recurrences' values up to rounding; the exact
 // recurrences are lp_lu_block_dev, lp_top_update_dev, lp_left_update_dev.
 int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
-    const int bs = f32_block(user_bs);
+    // where device memory has no room for the operands of the order's block,
+    // the caller's own (its operands are what the call has always needed)
+    int bs = f32_block(n);
+    if (bs > user_bs && bs > 128 && c->lt.ensure(2 * sizeof(float) * (size_t)bs * n) != LP_OK) {
+        cudaGetLastError();  // the allocation's
+        bs = std::max(128, user_bs);
+    }
     LP_CHECK(c->lt.ensure(2 * sizeof(float) * (size_t)bs * n));
     LP_CHECK(panel_ensure(c, n, bs));
     float* ltbuf[2] = {static_cast<float*>(c->lt.ptr), static_cast<float*>(c->lt.ptr) + (size_t)bs * n};
@@ -431,6 +445,13 @@ static std::vector<int> slab_cuts(int n, int bs) {
     return cuts;
 }
 
+// Events of the streamed form: one per block row, one per slab (no more than
+// block rows), the start and the second lane's end.
+size_t streamed_events(int n) {
+    const int bs = f32_block(n);
+    return 2 * (size_t)((n + bs - 1) / bs) + 2;
+}
+
 // gefa_f32 on a matrix that is still in page-locked host memory hA: every
 // row slab is queued for copying on the copy-in stream at once (after the
 // work already queued on st), and each slab is factored as soon as it is
@@ -440,10 +461,10 @@ static std::vector<int> slab_cuts(int n, int bs) {
 // lanes at once (a slab's own steps start after the other lane's last panel),
 // so the panel's scratch is shared.  With host_out, every block row goes back
 // to host_out (leading dimension lda) on the copy stream as soon as it is
-// final.  ev: at least 2 ceil(n / bs) + 2 events.
-int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int user_bs, cudaStream_t st,
-                      float* host_out, const std::vector<cudaEvent_t>& ev) {
-    const int bs = f32_block(user_bs);
+// final.  ev: streamed_events(n) events.
+int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, cudaStream_t st, float* host_out,
+                      const std::vector<cudaEvent_t>& ev) {
+    const int bs = f32_block(n);
     const std::vector<int> cuts = slab_cuts(n, bs);
     const int ns = (int)cuts.size() - 1, nb = (n + bs - 1) / bs;
     if ((int)ev.size() < nb + ns + 2) return fail(LP_E_INVALID, "streamed factorization: too few events");
@@ -903,7 +924,7 @@ int lp_calculate(lp_ctx* c, int n, int lda, int bs, int repetitions, float* A, f
     } evs;
     if (pinned) {
         evs.c = c;
-        evs.v.resize(2 * (size_t)(n / bs) + 2, nullptr);
+        evs.v.resize(streamed_events(n), nullptr);
         for (auto& e : evs.v) LP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     int status = LP_OK;
@@ -912,7 +933,7 @@ int lp_calculate(lp_ctx* c, int n, int lda, int bs, int repetitions, float* A, f
         LP_CUDA(cudaMemcpyAsync(dB, b, sizeof(float) * n, cudaMemcpyHostToDevice, st));
         if (pinned) {
             LP_CUDA(cudaEventRecord(c->ev[0], st));
-            status = gefa_f32_streamed(c, A, dA, n, lda, bs, st, last ? A : nullptr, evs.v);
+            status = gefa_f32_streamed(c, A, dA, n, lda, st, last ? A : nullptr, evs.v);
         } else {
             LP_CUDA(cudaMemcpyAsync(dA, A, abytes, cudaMemcpyHostToDevice, st));
             LP_CUDA(cudaEventRecord(c->ev[0], st));

@@ -27,6 +27,22 @@ def test_gefa_blocking_edges(ctx, dev, n, bs, pad):
     assert err.max() < 256 * FLT_EPS
 
 
+@pytest.mark.parametrize("n", [496, 512, 528, 4080, 4096, 4240, 9216])
+def test_gefa_block_of_the_order(ctx, dev, n):
+    """Orders on each side of the inner block's borders, last blocks that are no multiple of it, a caller's block of
+    16: max |L U - A| (the reference's storage: -1/u_kk on the diagonal, negated multipliers right of it, U^T below)
+    within 4 n eps max|L| max|U| on 64 sampled rows, in FP64."""
+    A, _, _, _ = oracle.gen_reference(n)
+    d = dev.put(A)
+    ctx.gefa(d.data_ptr(), n, n, 16)
+    F = dev.get(d).astype(np.float64)
+    M = np.triu(-F, 1) + np.eye(n)           # right of the diagonal: multipliers, unit diagonal
+    U = np.tril(F, -1) + np.diag(-1.0 / np.diag(F))
+    rows = np.unique(np.linspace(0, n - 1, 64).astype(int))
+    err = np.abs(U[rows] @ M - A[rows]).max()
+    assert err <= 4 * n * FLT_EPS * np.abs(U).max() * np.abs(M).max()
+
+
 @pytest.mark.parametrize("n,bs", [(1088, 64), (2096, 16), (1536, 128)])
 def test_streamed_ragged_blocks(ctx, lp, n, bs):
     """Page-locked buffers (factored in row slabs while copied in) give the pageable path's bits."""
