@@ -362,11 +362,11 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     __nv_bfloat16* a_left = b_top + (size_t)n * kq;                 // rest x kq: L
     // bs > 128: W^-1 and V are built 128 rows / columns behind the lu stage on
     // two side streams (lu_stage), rather than after it.  Measured on one B200,
-    // factorization alone, n = 32768, block 1024: BF16 55.3 -> 51.5 ms, E4M3
-    // 59.3 -> 54.5 ms; n = 65536, block 2048: unchanged.  Not for the emulated
-    // FP32 form (six segments), whose tensor-bound update only loses SMs to the
-    // side streams (143 -> 148 ms).
-    const bool beside = rest > 0 && bs > 128 && nseg < 6;
+    // factorization alone, after it -> beside it: BF16 n = 32768, block 1024
+    // 55.3 -> 51.5 ms, E4M3 59.3 -> 54.5 ms; emulated FP32 (six segments)
+    // n = 2048, block 512 1.15 -> 1.01 ms, n = 8192, block 512 6.70 -> 6.00 ms,
+    // n = 16384, block 1024 22.6 -> 21.4 ms, n = 32768, block 1024 equal.
+    const bool beside = rest > 0 && bs > 128;
     if (rest > 0) {
         LP_CUDA(cudaEventRecord(c->ev_side, s));
         LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
@@ -388,20 +388,9 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     int* err = static_cast<int*>(c->err.ptr);
 
     e = prof_begin(c, s);
-    if (!beside) {
-        if (bs <= 512) {
-            LP_CHECK(launch_tl(d, lda, dinv, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt,
-                               bs, c->num_sms, s));
-        } else {
-            LP_CUDA(cudaEventRecord(c->ev_inv[0], s));
-            LP_CUDA(cudaStreamWaitEvent(c->inv_left, c->ev_inv[0], 0));
-            for (int kk = 0; kk < bs / 128; kk++)
-                LP_CHECK(left_chunk_step(c, d, lda, dinv, vinv, bs, vlt, kk, c->inv_left));
-            LP_CUDA(cudaEventRecord(c->ev_inv_left, c->inv_left));
-            for (int kk = 0; kk < bs / 128; kk++) LP_CHECK(top_chunk_step(c, d, lda, dinv, winv, bs, kk, s));
-            LP_CUDA(cudaStreamWaitEvent(s, c->ev_inv_left, 0));
-        }
-    }
+    if (!beside)  // one chunk: the two recurrences in one launch
+        LP_CHECK(launch_tl(d, lda, dinv, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt, bs,
+                           c->num_sms, s));
     LP_CHECK(split_rows(winv, bs, bs, bs, a_top, s, nseg));
     LP_CHECK(split_trans(vinv, bs, bs, bs, b_left, s, nseg, true));
     LP_CUDA(cudaStreamWaitEvent(s, c->ev_side_done, 0));
