@@ -349,7 +349,7 @@ struct PanelOut {
 static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nseg, const PanelOut& q, cudaStream_t s) {
     float* d = dA + (size_t)K * bs * lda + (size_t)K * bs;
     const double b = bs;
-    const int rest = n - (K + 1) * bs;
+    const int rest = n - (K + 1) * bs;  // <= 0: the last block, of n - K bs
     const size_t bb = (size_t)bs * bs, kq = (size_t)nseg * bs;
     float* winv = static_cast<float*>(c->tri.ptr);
     float* vinv = winv + bb;
@@ -381,8 +381,9 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     const TriInverses inv{winv, vinv, vlt};
     float* dinv = block_inv(c, K * bs);
     int e = prof_begin(c, s);
-    LP_CHECK(lu_stage(c, d, lda, bs, dinv, s, beside ? &inv : nullptr));
-    LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * b * b * b / 3.0, 8.0 * b * b));
+    const int kb = std::min(bs, n - K * bs);
+    LP_CHECK(lu_stage(c, d, lda, kb, dinv, s, beside ? &inv : nullptr));
+    LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * kb * kb * (double)kb / 3.0, 8.0 * kb * (double)kb));
     if (rest <= 0) return LP_OK;
     const double r = rest;
     int* err = static_cast<int*>(c->err.ptr);
@@ -418,18 +419,45 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
     return prof_end(c, s, LP_STAGE_OTHER, e, 0.0, 2.0 * 4.0 * b * rest + 2.0 * esz * b * rest);
 }
 
-int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cudaStream_t st) {
+// Inner block of the emulated-FP32 form, and of BF16 from order 4096 on: 1024,
+// or the caller's if larger (the last block may be smaller).  Wide blocks read
+// and write the FP32 trailing matrix less often and give the update a longer
+// K; the chain of the 128-wide inner blocks is as long either way.  A matrix
+// of one block is the FP32 lu stage alone.  E4M3 and small BF16 matrices keep
+// the caller's block: what a wide block computes in FP32 instead of in rounded
+// operands moves their factors by more than FP32 accuracy (E4M3, n = 12288:
+// 6e-5 relative to the factors' norm; BF16 2e-5 at n = 2048, 1e-5 at 4096, 5e-6 at 12288).
+// Measured on one B200, factorization alone in ms, blocks of 128 / 512 / 1024:
+//   BF16          n = 4096 2.89 / 1.95 / 1.84   n = 8192 7.55 / 4.70 / 4.35   n = 32768 217 / 66.0 / 47.8
+//   emulated FP32 n = 3072 2.35 / 1.68 / 1.51   n = 8192 8.67 / 5.91 / 5.70   n = 32768 276 / 144 / 136
+constexpr int kMixedBlock = 1024;
+
+// Workspaces for blocks of up to bs.  With *grow, only what they need beyond
+// their present sizes is added up.
+static int mixed_ensure(lp_ctx* c, int precision, int n, int bs, int nseg, size_t* grow) {
+    const size_t esz = precision == LP_FP8_IR ? 1 : 2, kq = precision == LP_F32_BF16X6 ? 6 * (size_t)bs : bs;
+    const size_t nblk = (n + 511) / 512, b = bs;
+    const struct { Workspace* w; size_t bytes; } need[] = {
+        {&c->dinv, sizeof(float) * kInvFloats * (size_t)((n + 127) / 128)},
+        {&c->dt, sizeof(float) * b * b},
+        {&c->q, 4 * esz * kq * n},
+        {&c->qs, 2 * 6 * sizeof(float) * (size_t)kseg(bs) * nblk},
+        {&c->err, sizeof(int)},
+        {&c->tri, 3 * sizeof(float) * b * b},
+        {&c->tq, 2 * sizeof(__nv_bfloat16) * (size_t)nseg * b * (b + n)}};
+    for (const auto& x : need) {
+        if (grow == nullptr)
+            LP_CHECK(x.w->ensure(x.bytes));
+        else if (x.bytes > x.w->cap)
+            *grow += x.bytes;
+    }
+    return LP_OK;
+}
+
+int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
     const bool fp8 = precision == LP_FP8_IR;
     const bool x6 = precision == LP_F32_BF16X6;
-    if (bs < 128 || bs % 128 != 0) return fail(LP_E_INVALID, "mixed precision needs a block size >= 128");
-    const size_t esz = fp8 ? 1 : 2;
-    const int kq = x6 ? 6 * bs : bs;  // K of the tensor-core update
-    const size_t pan = (size_t)kq * n;      // one tensor-core operand
-    const int nblk = (n + 511) / 512;
-    LP_CHECK(panel_ensure(c, n, bs));
-    LP_CHECK(c->q.ensure(4 * esz * pan));
-    LP_CHECK(c->qs.ensure(2 * 6 * sizeof(float) * (size_t)kseg(bs) * nblk));
-    LP_CHECK(c->err.ensure(sizeof(int)));
+    if (user_bs < 128 || user_bs % 128 != 0) return fail(LP_E_INVALID, "mixed precision needs a block size >= 128");
     // the top / left products: FP32 accuracy (six segments) for the emulated-FP32
     // form.  For BF16 / E4M3 (the panel is rounded to them for the update anyway)
     // three segments, and plain BF16 operands from block 2048 on, where the panel
@@ -437,15 +465,24 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
     // flops per three segments.  Measured on one B200 (BF16+IR): n = 65536, block
     // 2048: 582 -> 638 TFLOP/s, one refinement either way; n = 32768, block 1024: no
     // gain, the plainer factors needing a second refinement.
-    const int nseg = x6 ? 6 : bs >= 2048 ? 1 : 3;
-    LP_CHECK(c->tri.ensure(3 * sizeof(float) * (size_t)bs * bs));
-    LP_CHECK(c->tq.ensure(2 * sizeof(__nv_bfloat16) * (size_t)nseg * bs * ((size_t)bs + n)));
+    const int nseg = x6 ? 6 : user_bs >= 2048 ? 1 : 3;
+    // the wide block's workspaces where device memory has ample room for them, else the caller's
+    int bs = x6 || (!fp8 && n >= 4096) ? std::max(kMixedBlock, user_bs) : user_bs;
+    size_t grow = 0, free_bytes = 0, total_bytes = 0;
+    LP_CHECK(mixed_ensure(c, precision, n, bs, nseg, &grow));
+    if (grow > 0 && bs > user_bs) LP_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    if (bs > user_bs && grow > free_bytes / 8) bs = user_bs;
+    LP_CHECK(mixed_ensure(c, precision, n, bs, nseg, nullptr));
+    const size_t esz = fp8 ? 1 : 2;
+    const int kq = x6 ? 6 * bs : bs;    // K of the tensor-core update
+    const size_t pan = (size_t)kq * n;  // one tensor-core operand
+    const int nblk = (n + 511) / 512;
     LP_CUDA(cudaMemsetAsync(c->err.ptr, 0, sizeof(int), st));
     uint8_t* q = static_cast<uint8_t*>(c->q.ptr);
     uint8_t* aqb[2] = {q, q + 2 * esz * pan};
     uint8_t* bqb[2] = {q + esz * pan, q + 3 * esz * pan};
     float* scb[2] = {static_cast<float*>(c->qs.ptr), static_cast<float*>(c->qs.ptr) + 6 * (size_t)kseg(bs) * nblk};
-    const int nb = n / bs;
+    const int nb = (n + bs - 1) / bs;
     const double b = bs;
 
     auto panel_q = [&](int K, cudaStream_t s) -> int {
@@ -453,17 +490,17 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
     };
     LP_CHECK(panel_q(0, st));
     for (int K = 0; K + 1 < nb; K++) {
-        const int rest = n - (K + 1) * bs;
-        const double r = rest;
+        const int rest = n - (K + 1) * bs, nx = std::min(bs, rest);  // nx: the next block
+        const double r = rest, x = nx;
         float* c11 = dA + (size_t)(K + 1) * bs * lda + (size_t)(K + 1) * bs;
         const uint8_t* aq = aqb[K & 1];
         const uint8_t* bq = bqb[K & 1];
         const float* sc = scb[K & 1];
         int e = prof_begin(c, st);
-        LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, 0, 0, bs, rest, kq, fp8, sc, nblk, st));
+        LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, 0, 0, nx, rest, kq, fp8, sc, nblk, st));
         if (rest > bs) LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, bs, 0, rest - bs, bs, kq, fp8, sc, nblk, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * b * r * b + 2.0 * (r - b) * b * b,
-                          8.0 * (b * r + (r - b) * b)));
+        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * x * r * b + 2.0 * (r - x) * x * b,
+                          8.0 * (x * r + (r - x) * x)));
         LP_CUDA(cudaEventRecord(c->ev_fork, st));
         LP_CUDA(cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
         LP_CHECK(panel_q(K + 1, c->aux));

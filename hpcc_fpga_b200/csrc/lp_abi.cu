@@ -292,15 +292,17 @@ int panel_ensure(lp_ctx* c, int n, int bs) {
 // The stages give the reference recurrences' values up to rounding; the exact
 // recurrences are lp_lu_block_dev, lp_top_update_dev, lp_left_update_dev.
 int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
-    // where device memory has no room for the operands of the order's block,
-    // the caller's own (its operands are what the call has always needed)
+    // the order's block where device memory has ample room for its operands, else the caller's
     int bs = f32_block(n);
-    if (bs > user_bs && bs > 128 && c->lt.ensure(2 * sizeof(float) * (size_t)bs * n) != LP_OK) {
-        cudaGetLastError();  // the allocation's
-        bs = std::max(128, user_bs);
+    // (never less than for one block of 512, so that a context warmed at one order has room for every smaller one)
+    auto lt_bytes = [&](int b) { return 2 * sizeof(float) * std::max((size_t)b * n, (size_t)512 * 512); };
+    if (bs > std::max(128, user_bs) && lt_bytes(bs) > c->lt.cap) {
+        size_t free_bytes = 0, total_bytes = 0;
+        LP_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+        if (lt_bytes(bs) > free_bytes / 8) bs = std::max(128, user_bs);
     }
-    LP_CHECK(c->lt.ensure(2 * sizeof(float) * (size_t)bs * n));
-    LP_CHECK(panel_ensure(c, n, bs));
+    LP_CHECK(c->lt.ensure(lt_bytes(bs)));
+    LP_CHECK(panel_ensure(c, n, 512));
     float* ltbuf[2] = {static_cast<float*>(c->lt.ptr), static_cast<float*>(c->lt.ptr) + (size_t)bs * n};
     const double b = bs;
     LP_CHECK(panel_f32(c, dA, n, lda, bs, 0, ltbuf[0], st));
@@ -472,7 +474,7 @@ int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, cud
     for (int s = 0; s < ns; s++) hmax = std::max(hmax, cuts[s + 1] - cuts[s]);
     const size_t ltf = (size_t)bs * hmax;
     LP_CHECK(c->lt.ensure(4 * sizeof(float) * ltf));
-    LP_CHECK(panel_ensure(c, n, bs));
+    LP_CHECK(panel_ensure(c, n, 512));
     if (c->copy_in == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
     if (host_out != nullptr && c->copy == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
     float* lt = static_cast<float*>(c->lt.ptr);

@@ -43,6 +43,23 @@ def test_gefa_block_of_the_order(ctx, dev, n):
     assert err <= 4 * n * FLT_EPS * np.abs(U).max() * np.abs(M).max()
 
 
+@pytest.mark.parametrize("prec,tol", [("bf16", 2e-3), ("fp8", 2e-2), ("f32_bf16x6", None)])
+@pytest.mark.parametrize("n,pad", [(128, 0), (896, 0), (1152, 4), (1920, 0), (2176, 0), (4224, 0)])
+def test_mixed_ragged_blocks(ctx, dev, prec, tol, n, pad):
+    """Tensor-core schedules whose order is no multiple of their inner block (one short block, a last block of 128
+    or 896): the bounds of the factors elsewhere (a few operand roundings; the emulated FP32 form 8 n eps)."""
+    A, _, _ = oracle.gen_baseline(n, seed=42, margin=1.0)
+    store = np.full((n, n + pad), 7.0, np.float32)
+    store[:, :n] = A
+    d = dev.put(store)
+    ctx.gefa_prec(prec, d.data_ptr(), n, n + pad, 128)
+    got = dev.get(d)
+    assert np.all(got[:, n:] == 7.0)
+    want = oracle.gefa_nopvt(A).astype(np.float64)
+    rel = np.abs(got[:, :n].astype(np.float64) - want).max() / np.abs(want).max()
+    assert rel < (tol or 8 * n * FLT_EPS)
+
+
 @pytest.mark.parametrize("n,bs", [(1088, 64), (2096, 16), (1536, 128)])
 def test_streamed_ragged_blocks(ctx, lp, n, bs):
     """Page-locked buffers (factored in row slabs while copied in) give the pageable path's bits."""
