@@ -36,67 +36,107 @@ namespace {
 
 constexpr int kLuThreads = 512;
 
+// The three recurrences below keep a column (row) in registers and run their
+// pivot loop rolled: a step writes each updated element one register down, so
+// the pivot's element is always x[0] and the loop body is the same code for
+// every pivot.  After eight steps the array is eight shorter (its upper
+// registers hold leftovers that nothing reads), and the next eight run as a
+// shorter body.  Unrolled over all pivots the straight-line code of a block
+// (several times the instruction cache) was fetched again for every chunk, the
+// more slowly the more the trailing update beside it used L2.
+//
 // (1) In-place LU of the NB x NB block at D (row stride SL), one warp; lane c
-// holds column c (x[j] = D[j][c]).  Kept out of line: inlined into the chunk
-// loop, its register array is not fully unrolled and lands in local memory.
+// holds column c, x[j] = D[k + j][c] at pivot k.
+template <typename T, int R, int SL>
+__device__ __forceinline__ void diag_steps(T (&x)[R], T* D, int k0, int lane, bool act) {
+    using A = Rn<T>;
+#pragma unroll 1
+    for (int k = k0; k < k0 + 8; k++) {
+        const bool below = lane > k;
+        const T d = A::neg_rcp(__shfl_sync(0xffffffffu, x[0], k));
+        const T scaled = A::mul(x[0], d);  // scaled row k: the multipliers
+        const T xk = below ? scaled : (lane == k ? d : x[0]);
+        if (act) D[k * SL + lane] = xk;
+#pragma unroll
+        for (int j = 1; j < R; j++) {
+            const T sjk = __shfl_sync(0xffffffffu, x[j], k);  // column k, row k + j
+            const T v = A::add(x[j], A::mul(xk, sjk));
+            x[j - 1] = below ? v : x[j];
+        }
+    }
+    if constexpr (R > 8) {
+        T y[R - 8];
+#pragma unroll
+        for (int j = 0; j < R - 8; j++) y[j] = x[j];
+        diag_steps<T, R - 8, SL>(y, D, k0 + 8, lane, act);
+    }
+}
+
 template <typename T, int NB, int SL>
 __device__ __noinline__ void diag_lu(T* D, int lane) {
-    using R = Rn<T>;
     T x[NB];
     const bool act = lane < NB;
 #pragma unroll
     for (int j = 0; j < NB; j++) x[j] = act ? D[j * SL + lane] : T(0);
-#pragma unroll
-    for (int k = 0; k < NB; k++) {
-        const bool below = lane > k;
-        const T d = R::neg_rcp(__shfl_sync(0xffffffffu, x[k], k));
-        const T scaled = R::mul(x[k], d);  // scaled row k: the multipliers
-        x[k] = below ? scaled : (lane == k ? d : x[k]);
-#pragma unroll
-        for (int j = k + 1; j < NB; j++) {
-            const T sjk = __shfl_sync(0xffffffffu, x[j], k);  // column k, row j
-            const T v = R::add(x[j], R::mul(x[k], sjk));
-            x[j] = below ? v : x[j];
-        }
-    }
-    if (act) {
-#pragma unroll
-        for (int j = 0; j < NB; j++) D[j * SL + lane] = x[j];
-    }
+    diag_steps<T, NB, SL>(x, D, 0, lane, act);
 }
 
 // (2a) Column `col` of the block row right of the diagonal block at k0:
-// for k: t_k *= D_kk; t_j += t_k D_jk (j > k).
+// for k: t_k *= D_kk; t_j += t_k D_jk (j > k).  D: the diagonal block at
+// pivot k, t: the column's element k.
+template <typename T, int R, int SL>
+__device__ __forceinline__ void top_steps(T (&x)[R], const T* D, T* t) {
+    using A = Rn<T>;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++, D += SL + 1, t += SL) {
+        const T xk = A::mul(x[0], D[0]);
+        *t = xk;
+#pragma unroll
+        for (int j = 1; j < R; j++)
+            x[j - 1] = j < R - 7 || k + j < R ? A::add(x[j], A::mul(xk, D[j * SL])) : x[j];
+    }
+    if constexpr (R > 8) {
+        T y[R - 8];
+#pragma unroll
+        for (int j = 0; j < R - 8; j++) y[j] = x[j];
+        top_steps<T, R - 8, SL>(y, D, t);
+    }
+}
+
 template <typename T, int NB, int SL>
 __device__ __forceinline__ void top_column(T* S, int k0, int col) {
-    using R = Rn<T>;
     T x[NB];
 #pragma unroll
     for (int j = 0; j < NB; j++) x[j] = S[(k0 + j) * SL + col];
-#pragma unroll
-    for (int k = 0; k < NB; k++) {
-        x[k] = R::mul(x[k], S[(k0 + k) * SL + k0 + k]);
-#pragma unroll
-        for (int j = k + 1; j < NB; j++) x[j] = R::add(x[j], R::mul(x[k], S[(k0 + j) * SL + k0 + k]));
-    }
-#pragma unroll
-    for (int j = 0; j < NB; j++) S[(k0 + j) * SL + col] = x[j];
+    top_steps<T, NB, SL>(x, S + k0 * SL + k0, S + k0 * SL + col);
 }
 
 // (2b) Row `row` of the block column below the diagonal block at k0:
 // for k, i > k: l_i += l_k D_ki.
+template <typename T, int R, int SL>
+__device__ __forceinline__ void left_steps(T (&x)[R], const T* D, T* l) {
+    using A = Rn<T>;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++, D += SL + 1, l++) {
+        const T xk = x[0];
+        *l = xk;
+#pragma unroll
+        for (int i = 1; i < R; i++) x[i - 1] = i < R - 7 || k + i < R ? A::add(x[i], A::mul(xk, D[i])) : x[i];
+    }
+    if constexpr (R > 8) {
+        T y[R - 8];
+#pragma unroll
+        for (int i = 0; i < R - 8; i++) y[i] = x[i];
+        left_steps<T, R - 8, SL>(y, D, l);
+    }
+}
+
 template <typename T, int NB, int SL>
 __device__ __forceinline__ void left_row(T* S, int k0, int row) {
-    using R = Rn<T>;
     T x[NB];
 #pragma unroll
     for (int i = 0; i < NB; i++) x[i] = S[row * SL + k0 + i];
-#pragma unroll
-    for (int k = 0; k < NB; k++)
-#pragma unroll
-        for (int i = k + 1; i < NB; i++) x[i] = R::add(x[i], R::mul(x[k], S[(k0 + k) * SL + k0 + i]));
-#pragma unroll
-    for (int i = 0; i < NB; i++) S[row * SL + k0 + i] = x[i];
+    left_steps<T, NB, SL>(x, S + k0 * SL + k0, S + row * SL + k0);
 }
 
 // (3) for one row r and column i: the chunk's NB updates of S[r][i] in
