@@ -159,9 +159,11 @@ __device__ __forceinline__ void diag_lu8(const float* dg, float* fd, int lane) {
 // Inverse of one triangle of the factored 32 x 32 block at db (row stride PS),
 // one warp, lane = column of the inverse.  LOWER: W^-1 = (diag(D_kk)^-1 -
 // strict-lower(D))^-1, written transposed; else V = (I - strict-upper(D))^-1.
-// Row by row, each a dot product with the rows before (after) it.
+// Row by row, each a dot product with the rows before (after) it.  One copy of
+// each form's straight-line code (10 KB) per kernel: inlined at its eight calls
+// every one of them was fetched cold.
 template <bool LOWER>
-__device__ __forceinline__ void invert32(const float* db, float* o, int lane) {
+__device__ __noinline__ void invert32(const float* db, float* o, int lane) {
     float x[32];
 #pragma unroll
     for (int q = 0; q < 32; q++) {
