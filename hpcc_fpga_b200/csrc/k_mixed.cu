@@ -488,31 +488,36 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int user_bs,
     auto panel_q = [&](int K, cudaStream_t s) -> int {
         return panel_tc(c, dA, n, lda, bs, K, nseg, PanelOut{fp8, x6, aqb[K & 1], bqb[K & 1], scb[K & 1], nblk}, s);
     };
-    LP_CHECK(panel_q(0, st));
-    for (int K = 0; K + 1 < nb; K++) {
+    cudaStream_t aux = c->aux;
+    LP_CUDA(cudaEventRecord(c->ev_fork, st));
+    LP_CUDA(cudaStreamWaitEvent(aux, c->ev_fork, 0));
+    LP_CHECK(panel_q(0, aux));
+    for (int K = 0; K + 1 < nb; K++) {  // streams as in gefa_f32
         const int rest = n - (K + 1) * bs, nx = std::min(bs, rest);  // nx: the next block
         const double r = rest, x = nx;
         float* c11 = dA + (size_t)(K + 1) * bs * lda + (size_t)(K + 1) * bs;
         const uint8_t* aq = aqb[K & 1];
         const uint8_t* bq = bqb[K & 1];
         const float* sc = scb[K & 1];
-        int e = prof_begin(c, st);
-        LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, 0, 0, nx, rest, kq, fp8, sc, nblk, st));
-        if (rest > bs) LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, bs, 0, rest - bs, bs, kq, fp8, sc, nblk, st));
-        LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * x * r * b + 2.0 * (r - x) * x * b,
+        if (K > 0) LP_CUDA(cudaStreamWaitEvent(aux, c->ev_join, 0));  // U_b of the last step
+        int e = prof_begin(c, aux);
+        LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, 0, 0, nx, rest, kq, fp8, sc, nblk, aux));
+        if (rest > bs) LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, bs, 0, rest - bs, bs, kq, fp8, sc, nblk, aux));
+        LP_CHECK(prof_end(c, aux, LP_STAGE_INNER, e, 2.0 * x * r * b + 2.0 * (r - x) * x * b,
                           8.0 * (x * r + (r - x) * x)));
-        LP_CUDA(cudaEventRecord(c->ev_fork, st));
-        LP_CUDA(cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
-        LP_CHECK(panel_q(K + 1, c->aux));
-        LP_CUDA(cudaEventRecord(c->ev_join, c->aux));
         if (rest > bs) {
+            LP_CUDA(cudaEventRecord(c->ev_fork, aux));
+            LP_CUDA(cudaStreamWaitEvent(st, c->ev_fork, 0));
             const double r2 = rest - bs;
             e = prof_begin(c, st);
             LP_CHECK(mixed_update(c, c11, lda, aq, bq, rest, bs, bs, rest - bs, rest - bs, kq, fp8, sc, nblk, st));
             LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, 2.0 * r2 * r2 * b, 8.0 * r2 * r2));
+            LP_CUDA(cudaEventRecord(c->ev_join, st));
         }
-        LP_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
+        LP_CHECK(panel_q(K + 1, aux));
     }
+    LP_CUDA(cudaEventRecord(c->ev_fork, aux));
+    LP_CUDA(cudaStreamWaitEvent(st, c->ev_fork, 0));
     int herr = 0;
     LP_CHECK(read_status(c, c->err.ptr, st, &herr));
     if (herr != 0)
