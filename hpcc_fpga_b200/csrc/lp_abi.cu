@@ -244,8 +244,10 @@ int left_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float*
 // diagonal block, then the block row right of it and the block column below
 // it in one launch (Lt written into `lt`, leading dimension the number of rows
 // below).  The left stage covers the rows below the diagonal block up to
-// row_end (default: all n).
-int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end) {
+// row_end (default: all n); the block column below the diagonal block is read
+// after column_ready (null: it is ready).
+int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end,
+              cudaEvent_t column_ready) {
     float* d = dA + (size_t)k0 * lda + k0;
     const int kb = std::min(bs, n - k0);
     const double b = kb;
@@ -257,6 +259,7 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
     if (rest <= 0) return LP_OK;
     const int below = (row_end < 0 ? n : row_end) - k0 - kb;
     const double r = rest, w = below;
+    if (column_ready != nullptr) LP_CUDA(cudaStreamWaitEvent(st, column_ready, 0));
     e = prof_begin(c, st);
     LP_CHECK(launch_tl(d, lda, inv, static_cast<const float*>(c->dt.ptr), kb, kb, d + kb, lda, rest,
                        d + (size_t)kb * lda, lda, below, lt, std::max(4, below), c->num_sms, st));
@@ -289,7 +292,11 @@ int panel_ensure(lp_ctx* c, int n, int bs) {
 // (lu, top, left) follow each other on the high-priority auxiliary stream,
 // U_b runs beside that panel on the main stream; they touch disjoint blocks,
 // and Lt is double-buffered so panel K+1 never overwrites the operand U_b
-// reads.  The event between the streams is on U_b's side: the chain has no
+// reads.  Only left reads the block column below the next diagonal block, so
+// that part of U_a runs on the side stream beside the rest of U_a and lu
+// (n = 2048 668 -> 618 us, n = 4096 2035 -> 1742, n = 8192 8800 -> 7810,
+// n = 16384 53.1 -> 51.3 ms).
+// The event between the streams is on U_b's side: the chain has no
 // event between U_a and its panel, and the one-CTA lu kernel is resident before
 // U_b's CTAs fill the SMs.  With the event on the panel's side (U_a on the main
 // stream) n = 2048 took 773 us for 717, n = 4096 2245 for 2182.
@@ -322,12 +329,18 @@ int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st)
         float* lt = ltbuf[K & 1];
         float* c11 = d + (size_t)bs * lda + bs;
         if (K > 0) LP_CUDA(cudaStreamWaitEvent(aux, c->ev_join, 0));  // U_b of the last step
-        int e = prof_begin(c, aux);
+        int e = 0;
+        if (rest > nx) {
+            LP_CUDA(cudaEventRecord(c->ev_side, aux));
+            LP_CUDA(cudaStreamWaitEvent(c->aux2, c->ev_side, 0));
+            e = prof_begin(c, c->aux2);
+            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda, lda, lt + nx, rest, top, lda, rest - nx, nx, bs, c->aux2));
+            LP_CHECK(prof_end(c, c->aux2, LP_STAGE_INNER, e, inner_flops(r - x, x, b), inner_bytes(r - x, x, b)));
+            LP_CUDA(cudaEventRecord(c->ev_side_done, c->aux2));
+        }
+        e = prof_begin(c, aux);
         LP_CHECK(launch_sgemm_update(c11, lda, lt, rest, top, lda, nx, rest, bs, aux));
-        if (rest > nx)
-            LP_CHECK(launch_sgemm_update(c11 + (size_t)nx * lda, lda, lt + nx, rest, top, lda, rest - nx, nx, bs, aux));
-        LP_CHECK(prof_end(c, aux, LP_STAGE_INNER, e, inner_flops(x, r, b) + inner_flops(r - x, x, b),
-                          inner_bytes(x, r, b) + inner_bytes(r - x, x, b)));
+        LP_CHECK(prof_end(c, aux, LP_STAGE_INNER, e, inner_flops(x, r, b), inner_bytes(x, r, b)));
         if (rest > nx) {
             LP_CUDA(cudaEventRecord(c->ev_fork, aux));
             LP_CUDA(cudaStreamWaitEvent(st, c->ev_fork, 0));
@@ -338,7 +351,8 @@ int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st)
             LP_CHECK(prof_end(c, st, LP_STAGE_INNER, e, inner_flops(r2, r2, b), inner_bytes(r2, r2, b)));
             LP_CUDA(cudaEventRecord(c->ev_join, st));
         }
-        LP_CHECK(panel_f32(c, dA, n, lda, bs, (K + 1) * bs, ltbuf[(K + 1) & 1], aux));
+        LP_CHECK(panel_f32(c, dA, n, lda, bs, (K + 1) * bs, ltbuf[(K + 1) & 1], aux, -1,
+                           rest > nx ? c->ev_side_done : nullptr));
     }
     LP_CUDA(cudaEventRecord(c->ev_fork, aux));
     LP_CUDA(cudaStreamWaitEvent(st, c->ev_fork, 0));

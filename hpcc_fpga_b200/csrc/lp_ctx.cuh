@@ -38,7 +38,8 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
 // Panel work of the block step at row k0 (lu, top, left; Lt into lt), on
 // stream st; the left stage covers the rows below the diagonal block up to
 // row_end (-1: n).
-int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end = -1);
+int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end = -1,
+              cudaEvent_t column_ready = nullptr);
 // Workspaces of the panel stages for order n and (inner) block bs.
 int panel_ensure(lp_ctx* c, int n, int bs);
 // k_panel.cu: LU of a 128 x 128 diagonal block, its 32 x 32 inverses into inv
