@@ -850,9 +850,14 @@ int launch_umma_update(float* c, int ldc, const void* aq, int aq_rows, const voi
     // on B200 (BF16 factorization alone): block 512, n = 32768: 8 free SMs +9 %
     // over none; block 1024, n = 32768: 32 instead of 16 50.1 -> 48.1 ms (E4M3
     // 46.4 -> 47.1); block 512, n = 16384: 14.4 -> 13.8 ms (E4M3 14.9 -> 14.2);
-    // emulated FP32, n = 16384: 23.4 -> 22.4 ms; 48 no further gain.
-    constexpr int kPanelSMs = 32;
-    const int usable = sms - kPanelSMs > 1 ? sms - kPanelSMs : 1;
+    // emulated FP32, n = 16384: 23.4 -> 22.4 ms; 48 no further gain.  Where the
+    // update is the longer side -- large remainders of the E4M3 form (narrow
+    // tiles above K = 512) and of the emulated FP32 form (six segments) -- 16:
+    // E4M3 n = 65536, block 2048 238.5 -> 231.6 ms, n = 32768 44.2 -> 43.6;
+    // emulated FP32 n = 32768 138.5 -> 133.5 ms; BF16 there 42.3 -> 42.9, so not.
+    const bool update_bound = (fp8 || k > 2048) && std::min(m, n) > 24576;
+    const int panel_sms = update_bound ? 16 : 32;
+    const int usable = sms - panel_sms > 1 ? sms - panel_sms : 1;
     if (pair) {
         const int tiles_n = n / 256, tiles = tiles_n * (m / 256);
         const int clusters = std::max(1, std::min(tiles, usable / 2));
