@@ -17,7 +17,8 @@
 // beside two workers on one scheduler its instructions wait for theirs.  A
 // further warp inverts each finished 32 x 32 diagonal block of both triangles
 // for k_tl while the workers go on.  Measured on one B200 per block, beside
-// 31 us for k_lu_block<128>: 22.2 us.
+// 31 us for k_lu_block<128>: 22.2 us, and some 2.5 us less since the inversions
+// are one copy of code each (invert32).
 //
 // k_tl applies top and left to strips of 32 or 64 columns / rows, all bs of
 // the block's unknowns at once.  With X the strip (left: transposed) the

@@ -272,10 +272,11 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
 // the chain of a step (what bounds small orders) and large blocks read and
 // write the trailing matrix less often (what bounds large ones).  Measured on
 // one B200, factorization alone in us with blocks of 128 / 256 / 512:
-//   n =  512: 158 / 155 / 139         n =  6144: 5093 / 4784 / 5063
-//   n = 1024: 341 / 359 / 356         n =  8192: 9772 / 9104 / 9124
-//   n = 2048: 773 / 824 / 903         n = 12288: 27395 / 25235 / 24717
-//   n = 4096: 2199 / 2222 / 2435      n = 16384: 59371 / 55091 / 53552
+//   n =  512: 139 / 146 / 129         n =  6144: 4112 / 3949 / 4260
+//   n = 1024: 290 / 319 / 342         n =  8192: 8183 / 7806 / 8019
+//   n = 2048: 618 / 696 / 788         n =  9216: 11091 / 10585 / 10767
+//   n = 3968: 1673 / 1670 / 1901      n = 12288: 24273 / 23099 / 23044
+//   n = 4096: 1747 / 1752 / 1962      n = 16384: 54642 / 51983 / 51272
 static int f32_block(int n) { return n <= 512 ? 512 : n < 4096 ? 128 : n < 9216 ? 256 : 512; }
 
 // Workspaces of the FP32 panel: the inverses of every 128-wide diagonal block
