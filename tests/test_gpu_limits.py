@@ -1,0 +1,46 @@
+"""Calls at the limits of what the entry points accept: pivots over the whole
+float range, matrices whose factors are exact numbers (so that nothing may be
+lost to a reordering), pointers that are not aligned, and waits that run out."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+FLT_EPS = float(np.finfo(np.float32).eps)
+
+
+@pytest.mark.parametrize("prec,n,bs", [("f32", 128, 16), ("f32", 256, 64), ("f32", 640, 128), ("bf16", 128, 128),
+                                       ("fp8", 128, 128), ("f32_bf16x6", 128, 128)])
+def test_reciprocal_pivots_over_the_float_range(ctx, dev, prec, n, bs):
+    """A diagonal matrix is its own U: the factors hold -1/u_kk, correctly rounded (the quotient in double rounded to
+    float), for pivots of every exponent whose reciprocal is finite, subnormal pivots and reciprocals among them."""
+    rng = np.random.default_rng(n)
+    u = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-127, 128, n)) * rng.choice([-1.0, 1.0], n)
+    u[:8] = [1e38, -3e38, 5e-39, -1.1e-38, 2.0 ** 126, 2.0 ** 127, 2.0 ** -126, 2.0 ** -127]
+    u = u.astype(np.float32)
+    d = dev.put(np.diag(u))
+    ctx.gefa_prec(prec, d.data_ptr(), n, n, bs)
+    got = dev.get(d)
+    want = (-1.0 / u.astype(np.float64)).astype(np.float32)
+    assert np.all(np.isfinite(want)) and np.any(np.abs(want) < 2.0 ** -126)
+    assert np.array_equal(np.diag(got), want)
+    assert np.count_nonzero(got) == n
+
+
+def test_solution_with_pivots_at_the_ends_of_the_range(ctx, dev):
+    """A dominant matrix with a pivot of 1e38 and one of 5e-39 in a whole 128 block: the solution of a right-hand side
+    M * ones within 8 n eps (the two rows' own rounding: subnormal numbers near 5e-39 carry 21 bits)."""
+    n = 128
+    rng = np.random.default_rng(5)
+    S = rng.uniform(-0.5, 0.5, (n, n))
+    S[np.arange(n), np.arange(n)] = np.abs(S).sum(1) + 1.0
+    S[40, 40] = 1e38
+    S[9, :], S[:, 9] = 0.0, 0.0
+    S[9, 9] = 5e-39
+    S = S.astype(np.float32)
+    b = S.astype(np.float64).sum(0).astype(np.float32)
+    dA, dB = dev.put(S), dev.put(b)
+    ctx.gefa(dA.data_ptr(), n, n, 128)
+    ctx.gesl(dA.data_ptr(), n, n, dB.data_ptr(), 1)
+    assert np.abs(dev.get(dB) - 1.0).max() <= 8 * n * FLT_EPS
