@@ -46,7 +46,7 @@ __device__ __forceinline__ void bar_sync() { asm volatile("bar.sync %0, %1;\n" :
 // -1 / x, correctly rounded over the whole range of floats, as in the exact
 // kernels: an approximate reciprocal flushes subnormal results, so that a pivot
 // above 2^126 would get multipliers of zero.  0.3 us more per 128 pivots than
-that reciprocal and one Newton step.
+// that reciprocal and one Newton step.
 __device__ __forceinline__ float neg_rcp(float x) { return -__frcp_rn(x); }
 
 __device__ __forceinline__ void ld4(float* d, const float* s) {
