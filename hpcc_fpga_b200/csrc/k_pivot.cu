@@ -120,10 +120,10 @@ __device__ __forceinline__ unsigned long long key_word(unsigned rank, unsigned r
 
 // One more unsuccessful poll: false (and the error word set) past the limit or
 // when another CTA gave up.
-__device__ __forceinline__ bool keep_polling(unsigned& spins, int* err) {
+__device__ __forceinline__ bool keep_polling(unsigned& spins, unsigned limit, int* err) {
     if ((++spins & 255u) != 0) return true;
     if (*reinterpret_cast<volatile int*>(err) != 0) return false;
-    if (spins > kSpinLimit) {
+    if (spins > limit) {
         atomicExch(err, 1);
         return false;
     }
@@ -131,11 +131,12 @@ __device__ __forceinline__ bool keep_polling(unsigned& spins, int* err) {
 }
 
 // The value of the message word at p once it carries `tag`.
-__device__ __forceinline__ unsigned poll_word(const unsigned long long* p, unsigned tag, int* err, bool& ok) {
+__device__ __forceinline__ unsigned poll_word(const unsigned long long* p, unsigned tag, unsigned limit, int* err,
+                                              bool& ok) {
     unsigned spins = 0;
     unsigned long long w = ld_word(p);
     while ((unsigned)(w >> 32) != tag) {
-        if (!keep_polling(spins, err)) {
+        if (!keep_polling(spins, limit, err)) {
             ok = false;
             break;
         }
@@ -156,7 +157,12 @@ __device__ __forceinline__ unsigned poll_word(const unsigned long long* p, unsig
 // s + 1, and so had read all it needs of s.  Measured on one B200, 128 steps:
 // m = 4500 855 -> 330 us (a grid barrier, then keys and row, each an L2 round
 // trip, before), m = 900 280 us.
-// R is a multiple of 4.
+// R is a multiple of 4.  A wait of more than `limit` polls gives up: the error
+// word is set and every CTA returns.  The panel's pivots start as "no exchange",
+// so that the kernels already queued behind it then find valid rows in ipvt
+// whatever it held before.  STALL (tests): the last CTA never sends its first
+// candidate.
+template <bool STALL>
 __global__ void __launch_bounds__(PT, 1)
     k_piv_panel(float* __restrict__ a, int lda, int n, int k0, int kb, int R, int* __restrict__ ipvt,
                 unsigned char* __restrict__ sync) {
@@ -173,6 +179,8 @@ __global__ void __launch_bounds__(PT, 1)
     const int row0 = g * R;                       // M rows k0 + row0 ... belong to this CTA
     const int nr = max(0, min(R, n - k0 - row0));
     const size_t cbase = (size_t)k0 + row0;       // their storage column
+    constexpr unsigned limit = STALL ? kSpinLimit / 8 : kSpinLimit;
+    if (g == 0 && tid < kb) ipvt[k0 + tid] = k0 + tid;  // (kb <= PT; see above)
     for (int c = 0; c < kb; c++) {  // every copy in flight before the first wait
         const float* src = a + (size_t)(k0 + c) * lda + cbase;
         for (int r = tid; r < nr; r += PT) cp_async4(slab + c * R + r, src + r);
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(PT, 1)
             bi = __reduce_min_sync(0xffffffffu, v == best ? i : 0xFFFFFFFFu);
         }
         // publish the candidate, its panel row and, from the owner, row k
-        if (tid == PT - 1) {
+        if (tid == PT - 1 && !(STALL && kk == 0 && g == G - 1)) {
             const unsigned long long w = key_word(best, bi & ((1u << kKeyRowBits) - 1u), tag);
             asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(keys + par * GMAX + g), "l"(w) : "memory");
         }
@@ -249,7 +257,7 @@ __global__ void __launch_bounds__(PT, 1)
                 if (q < G) {
                     unsigned spins = 0;
                     while (((unsigned)w[j] & ((1u << kKeyTagBits) - 1u)) != tag && ok) {
-                        ok = keep_polling(spins, err);
+                        ok = keep_polling(spins, limit, err);
                         w[j] = ld_word(keys + par * GMAX + q);
                     }
                     const unsigned x = (unsigned)(w[j] >> 32), y = (unsigned)(k0 + q * R) + ((unsigned)w[j] >> kKeyTagBits);
@@ -296,15 +304,15 @@ __global__ void __launch_bounds__(PT, 1)
         const unsigned long long* won = rows + ((size_t)par * GMAX + wg) * RW;
         if (c0 < kb) {
             if (half == 0) {
-                const float v = __uint_as_float(poll_word(won + c0, tag, err, ok));
+                const float v = __uint_as_float(poll_word(won + c0, tag, limit, err, ok));
                 newk[c0] = v;
                 if (p != k && own_k) slab[c0 * R + rk] = v;  // exchange M rows k and p over the whole panel
             } else if (own_p) {
-                slab[c0 * R + rp] = __uint_as_float(poll_word(krow + par * PBMAX + c0, tag, err, ok));
+                slab[c0 * R + rp] = __uint_as_float(poll_word(krow + par * PBMAX + c0, tag, limit, err, ok));
             }
         }
         if (warp == PT / 32 - 1) {  // the reciprocal, by two lanes
-            const unsigned h = lane < 2 ? poll_word(won + PBMAX + lane, tag, err, ok) : 0u;
+            const unsigned h = lane < 2 ? poll_word(won + PBMAX + lane, tag, limit, err, ok) : 0u;
             const unsigned hi = __shfl_sync(0xffffffffu, h, 1);
             if (lane == 0) s_rcp = __hiloint2double((int)hi, (int)h);
         }
@@ -704,9 +712,10 @@ int piv_init_attrs() {
     LP_CUDA(cudaGetDevice(&dev));
     LP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa{};
-    LP_CUDA(cudaFuncGetAttributes(&fa, k_piv_panel));
+    LP_CUDA(cudaFuncGetAttributes(&fa, k_piv_panel<false>));
     g_panel_smem_max = optin - (int)fa.sharedSizeBytes;
-    LP_CUDA(cudaFuncSetAttribute(k_piv_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_panel_smem_max));
+    LP_CUDA(cudaFuncSetAttribute(k_piv_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_panel_smem_max));
+    LP_CUDA(cudaFuncSetAttribute(k_piv_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_panel_smem_max));
     LP_CUDA(cudaFuncSetAttribute(k_piv_rows<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<128>()));
     LP_CUDA(cudaFuncSetAttribute(k_piv_rows<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<64>()));
     LP_CUDA(cudaFuncGetAttributes(&fa, k_piv_gesl<128>));
@@ -735,7 +744,8 @@ static void panel_grid(int m, int kb, int sms, int* G, int* R) {
     *G = (m + *R - 1) / *R;
 }
 
-int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, int sms,
+// stall (tests): the first pivot step's wait runs out, after some 0.2 s.
+int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, bool stall, int sms,
                      cudaStream_t st) {
     const int m = n - k0;
     int G = 0, R = 0;
@@ -744,7 +754,9 @@ int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsign
     if (kb > PBMAX || G > GMAX || R >= 1 << kKeyRowBits || n >= 1 << kKeyTagBits || (long long)smem > g_panel_smem_max)
         return fail(LP_E_INVALID, "pivoting panel: matrix too large for the panel width");
     void* args[] = {&a, &lda, &n, &k0, &kb, &R, &ipvt, &sync};
-    LP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_piv_panel), dim3(G), dim3(PT), args, smem, st));
+    const void* fn = stall ? reinterpret_cast<const void*>(k_piv_panel<true>)
+                           : reinterpret_cast<const void*>(k_piv_panel<false>);
+    LP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(PT), args, smem, st));
     count_launch();
     return LP_OK;
 }

@@ -775,7 +775,7 @@ int lp_ctx_read_timeline(lp_ctx* c, lp_stage_event* out, int max, int* count) {
 }
 
 int lp_ctx_test_stall(lp_ctx* c, int site) {
-    if (c == nullptr || site < 0 || site > LP_STALL_GESL) return fail(LP_E_INVALID, "lp_ctx_test_stall: bad argument");
+    if (c == nullptr || site < 0 || site > LP_STALL_PIVOT) return fail(LP_E_INVALID, "lp_ctx_test_stall: bad argument");
     c->stall_site = site;
     return LP_OK;
 }

@@ -115,7 +115,7 @@ int gesl_f64_on_f32(lp_ctx* c, const float* a, int n, int lda, double* b, int nr
 int piv_init_attrs();
 size_t piv_sync_bytes();
 int piv_panel_width(int n, int sms);
-int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, int sms,
+int launch_piv_panel(float* a, int lda, int n, int k0, int kb, int* ipvt, unsigned char* sync, bool stall, int sms,
                      cudaStream_t st);
 int launch_piv_rows(float* a, int lda, int k0, int pb, int first, int last, const int* ipvt, float* at, int ldat,
                     int sms, cudaStream_t st);

@@ -11,7 +11,7 @@ namespace {
 int piv_error(lp_ctx* c, cudaStream_t st, const char* who) {
     int herr = 0;
     LP_CHECK(read_status(c, static_cast<unsigned char*>(c->psync.ptr) + 4, st, &herr));
-    if (herr != 0) return fail(LP_E_TIMEOUT, std::string(who) + ": a grid barrier did not complete in time");
+    if (herr != 0) return fail(LP_E_TIMEOUT, std::string(who) + ": a bounded wait expired");
     return LP_OK;
 }
 
@@ -44,10 +44,12 @@ int gefa_pvt_block(lp_ctx* c, float* a, int n, int lda, int* ipvt, int pb, cudaS
     unsigned char* sync = static_cast<unsigned char*>(c->psync.ptr);
     float* at = static_cast<float*>(c->pat.ptr);
     LP_CUDA(cudaMemsetAsync(sync, 0, piv_sync_bytes(), st));
+    const bool stall = c->stall_site == LP_STALL_PIVOT;  // (failure-path tests: the first panel)
+    c->stall_site = stall ? LP_STALL_NONE : c->stall_site;
     auto panel = [&](int k0, cudaStream_t s) -> int {
         const int m = n - k0, kb = std::min(pb, m);
         const int e = prof_begin(c, s);
-        LP_CHECK(launch_piv_panel(a, lda, n, k0, kb, ipvt, sync, c->num_sms, s));
+        LP_CHECK(launch_piv_panel(a, lda, n, k0, kb, ipvt, sync, stall && k0 == 0, c->num_sms, s));
         return prof_end(c, s, LP_STAGE_LU, e, (double)m * kb * kb, 8.0 * m * kb);
     };
     // storage rows [r0 + first, r0 + last): interchanges, block row, trailing update

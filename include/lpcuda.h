@@ -135,13 +135,16 @@ int lp_ctx_read_timeline(lp_ctx* ctx, lp_stage_event* out, int max, int* count);
  * Every wait inside this library's kernels is bounded: a kernel that gives up
  * records an error word, finishes without touching memory it does not own,
  * and the entry point returns LP_E_TIMEOUT with the context still usable.
- * lp_ctx_test_stall arms that path for tests: the next substitution sweep on
- * this context (LP_STALL_GESL) makes one tile wait on a word that nothing
- * sets, so its bounded wait (250 ms) runs out; the call then returns
- * LP_E_TIMEOUT and the affected solution entries are NaN.  The stall is used
- * once; site 0 disarms it. */
+ * lp_ctx_test_stall arms that path for tests, once (site 0 disarms it):
+ * LP_STALL_GESL: the next substitution sweep on this context makes one tile
+ * wait on a word that nothing sets, so its bounded wait (250 ms) runs out; the
+ * call then returns LP_E_TIMEOUT and the affected solution entries are NaN.
+ * LP_STALL_PIVOT: in the next pivoting factorization one CTA never sends its
+ * first candidate, so the others' wait (about 0.2 s) runs out; the call returns
+ * LP_E_TIMEOUT, the matrix is undefined and ipvt holds valid row numbers. */
 #define LP_STALL_NONE 0
 #define LP_STALL_GESL 1
+#define LP_STALL_PIVOT 2
 int lp_ctx_test_stall(lp_ctx* ctx, int site);
 
 /* ---- block stages (device pointers) -------------------------------------

@@ -44,3 +44,38 @@ def test_solution_with_pivots_at_the_ends_of_the_range(ctx, dev):
     ctx.gefa(dA.data_ptr(), n, n, 128)
     ctx.gesl(dA.data_ptr(), n, n, dB.data_ptr(), 1)
     assert np.abs(dev.get(dB) - 1.0).max() <= 8 * n * FLT_EPS
+
+
+@pytest.mark.parametrize("n,kind", [(100, "dev"), (644, "dev"), (1156, "dev"), (644, "calculate")])
+def test_pivot_wait_that_runs_out_reports_timeout(ctx, dev, lp, torch_cuda, n, kind):
+    """A pivot step's wait that runs out (lp_ctx_test_stall) comes back as LP_E_TIMEOUT; nothing outside the matrix is
+    written, ipvt holds rows of the matrix (stale entries in it, here the numbers of padding columns, are not used),
+    and the next call gives the oracle's pivots."""
+    rng = np.random.default_rng(n)
+    A = rng.uniform(-0.5, 0.5, (n, n)).astype(np.float32)
+    A[np.arange(n), rng.permutation(n)] += np.float32(np.sqrt(n))
+    want = oracle.gefa_pvt(A)[1]
+    ctx.test_stall(lp.LP_STALL_PIVOT)
+    if kind == "calculate":
+        with pytest.raises(lp.LpError) as e:
+            ctx.calculate_pvt(A.copy(), A.sum(0))
+        assert e.value.status == lp.LP_E_TIMEOUT
+        assert np.array_equal(ctx.calculate_pvt(A.copy(), A.sum(0))[1], want)
+        return
+    pad = 64
+    store = np.full((n + 2, n + pad), 7.0, np.float32)
+    store[1:n + 1, :n] = A
+    d = dev.put(store)
+    piv = torch_cuda.full((n,), n + 1, dtype=torch_cuda.int32, device="cuda")
+    piv += torch_cuda.arange(n, dtype=torch_cuda.int32, device="cuda") % (pad - 2)
+    torch_cuda.cuda.synchronize()
+    with pytest.raises(lp.LpError) as e:
+        ctx.gefa_pvt(d.data_ptr() + 4 * (n + pad), n, n + pad, piv.data_ptr())
+    assert e.value.status == lp.LP_E_TIMEOUT and "bounded wait" in str(e.value)
+    got, p = dev.get(d), piv.cpu().numpy()
+    assert np.all(got[0] == 7.0) and np.all(got[n + 1] == 7.0) and np.all(got[1:n + 1, n:] == 7.0)
+    assert np.all((p >= np.arange(n)) & (p < n))
+    d = dev.put(store)
+    ctx.gefa_pvt(d.data_ptr() + 4 * (n + pad), n, n + pad, piv.data_ptr())
+    ctx.sync()
+    assert np.array_equal(piv.cpu().numpy(), want)
