@@ -580,6 +580,7 @@ int panel_init_attrs() {
 }
 
 int launch_lu128(float* a, int lda, float* inv, float* dt, int lddt, cudaStream_t st) {
+    if (lda % 4 != 0 || !aligned16(a)) return fail(LP_E_INVALID, "128 block LU: block must be 16-byte aligned, lda % 4 == 0");
     LP_CUDA(launch_pdl(k_lu128, dim3(1), dim3(LUT), kLu128Smem, st, a, lda, inv, dt, lddt));
     count_launch();
     return LP_OK;
@@ -593,8 +594,8 @@ int launch_tl(const float* d, int ldd, const float* inv, const float* dt, int ld
               int ncols, float* l, int ldl, int nrows, float* lt, int ldlt, int sms, cudaStream_t st) {
     if (ncols <= 0 && nrows <= 0) return LP_OK;
     if (bs % PB != 0 || bs > 512 || ncols % 4 != 0 || nrows % 4 != 0 || ldd % 4 != 0 || ldt % 4 != 0 || ldl % 4 != 0 ||
-        ldlt % 4 != 0 || lddt % 4 != 0)
-        return fail(LP_E_INVALID, "top/left update: sizes must be multiples of 4 and the block of 128");
+        ldlt % 4 != 0 || lddt % 4 != 0 || !aligned16(d) || !aligned16(t) || !aligned16(l) || !aligned16(lt))
+        return fail(LP_E_INVALID, "top/left update: sizes must be multiples of 4, the block of 128, pointers 16-byte aligned");
     TlArgs p{d, inv, dt, ldd, bs, lddt, t, ldt, ncols, 0, l, ldl, nrows, lt, ldlt};
     // narrow strips while they leave SMs idle (less work per CTA), wide ones (fewer loads per product) once they do not
     const int wide = (ncols + 63) / 64 + (nrows + 63) / 64;

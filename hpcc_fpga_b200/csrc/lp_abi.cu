@@ -800,6 +800,7 @@ int lp_lu_block_dev(lp_ctx* c, float* dA, int lda, int bs) {
         return fail(LP_E_INVALID, "lp_lu_block_dev: bs must be a power of two in [16, 512], lda >= bs, lda % 4 == 0");
     LP_CUDA(cudaSetDevice(c->device));
     if (bs <= 128) return launch_lu_small(dA, lda, bs, c->stream);
+    if (!aligned16(dA)) return fail(LP_E_INVALID, "lp_lu_block_dev: blocks above 128 must be 16-byte aligned");
     LP_CHECK(panel_ensure(c, bs, bs));
     return lu_stage(c, dA, lda, bs, block_inv(c, 0), c->stream);
 }

@@ -152,7 +152,9 @@ int lp_ctx_test_stall(lp_ctx* ctx, int site);
  * launches.  bs is the block size (power of two, 16..512). */
 
 /* lu: factor the bs x bs diagonal block at dA in place
- * (hpl_torus_PCIE.cl:211-446; arithmetic of linpack_data.cpp:166-196). */
+ * (hpl_torus_PCIE.cl:211-446; arithmetic of linpack_data.cpp:166-196): in the
+ * reference's exact operation order up to bs 128, blocked (equal to rounding)
+ * above.  lda a multiple of 4; above bs 128 dA 16-byte aligned. */
 int lp_lu_block_dev(lp_ctx* ctx, float* dA, int lda, int bs);
 /* top: update the bs x ncols block row right of a factored diagonal block
  * (hpl_torus_PCIE.cl:452-582; host loop test_kernel_communication.cpp:776-789). */

@@ -79,3 +79,23 @@ def test_pivot_wait_that_runs_out_reports_timeout(ctx, dev, lp, torch_cuda, n, k
     ctx.gefa_pvt(d.data_ptr() + 4 * (n + pad), n, n + pad, piv.data_ptr())
     ctx.sync()
     assert np.array_equal(piv.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("off", [1, 2, 3])
+@pytest.mark.parametrize("bs", [64, 128, 256, 512])
+def test_lu_block_at_an_unaligned_address(ctx, dev, lp, bs, off):
+    """lp_lu_block_dev takes blocks of up to 128 at any float's address (the exact factors), and refuses larger ones
+    before anything is launched."""
+    A = oracle.gen_reference(bs)[0]
+    store = np.full(bs * bs + 8, 7.0, np.float32)
+    store[off:off + bs * bs] = A.ravel()
+    d = dev.put(store)
+    if bs > 128:
+        with pytest.raises(lp.LpError) as e:
+            ctx.lu_block(d.data_ptr() + 4 * off, bs, bs)
+        assert e.value.status == lp.LP_E_INVALID
+        assert np.array_equal(dev.get(d), store)
+        return
+    ctx.lu_block(d.data_ptr() + 4 * off, bs, bs)
+    store[off:off + bs * bs] = oracle.gefa_nopvt(A).ravel()
+    assert np.array_equal(dev.get(d), store)
