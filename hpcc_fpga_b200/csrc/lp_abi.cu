@@ -726,7 +726,7 @@ int lp_ctx_sync(lp_ctx* c) {
     if (c == nullptr) return fail(LP_E_INVALID, "lp_ctx_sync: null context");
     LP_CUDA(cudaSetDevice(c->device));
     LP_CUDA(cudaStreamSynchronize(c->stream));
-    return LP_OK;
+    return gesl64_status(c, 0, "lp_ctx_sync");
 }
 
 int lp_ctx_device_name(lp_ctx* c, char* buf, int buflen) {
@@ -775,7 +775,7 @@ int lp_ctx_read_timeline(lp_ctx* c, lp_stage_event* out, int max, int* count) {
 }
 
 int lp_ctx_test_stall(lp_ctx* c, int site) {
-    if (c == nullptr || site < 0 || site > LP_STALL_PIVOT) return fail(LP_E_INVALID, "lp_ctx_test_stall: bad argument");
+    if (c == nullptr || site < 0 || site > LP_STALL_GESL64) return fail(LP_E_INVALID, "lp_ctx_test_stall: bad argument");
     c->stall_site = site;
     return LP_OK;
 }

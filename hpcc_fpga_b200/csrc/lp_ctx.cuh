@@ -108,7 +108,10 @@ int gesl_status(lp_ctx* c, cudaStream_t st, const char* who);
 // FP64 form (lp_fp64.cu): factorization and substitution in double.
 int gefa_f64(lp_ctx* c, double* a, int n, int lda, int bs, cudaStream_t st);
 int gesl64_init_attrs();
-int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st);
+// (slot: 0 for a caller that does not wait, 1 for one that does)
+int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, int slot, cudaStream_t st);
+// LP_E_TIMEOUT (once) if a substitution of that slot gave up; call it after a wait for the stream.
+int gesl64_status(lp_ctx* c, int slot, const char* who);
 // The same substitution in FP64 arithmetic on FP32 factors (widened exactly).
 int gesl_f64_on_f32(lp_ctx* c, const float* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st);
 // Partial pivoting (k_pivot.cu): kernels of the blocked LINPACK-convention LU.
@@ -179,6 +182,7 @@ struct lp_ctx {
     lp::Workspace gw;    // substitution: published values of the sweeps (64-bit pairs) and their tickets
     lp::Workspace gerr;  // error word of the substitution sweeps (non-zero: a bounded wait gave up)
     int* hstat = nullptr;                     // pinned host copy of an error word
+    int* f64stat = nullptr;                   // pinned words set by an FP64 substitution that gives up (lp_fp64.cu)
     int stall_site = 0;                       // lp_ctx_test_stall: the next wait of this site never completes
     lp::Workspace dA, dA0, dB;                // host-entry-point matrix, original copy, FP32 rhs
     int fac_n = 0, fac_lda = 0, fac_prec = -1;  // factors resident in dA (lp_factor); fac_n 0: none
@@ -232,6 +236,8 @@ struct lp_ctx {
         hgm_cap = 0;
         if (hstat != nullptr) cudaFreeHost(hstat);
         hstat = nullptr;
+        if (f64stat != nullptr) cudaFreeHost(f64stat);
+        f64stat = nullptr;
     }
 };
 

@@ -99,18 +99,19 @@ __global__ void __launch_bounds__(128) k_inv64(const FT* __restrict__ a, int lda
 constexpr size_t kInv64Smem = sizeof(double) * (SB * (SB + 1) + 64 * 33);
 
 // Bounded grid barrier of a cooperative launch; the counter only grows.
-__device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, int* err) {
+// absent (tests): this CTA does not arrive.
+__device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, unsigned limit, bool absent, int* err) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        atomicAdd(bar, 1u);
+        if (!absent) atomicAdd(bar, 1u);
         int ok = 1;
         unsigned spins = 0, v;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if (v >= target) break;
-            if ((++spins & 255u) == 0 && (*reinterpret_cast<volatile int*>(err) != 0 || spins > kSpinLimit64)) {
+            if ((++spins & 255u) == 0 && (*reinterpret_cast<volatile int*>(err) != 0 || spins > limit)) {
                 atomicExch(err, 1);
                 ok = 0;
                 break;
@@ -132,11 +133,12 @@ __device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, int*
 // the two sweeps (the forward sweep's results are the second's input).  A
 // chain of 2 n / 64 short steps, where one launch per block and direction took
 // 15 us each (n = 6144: 192 launches, 2.9 ms).  A barrier that gives up leaves
-// NaN in the solutions.
+// NaN in the solutions and sets *gave_up, a word in page-locked host memory.
+// stall (tests): CTA 0 never arrives at the first barrier.
 template <typename FT>
 __global__ void __launch_bounds__(GT, 1)
     k_gesl64(const FT* __restrict__ a, int lda, int n, const double* __restrict__ op, double* w1, double* w2, double* b,
-             int ldb, int nrhs, unsigned* sync) {
+             int ldb, int nrhs, unsigned* sync, int* gave_up, int stall) {
     extern __shared__ __align__(16) double sm[];
     double* Ob = sm;                          // 2 x SB x SB: the block's inverse, alternating
     double* in = Ob + 2 * SB * SB;            // RMAX x SB: the block's accumulated values
@@ -233,7 +235,12 @@ __global__ void __launch_bounds__(GT, 1)
         if (s + 1 == steps) break;
         range(s + 1, i0, i1);
         load_rows(s + 1, i0 + lane, i0 + lane < i1);
-        if (!grid_sync64(sync, (unsigned)(s + 1) * (unsigned)G, err)) {
+        if (!grid_sync64(sync, (unsigned)(s + 1) * (unsigned)G, stall != 0 ? kSpinLimit64 / 16 : kSpinLimit64,
+                         stall != 0 && g == 0 && s == 0, err)) {
+            if (tid == 0) {
+                *reinterpret_cast<volatile int*>(gave_up) = 1;
+                __threadfence_system();
+            }
             for (int idx = g * GT + tid; idx < nrhs * n; idx += G * GT)
                 b[(size_t)(idx / n) * ldb + idx % n] = __longlong_as_double(0x7ff8000000000000ll);
             return;
@@ -381,7 +388,8 @@ int gefa_f64(lp_ctx* c, double* a, int n, int lda, int bs, cudaStream_t st) {
 }
 
 template <typename FT>
-static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st) {
+static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrhs, int ldb, int* gave_up,
+                      cudaStream_t st) {
     const int g0 = nrhs < RMAX ? nrhs : RMAX, nblk = (n + SB - 1) / SB;
     const size_t ops = 2 * (size_t)nblk * SB * SB;
     LP_CHECK(c->f64w.ensure(sizeof(double) * (2 * (size_t)n * g0 + ops + 2)));
@@ -393,6 +401,8 @@ static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrh
     k_inv64<FT><<<nblk, 128, kInv64Smem, st>>>(a, lda, n, op);
     LP_CUDA(cudaGetLastError());
     count_launch();
+    int stall = c->stall_site == LP_STALL_GESL64;  // (failure-path tests: the first group)
+    if (stall) c->stall_site = LP_STALL_NONE;
     // enough CTAs that a step's products are one pass of 32 unknowns each, at most one per SM
     const int grid = std::max(1, std::min(c->num_sms, (n + 31) / 32));
     for (int r0 = 0; r0 < nrhs; r0 += RMAX) {
@@ -401,10 +411,11 @@ static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrh
         LP_CUDA(cudaMemcpy2DAsync(w1, sizeof(double) * n, bb, sizeof(double) * ldb, sizeof(double) * n, g,
                                   cudaMemcpyDeviceToDevice, st));
         LP_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st));
-        void* args[] = {&a, &lda, &n, &op, &w1, &w2, &bb, &ldb, &g, &sync};
+        void* args[] = {&a, &lda, &n, &op, &w1, &w2, &bb, &ldb, &g, &sync, &gave_up, &stall};
         LP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_gesl64<FT>), dim3(grid), dim3(GT), args,
                                             kGesl64Smem, st));
         count_launch();
+        stall = 0;
     }
     return prof_end(c, st, LP_STAGE_GESL, e, 2.0 * n * n * nrhs,
                     (double)sizeof(FT) * n * n * ((nrhs + RMAX - 1) / RMAX));
@@ -418,12 +429,33 @@ int gesl64_init_attrs() {
     return LP_OK;
 }
 
-int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st) {
-    return gesl64_any(c, a, n, lda, b, nrhs, ldb, st);
+// The host words that a substitution sets when it gives up (page-locked, so
+// they can be read once the stream was waited for): [0] for lp_gesl_f64_dev,
+// which does not wait, [1] for the calls that do.
+static int gesl64_words(lp_ctx* c) {
+    if (c->f64stat != nullptr) return LP_OK;
+    LP_CUDA(cudaHostAlloc(&c->f64stat, 2 * sizeof(int), cudaHostAllocPortable));
+    c->f64stat[0] = c->f64stat[1] = 0;
+    return LP_OK;
+}
+
+int gesl64_status(lp_ctx* c, int slot, const char* who) {
+    if (c->f64stat == nullptr) return LP_OK;
+    volatile int* w = c->f64stat + slot;
+    if (*w == 0) return LP_OK;
+    *w = 0;
+    return fail(LP_E_TIMEOUT, std::string(who) + ": a bounded wait of the FP64 substitution expired "
+                                                 "(its solutions are NaN)");
+}
+
+int gesl_f64(lp_ctx* c, const double* a, int n, int lda, double* b, int nrhs, int ldb, int slot, cudaStream_t st) {
+    LP_CHECK(gesl64_words(c));
+    return gesl64_any(c, a, n, lda, b, nrhs, ldb, c->f64stat + slot, st);
 }
 
 int gesl_f64_on_f32(lp_ctx* c, const float* a, int n, int lda, double* b, int nrhs, int ldb, cudaStream_t st) {
-    return gesl64_any(c, a, n, lda, b, nrhs, ldb, st);
+    LP_CHECK(gesl64_words(c));
+    return gesl64_any(c, a, n, lda, b, nrhs, ldb, c->f64stat + 1, st);
 }
 
 }  // namespace lp
@@ -443,7 +475,7 @@ int lp_gesl_f64_dev(lp_ctx* c, const double* dLU, int n, int lda, double* dB, in
     if (c == nullptr || dLU == nullptr || dB == nullptr) return fail(LP_E_INVALID, "lp_gesl_f64_dev: null argument");
     if (n <= 0 || lda < n || nrhs <= 0 || ldb < n) return fail(LP_E_INVALID, "lp_gesl_f64_dev: bad sizes");
     LP_CUDA(cudaSetDevice(c->device));
-    return gesl_f64(c, dLU, n, lda, dB, nrhs, ldb, c->stream);
+    return gesl_f64(c, dLU, n, lda, dB, nrhs, ldb, 0, c->stream);
 }
 
 int lp_calculate_f64(lp_ctx* c, int n, int lda, int bs, int repetitions, double* A, double* b, double* gefa_times,
@@ -466,9 +498,10 @@ int lp_calculate_f64(lp_ctx* c, int n, int lda, int bs, int repetitions, double*
         LP_CUDA(cudaEventRecord(c->ev[0], st));
         LP_CHECK(gefa_f64(c, dA, n, lda, bs, st));
         LP_CUDA(cudaEventRecord(c->ev[1], st));
-        LP_CHECK(gesl_f64(c, dA, n, lda, dB, 1, n, st));
+        LP_CHECK(gesl_f64(c, dA, n, lda, dB, 1, n, 1, st));
         LP_CUDA(cudaEventRecord(c->ev[2], st));
         LP_CUDA(cudaStreamSynchronize(st));
+        LP_CHECK(gesl64_status(c, 1, "lp_calculate_f64"));
         gefa_times[rep] = event_s64(c->ev[0], c->ev[1]);
         gesl_times[rep] = event_s64(c->ev[1], c->ev[2]);
     }

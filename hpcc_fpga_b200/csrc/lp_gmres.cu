@@ -326,5 +326,6 @@ extern "C" int lp_gmres_dev(lp_ctx* c, const float* dA0, int lda, const float* d
         t->ir_iters = steps;
         t->hpl_resid = resid;
     }
+    LP_CHECK(gesl64_status(c, 1, "lp_gmres_dev"));  // (else its NaN would read as LP_E_NUMERIC)
     return s;
 }

@@ -26,7 +26,7 @@ LP_E_BUDGET = -7
 LP_E_NODEVICE = -8
 
 LP_F32, LP_BF16_IR, LP_FP8_IR, LP_F32_BF16X6 = 0, 1, 2, 3
-LP_STALL_NONE, LP_STALL_GESL, LP_STALL_PIVOT = 0, 1, 2
+LP_STALL_NONE, LP_STALL_GESL, LP_STALL_PIVOT, LP_STALL_GESL64 = 0, 1, 2, 3
 PRECISIONS = {"f32": LP_F32, "bf16": LP_BF16_IR, "fp8": LP_FP8_IR, "f32_bf16x6": LP_F32_BF16X6}
 
 _F32P = np.ctypeslib.ndpointer(dtype=np.float32, flags="C_CONTIGUOUS")

@@ -86,6 +86,9 @@ int lp_ctx_create(int device, lp_ctx** out);
 int lp_ctx_destroy(lp_ctx* ctx);
 /* The cudaStream_t the *_dev calls are ordered on (as void*). */
 int lp_ctx_stream(lp_ctx* ctx, void** stream);
+/* Waits for the calls ordered on the context's stream.  LP_E_TIMEOUT if a
+ * bounded wait of a substitution of lp_gesl_f64_dev (which itself does not
+ * wait for the device) expired since the last lp_ctx_sync. */
 int lp_ctx_sync(lp_ctx* ctx);
 /* Name of the device ("NVIDIA B200"), for the JSON "device" key
  * (hpcc_benchmark.hpp:501 getDeviceName). */
@@ -141,10 +144,13 @@ int lp_ctx_read_timeline(lp_ctx* ctx, lp_stage_event* out, int max, int* count);
  * call then returns LP_E_TIMEOUT and the affected solution entries are NaN.
  * LP_STALL_PIVOT: in the next pivoting factorization one CTA never sends its
  * first candidate, so the others' wait (about 0.2 s) runs out; the call returns
- * LP_E_TIMEOUT, the matrix is undefined and ipvt holds valid row numbers. */
+ * LP_E_TIMEOUT, the matrix is undefined and ipvt holds valid row numbers.
+ * LP_STALL_GESL64: in the next FP64 substitution one CTA never arrives at the
+ * first grid barrier (about 0.2 s); see lp_gesl_f64_dev. */
 #define LP_STALL_NONE 0
 #define LP_STALL_GESL 1
 #define LP_STALL_PIVOT 2
+#define LP_STALL_GESL64 3
 int lp_ctx_test_stall(lp_ctx* ctx, int site);
 
 /* ---- block stages (device pointers) -------------------------------------
@@ -257,7 +263,12 @@ int lp_gesl_dev_noalloc(const float* dLU, int n, int lda, float* dB, int nrhs, i
  * gefa_ref_nopvt / gesl_ref_nopvt of the double build.  bs 64, 128 or 256, n a
  * multiple of bs, lda even, dA 16-byte aligned. */
 int lp_gefa_f64_dev(lp_ctx* ctx, double* dA, int n, int lda, int bs);
-/* Forward + back substitution, nrhs right-hand sides as rows of dB. */
+/* Forward + back substitution, nrhs right-hand sides as rows of dB.  It does
+ * not wait for the device: should a bounded wait of its kernels expire, the
+ * solutions of that group of 16 right-hand sides are NaN and the next
+ * lp_ctx_sync returns LP_E_TIMEOUT.  (lp_calculate_f64 and lp_gmres_dev, which
+ * wait, return LP_E_TIMEOUT themselves.)  The first call on a context and
+ * calls of a larger size than before allocate. */
 int lp_gesl_f64_dev(lp_ctx* ctx, const double* dLU, int n, int lda, double* dB, int nrhs, int ldb);
 
 /* ---- LU with partial pivoting (device pointers) ------------------------------

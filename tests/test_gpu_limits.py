@@ -99,3 +99,39 @@ def test_lu_block_at_an_unaligned_address(ctx, dev, lp, bs, off):
     ctx.lu_block(d.data_ptr() + 4 * off, bs, bs)
     store[off:off + bs * bs] = oracle.gefa_nopvt(A).ravel()
     assert np.array_equal(dev.get(d), store)
+
+
+@pytest.mark.parametrize("api,n,nrhs", [("gesl_f64", 20, 1), ("gesl_f64", 200, 17), ("calculate", 256, 1), ("gmres", 256, 1)])
+def test_fp64_substitution_wait_that_runs_out_reports_timeout(ctx, dev, lp, api, n, nrhs):
+    """A barrier of the FP64 substitution that runs out (lp_ctx_test_stall) comes back as LP_E_TIMEOUT: from the calls
+    that wait, and for lp_gesl_f64_dev from the next lp_ctx_sync, with NaN in the first group of 16 right-hand sides
+    and the second group's solutions as they should be.  The next call succeeds."""
+    A = oracle.gen_reference(n)[0]
+    LU = oracle.gefa_nopvt(A.astype(np.float64))
+    B = np.tile(A.astype(np.float64).sum(0), (nrhs, 1))
+
+    def run():
+        if api == "gesl_f64":
+            dLU, dB = dev.put(LU), dev.put(B)
+            ctx.gesl_f64(dLU.data_ptr(), n, n, dB.data_ptr(), nrhs)
+            try:
+                ctx.sync()
+            finally:
+                x = dB.cpu().numpy()
+                assert np.all(np.abs(x[16:] - 1.0) < 1e-9)
+                assert np.all(np.isnan(x[:16])) or np.all(np.abs(x - 1.0) < 1e-9)
+            return x
+        if api == "calculate":
+            b = B[0].copy()
+            ctx.calculate_f64(A.astype(np.float64), b, 128)
+            return b
+        dA, dLU, db = dev.put(A), dev.put(LU.astype(np.float32)), dev.put(B[0])
+        dx = dev.empty(n, np.float64)
+        ctx.gmres(dA.data_ptr(), n, dLU.data_ptr(), n, db.data_ptr(), dx.data_ptr(), tol=1e-12)
+        return dev.get(dx)
+
+    ctx.test_stall(lp.LP_STALL_GESL64)
+    with pytest.raises(lp.LpError) as e:
+        run()
+    assert e.value.status == lp.LP_E_TIMEOUT and "bounded wait" in str(e.value)
+    assert np.abs(run() - 1.0).max() < 1e-9
