@@ -379,10 +379,9 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
         LP_CUDA(cudaGetLastError());
     }
     const TriInverses inv{winv, vinv, vlt};
-    float* dinv = block_inv(c, K * bs);
     int e = prof_begin(c, s);
     const int kb = std::min(bs, n - K * bs);
-    LP_CHECK(lu_stage(c, d, lda, kb, dinv, s, beside ? &inv : nullptr));
+    LP_CHECK(lu_stage(c, d, lda, kb, s, beside ? &inv : nullptr));
     LP_CHECK(prof_end(c, s, LP_STAGE_LU, e, 2.0 * kb * kb * (double)kb / 3.0, 8.0 * kb * (double)kb));
     if (rest <= 0) return LP_OK;
     const double r = rest;
@@ -390,7 +389,7 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
 
     e = prof_begin(c, s);
     if (!beside)  // one chunk: the two recurrences in one launch
-        LP_CHECK(launch_tl(d, lda, dinv, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt, bs,
+        LP_CHECK(launch_tl(d, lda, static_cast<const float*>(c->dt.ptr), bs, bs, winv, bs, bs, vinv, bs, bs, vlt, bs,
                            c->num_sms, s));
     LP_CHECK(split_rows(winv, bs, bs, bs, a_top, s, nseg));
     LP_CHECK(split_trans(vinv, bs, bs, bs, b_left, s, nseg, true));
@@ -438,7 +437,6 @@ static int mixed_ensure(lp_ctx* c, int precision, int n, int bs, int nseg, size_
     const size_t esz = precision == LP_FP8_IR ? 1 : 2, kq = precision == LP_F32_BF16X6 ? 6 * (size_t)bs : bs;
     const size_t nblk = (n + 511) / 512, b = bs;
     const struct { Workspace* w; size_t bytes; } need[] = {
-        {&c->dinv, sizeof(float) * kInvFloats * (size_t)((n + 127) / 128)},
         {&c->dt, sizeof(float) * b * b},
         {&c->q, 4 * esz * kq * n},
         {&c->qs, 2 * 6 * sizeof(float) * (size_t)kseg(bs) * nblk},

@@ -2,7 +2,7 @@
 // diagonal block and the triangular updates of the block row and column
 // beside it.  They compute the recurrences of k_lu.cu / k_trsm.cu (gefa's lu,
 // top and left, LINPACK/src/host/linpack_data.cpp:166-196) with fused
-// multiply-adds and 32 x 32 inverses, so their results agree with those to
+// multiply-adds and sums in another order, so their results agree with those to
 // rounding; the stage entry points that promise the reference's exact
 // operation order keep the other kernels.
 //
@@ -14,22 +14,22 @@
 // diagonal warp brings the next 8 x 8 diagonal block up to date and factors
 // it, redundantly in every lane's registers (a chain of eight reciprocals
 // without an exchange between threads).  It has an SM partition to itself:
-// beside two workers on one scheduler its instructions wait for theirs.  A
-// further warp inverts each finished 32 x 32 diagonal block of both triangles
-// for k_tl while the workers go on.  Measured on one B200 per block, beside
-// 31 us for k_lu_block<128>: 22.2 us, and some 2.5 us less since the inversions
-// are one copy of code each (invert32).
+// beside two workers on one scheduler its instructions wait for theirs.
+// Measured on one B200 per block, beside 31 us for k_lu_block<128>: 19.6 us.
 //
 // k_tl applies top and left to strips of 32 or 64 columns / rows, all bs of
-// the block's unknowns at once.  With X the strip (left: transposed) the
-// update is, per 32-wide chunk c, X_c = inv_c (X0_c + sum_{b<c} D_cb X_b),
-// inv_c the inverse 32 x 32 triangle.  One launch covers the block row and
-// the block column (they are independent), the strip stays in shared memory,
-// and per 128 rows a thread keeps its outputs in registers.  9.1 us beside a
-// 128 block (384 rows and columns), 21 us beside 256, 59 us beside 512, where
-// top and left took 13 us each beside 128 and a chain of such launches,
-// transposes and GEMMs beside wider blocks.  The whole chain of a 128 step (LU,
-// top and left, update of the 384 behind it): 39 us, was 70.
+// the block's unknowns at once.  With X the strip (left: transposed) each
+// 32-wide chunk c of it becomes X0_c + sum_{b<c} D_cb X_b and then runs the
+// recurrence of its own triangle, one column per lane (solve32): a product with
+// the triangle's inverse in its place was 1 us shorter per 128 rows, but lost
+// what the condition of the triangle allows on matrices that are not dominant,
+// and the inversions cost k_lu128 2 us.  One launch covers the block row and the
+// block column (they are independent), the strip stays in shared memory, and
+// per 128 rows a thread keeps its outputs in registers.  9.9 us beside a 128
+// block (384 rows and columns), 22.6 us beside 256 and 61 us beside 512 (512
+// rows and columns), where top and left took 13 us each beside 128 and a chain
+// of such launches, transposes and GEMMs beside wider blocks.  The whole chain of
+// a 128 step (LU, top and left, update of the 384 behind it): 36 us, was 70.
 #include "lp_ctx.cuh"
 
 namespace lp {
@@ -152,51 +152,13 @@ __device__ __forceinline__ void diag_lu8(const float* dg, float* fd, int lane) {
     }
 }
 
-// Inverse of one triangle of the factored 32 x 32 block at db (row stride PS),
-// one warp, lane = column of the inverse.  LOWER: W^-1 = (diag(D_kk)^-1 -
-// strict-lower(D))^-1, written transposed; else V = (I - strict-upper(D))^-1.
-// Row by row, each a dot product with the rows before (after) it.  One copy of
-// each form's straight-line code (10 KB) per kernel: inlined at its eight calls
-// every one of them was fetched cold.
-template <bool LOWER>
-__device__ __noinline__ void invert32(const float* db, float* o, int lane) {
-    float x[32];
-#pragma unroll
-    for (int q = 0; q < 32; q++) {
-        const int r = LOWER ? q : 31 - q;
-        const float* row = db + r * PS;
-        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-            if (LOWER ? c >= r : c + 3 <= r) continue;
-            const float4 v = *reinterpret_cast<const float4*>(row + c);
-            if (LOWER ? c < r : c > r) s0 = fmaf(v.x, x[c], s0);
-            if (LOWER ? c + 1 < r : c + 1 > r) s1 = fmaf(v.y, x[c + 1], s1);
-            if (LOWER ? c + 2 < r : c + 2 > r) s2 = fmaf(v.z, x[c + 2], s2);
-            if (LOWER ? c + 3 < r : c + 3 > r) s3 = fmaf(v.w, x[c + 3], s3);
-        }
-        const float s = ((s0 + s1) + (s2 + s3)) + (r == lane ? 1.0f : 0.0f);
-        x[r] = LOWER ? s * row[r] : s;
-    }
-    if (LOWER) {
-#pragma unroll
-        for (int r = 0; r < 32; r += 4)
-            *reinterpret_cast<float4*>(o + lane * 32 + r) = make_float4(x[r], x[r + 1], x[r + 2], x[r + 3]);
-    } else {
-#pragma unroll
-        for (int r = 0; r < 32; r++) o[r * 32 + lane] = x[r];
-    }
-}
-
 // Warps of k_lu128 (warp % 4 is its SM partition): 0 the diagonal warp, 4 and 8
-// leave at once, 11 the inverses, the other eight the workers.
-constexpr int LUT = 384;
+// leave at once, the other eight the workers.
+constexpr int LUT = 352;
 
-// inv: for each 32-wide chunk c = 0..3 the operators of k_tl, 32 x 32 each:
-// W_c^-1 transposed (block 2c), V_c (block 2c + 1).  dt (leading dimension
-// lddt): the block's lower triangle outside those chunks, transposed.
-__global__ void __launch_bounds__(LUT, 1) k_lu128(float* __restrict__ a, int lda, float* __restrict__ inv,
-                                                  float* __restrict__ dt, int lddt) {
+// dt (leading dimension lddt): the block's lower triangle transposed (rows of
+// 32-wide chunks whole, so a chunk's own upper triangle comes along).
+__global__ void __launch_bounds__(LUT, 1) k_lu128(float* __restrict__ a, int lda, float* __restrict__ dt, int lddt) {
     extern __shared__ __align__(16) float sm[];
     float* F = sm;                     // the factored block
     float* panels = F + PB * PS;       // two pairs of panels, alternating by step
@@ -225,22 +187,6 @@ __global__ void __launch_bounds__(LUT, 1) k_lu128(float* __restrict__ a, int lda
             diag_lu8(dg, fds + ((b + 1) & 1) * 64, lane);
             bar_sync<1, 288>();
         }
-        bar_sync<5, 320>();
-        invert32<false>(F + 96 * (PS + 1), inv + 7 * 1024, lane);
-        return;
-    }
-    if (warp == 11) {
-        bar_sync<2, 288>();
-        invert32<true>(F, inv, lane);
-        invert32<false>(F, inv + 1024, lane);
-        bar_sync<3, 288>();
-        invert32<true>(F + 32 * (PS + 1), inv + 2 * 1024, lane);
-        invert32<false>(F + 32 * (PS + 1), inv + 3 * 1024, lane);
-        bar_sync<4, 288>();
-        invert32<true>(F + 64 * (PS + 1), inv + 4 * 1024, lane);
-        invert32<false>(F + 64 * (PS + 1), inv + 5 * 1024, lane);
-        bar_sync<5, 320>();
-        invert32<true>(F + 96 * (PS + 1), inv + 6 * 1024, lane);
         return;
     }
     if ((warp & 3) == 0) return;
@@ -333,9 +279,6 @@ __global__ void __launch_bounds__(LUT, 1) k_lu128(float* __restrict__ a, int lda
 #pragma unroll
             for (int k = 0; k < 8; k++) F[(k0 + k) * PS + e] = x[k];
         }
-        if (b == 3) asm volatile("bar.arrive 2, 288;\n" ::: "memory");
-        if (b == 7) asm volatile("bar.arrive 3, 288;\n" ::: "memory");
-        if (b == 11) asm volatile("bar.arrive 4, 288;\n" ::: "memory");
         if (b == 15) break;
         // rank-8 update of what is still open (warps skip finished groups of rows and columns; values left of or
         // above the open part are never read again)
@@ -353,14 +296,14 @@ __global__ void __launch_bounds__(LUT, 1) k_lu128(float* __restrict__ a, int lda
                 rank8<false, false>(c, lp, tp);
         }
     }
-    bar_sync<5, 320>();
-    // the factored block, and its lower triangle outside the 32-wide chunks transposed (lane = row)
+    bar_sync<2, 256>();
+    // the factored block, and its lower triangle transposed (lane = row)
     for (int idx = w * 32 + lane; idx < PB * PB / 4; idx += 256) {
         const int r = idx >> 5, i = (idx & 31) * 4;
         *reinterpret_cast<float4*>(a + (size_t)r * lda + i) = *reinterpret_cast<const float4*>(F + r * PS + i);
     }
-    for (int q = w; q < 48; q += 8) {  // 32 rows x 4 columns each
-        const int rb = q < 8 ? 1 : (q < 24 ? 2 : 3), k = 4 * (q - (rb == 1 ? 0 : (rb == 2 ? 8 : 24)));
+    for (int q = w; q < 80; q += 8) {  // 32 rows x 4 columns each
+        const int rb = q < 8 ? 0 : (q < 24 ? 1 : (q < 48 ? 2 : 3)), k = 4 * (q - 4 * rb * (rb + 1));
         const int r = 32 * rb + lane;
         const float4 v = *reinterpret_cast<const float4*>(F + r * PS + k);
         float* o = dt + (size_t)k * lddt + r;
@@ -377,7 +320,6 @@ constexpr size_t kLu128Smem = sizeof(float) * (PB * PS + 32 * PS + 4 * 64);
 
 struct TlArgs {
     const float* d;    // factored diagonal block (bs x bs, leading dimension ldd)
-    const float* inv;  // its 32 x 32 inverses (8 per 128 rows, k_lu128)
     const float* dt;   // its lower triangle transposed (leading dimension lddt; top only)
     int ldd, bs, lddt;
     float* t;          // block row: bs x ncols
@@ -422,10 +364,36 @@ __device__ __forceinline__ void tile_mul(float2 (&y)[RT][2], const float* op, co
     }
 }
 
+// The recurrence of a 32-row chunk, one column per lane: x_k *= D_kk (scale),
+// x_i += x_k D_ki (i > k).  x: the column in the strip (row stride XS), d: D_ki
+// at d[k * PS + i]; out: the column in global memory, or null.
+template <int XS>
+__device__ __forceinline__ void solve32(float* xs, const float* d, bool scale, float* out, int ldo) {
+    float x[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) x[i] = xs[i * XS];
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+        x[k] *= scale ? d[k * PS + k] : 1.0f;
+#pragma unroll
+        for (int i = (k + 1) / 4 * 4; i < 32; i += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(d + k * PS + i);
+            if (i > k) x[i] = fmaf(x[k], v.x, x[i]);
+            if (i + 1 > k) x[i + 1] = fmaf(x[k], v.y, x[i + 1]);
+            if (i + 2 > k) x[i + 2] = fmaf(x[k], v.z, x[i + 2]);
+            if (i + 3 > k) x[i + 3] = fmaf(x[k], v.w, x[i + 3]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        xs[i * XS] = x[i];
+        if (out != nullptr) out[(size_t)i * ldo] = x[i];
+    }
+}
+
 // Per 128 rows B of the block: acc = sum over the rows before B of D X (tiles
-// of 32 x 128), then four chunks of 32 rows: X_c = inv_c (X0_c + acc_c), and
-// acc of the later chunks += D X_c.  A tile of a chunk holds the chunk's
-// inverse in the chunk's own columns and D right of it.  256 threads even for
+// of 32 x 128), then four chunks of 32 rows: the recurrence of X0_c + acc_c
+// within the chunk, and acc of the later chunks += D X_c.  256 threads even for
 // narrow strips: 128 with twice the outputs each load less per product but
 // were slower (12.5 against 10.4 us for 128 rows, 72 against 61 us for 512).
 template <int TW>
@@ -453,14 +421,10 @@ __global__ void __launch_bounds__(TT, 2) k_tl(const TlArgs p) {
             float* dst = ring + (in % TR) * (32 * PS);
             const int own = ik - 4 * iB;  // >= 0: chunk `own` of the block itself
             const float* src = off + (size_t)(32 * ik) * ldo + PB * iB;
-            const float* inv = p.inv + (size_t)(2 * ik + (top ? 0 : 1)) * 1024;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int k = (tid >> 5) + 8 * q, i = lane * 4, rel = i - 32 * own;
-                if (own < 0 || rel >= 32)
-                    cp_async_vec16(dst + k * PS + i, src + (size_t)k * ldo + i);
-                else if (rel >= 0)
-                    cp_async_vec16(dst + k * PS + i, inv + k * 32 + rel);
+                const int k = (tid >> 5) + 8 * q, i = lane * 4;
+                if (i >= 32 * own) cp_async_vec16(dst + k * PS + i, src + (size_t)k * ldo + i);
             }
             if (own == 3)
                 iB++, ik = 0;
@@ -505,9 +469,6 @@ __global__ void __launch_bounds__(TT, 2) k_tl(const TlArgs p) {
     // a warp covers 4 RT rows x 32 columns (4 x 8 threads)
     const int wr = warp / CG, wc = warp - wr * CG;
     const int row = RT * (4 * wr + (lane >> 3)), col = 32 * wc + 4 * (lane & 7);
-    // the chunks' own 32 x TW products, spread over all threads: QT rows each
-    constexpr int QT = CG;
-    const int qrow = QT * (4 * wr + (lane >> 3));
     int tile = 0;
     for (int B = 0; B < nb; B++) {
         float2 acc[RT][2];
@@ -524,7 +485,7 @@ __global__ void __launch_bounds__(TT, 2) k_tl(const TlArgs p) {
                 continue;
             }
             const int c = ck - 4 * B;
-            if ((row >> 5) == c) {  // X0_c + acc, by the warps that hold it
+            if ((row >> 5) == c) {  // X0_c + acc and its recurrence, by the two warps that hold it
 #pragma unroll
                 for (int i = 0; i < RT; i++) {
                     float4* q = reinterpret_cast<float4*>(XB + (row + i) * XS + col);
@@ -532,22 +493,15 @@ __global__ void __launch_bounds__(TT, 2) k_tl(const TlArgs p) {
                     v.x += acc[i][0].x, v.y += acc[i][0].y, v.z += acc[i][1].x, v.w += acc[i][1].y;
                     *q = v;
                 }
-            }
-            __syncthreads();
-            float2 y[QT][2];
-#pragma unroll
-            for (int i = 0; i < QT; i++) y[i][0] = y[i][1] = make_float2(0.0f, 0.0f);
-            // the inverse is zero for k > row
-            tile_mul<QT, XS>(y, op + 32 * c + qrow, XB + 32 * c * XS + col, 4 * QT * (wr + 1));
-            __syncthreads();
-            const int k = PB * B + 32 * c + qrow;
-#pragma unroll
-            for (int i = 0; i < QT; i++) {
-                const float4 v = make_float4(y[i][0].x, y[i][0].y, y[i][1].x, y[i][1].y);
-                *reinterpret_cast<float4*>(X + (k + i) * XS + col) = v;
-                if (col < width) {
-                    float* o = top ? p.t + (size_t)(k + i) * p.ldt : p.lt + (size_t)(k + i) * p.ldlt;
-                    *reinterpret_cast<float4*>(o + s0 + col) = v;
+                if (CG == 1)
+                    bar_sync<1, 64>();  // (each warp holds half of the rows)
+                else
+                    __syncwarp();
+                const int cl = 32 * wc + lane, k = PB * B + 32 * c;
+                if (CG == 2 || (warp & 1) == 0) {
+                    float* o = top ? p.t + (size_t)k * p.ldt : p.lt + (size_t)k * p.ldlt;
+                    solve32<XS>(X + k * XS + cl, op + 32 * c, top, cl < width ? o + s0 + cl : nullptr,
+                                top ? p.ldt : p.ldlt);
                 }
             }
             if (c < 3) {
@@ -579,9 +533,9 @@ int panel_init_attrs() {
     return LP_OK;
 }
 
-int launch_lu128(float* a, int lda, float* inv, float* dt, int lddt, cudaStream_t st) {
+int launch_lu128(float* a, int lda, float* dt, int lddt, cudaStream_t st) {
     if (lda % 4 != 0 || !aligned16(a)) return fail(LP_E_INVALID, "128 block LU: block must be 16-byte aligned, lda % 4 == 0");
-    LP_CUDA(launch_pdl(k_lu128, dim3(1), dim3(LUT), kLu128Smem, st, a, lda, inv, dt, lddt));
+    LP_CUDA(launch_pdl(k_lu128, dim3(1), dim3(LUT), kLu128Smem, st, a, lda, dt, lddt));
     count_launch();
     return LP_OK;
 }
@@ -590,13 +544,13 @@ int launch_lu128(float* a, int lda, float* inv, float* dt, int lddt, cudaStream_
 // factored block d, in place; bs a multiple of 128, at most 512; ncols and
 // nrows multiples of 4 (either may be 0).  dt: d's lower triangle transposed
 // (needed for ncols > 0).
-int launch_tl(const float* d, int ldd, const float* inv, const float* dt, int lddt, int bs, float* t, int ldt,
+int launch_tl(const float* d, int ldd, const float* dt, int lddt, int bs, float* t, int ldt,
               int ncols, float* l, int ldl, int nrows, float* lt, int ldlt, int sms, cudaStream_t st) {
     if (ncols <= 0 && nrows <= 0) return LP_OK;
     if (bs % PB != 0 || bs > 512 || ncols % 4 != 0 || nrows % 4 != 0 || ldd % 4 != 0 || ldt % 4 != 0 || ldl % 4 != 0 ||
         ldlt % 4 != 0 || lddt % 4 != 0 || !aligned16(d) || !aligned16(t) || !aligned16(l) || !aligned16(lt))
         return fail(LP_E_INVALID, "top/left update: sizes must be multiples of 4, the block of 128, pointers 16-byte aligned");
-    TlArgs p{d, inv, dt, ldd, bs, lddt, t, ldt, ncols, 0, l, ldl, nrows, lt, ldlt};
+    TlArgs p{d, dt, ldd, bs, lddt, t, ldt, ncols, 0, l, ldl, nrows, lt, ldlt};
     // narrow strips while they leave SMs idle (less work per CTA), wide ones (fewer loads per product) once they do not
     const int wide = (ncols + 63) / 64 + (nrows + 63) / 64;
     if (wide >= sms) {

@@ -167,19 +167,17 @@ static int lu_tail(float* d, int lda, int m, float* lt, cudaStream_t st) {
 // lu stage of one diagonal block of any size (a multiple of 16): blocked with
 // 128-wide inner blocks.  Per inner block a chain of three launches: its LU
 // (one CTA), top and left beside it (one launch, k_panel.cu) and the rank-128
-// update of what follows.  inv: the inner blocks' 32 x 32 inverses, and dt
-// (bs x bs): the block's lower triangle transposed; both serve the top / left
-// updates with this block.
-int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, const TriInverses* tri) {
+// update of what follows.  dt (bs x bs) receives the block's lower triangle
+// transposed, for the top updates with this block.
+int lu_stage(lp_ctx* c, float* d, int lda, int bs, cudaStream_t st, const TriInverses* tri) {
     float* dt = static_cast<float*>(c->dt.ptr);
     for (int k0 = 0, kk = 0; k0 < bs; k0 += 128, kk++) {
         float* dd = d + (size_t)k0 * lda + k0;
         float* tt = dt + (size_t)k0 * bs + k0;
         const int ib = std::min(128, bs - k0), r = bs - k0 - ib;
         if (ib < 128) return lu_tail(dd, lda, ib, dt, st);
-        float* vv = inv + (size_t)kk * kInvFloats;
-        LP_CHECK(launch_lu128(dd, lda, vv, tt, bs, st));
-        LP_CHECK(launch_tl(dd, lda, vv, tt, bs, ib, dd + ib, lda, r, dd + (size_t)ib * lda, lda, r, tt + ib, bs,
+        LP_CHECK(launch_lu128(dd, lda, tt, bs, st));
+        LP_CHECK(launch_tl(dd, lda, tt, bs, ib, dd + ib, lda, r, dd + (size_t)ib * lda, lda, r, tt + ib, bs,
                            c->num_sms, st));
         if (tri != nullptr) {
             // block row and column kk of d are final (the trailing update below
@@ -188,8 +186,8 @@ int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, 
             LP_CUDA(cudaEventRecord(c->ev_inv[kk], st));
             LP_CUDA(cudaStreamWaitEvent(c->inv_top, c->ev_inv[kk], 0));
             LP_CUDA(cudaStreamWaitEvent(c->inv_left, c->ev_inv[kk], 0));
-            LP_CHECK(top_chunk_step(c, d, lda, inv, tri->winv, bs, kk, c->inv_top));
-            LP_CHECK(left_chunk_step(c, d, lda, inv, tri->vinv, bs, tri->vlt, kk, c->inv_left));
+            LP_CHECK(top_chunk_step(c, d, lda, tri->winv, bs, kk, c->inv_top));
+            LP_CHECK(left_chunk_step(c, d, lda, tri->vinv, bs, tri->vlt, kk, c->inv_left));
         }
         if (r > 0)
             LP_CHECK(launch_sgemm_update(dd + (size_t)ib * lda + ib, lda, tt + ib, bs, dd + ib, lda, r, r, ib, st));
@@ -208,13 +206,13 @@ int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, 
 // contribution to the rows below as one GEMM, T[below] += D[below][chunk] *
 // T[chunk].  Column j stays zero above row j, so chunk kk only touches columns
 // below (kk + 1) * 128; the skipped entries are exact zeros.
-int top_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* t, int bs, int kk, cudaStream_t st) {
+int top_chunk_step(lp_ctx* c, const float* d, int lda, float* t, int bs, int kk, cudaStream_t st) {
     const int ib = 128;
     const float* dt = static_cast<const float*>(c->dt.ptr) + (size_t)kk * ib * bs + (size_t)kk * ib;
     const float* dkk = d + (size_t)kk * ib * lda + (size_t)kk * ib;
     float* tk = t + (size_t)kk * ib * bs;
     const int cols = (kk + 1) * ib;
-    LP_CHECK(launch_tl(dkk, lda, inv + (size_t)kk * kInvFloats, dt, bs, ib, tk, bs, cols, nullptr, 4, 0, nullptr, 4,
+    LP_CHECK(launch_tl(dkk, lda, dt, bs, ib, tk, bs, cols, nullptr, 4, 0, nullptr, 4,
                        c->num_sms, st));
     const int m2 = bs - (kk + 1) * ib;
     if (m2 <= 0) return LP_OK;
@@ -226,14 +224,13 @@ int top_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* 
 // chunk's rows of lt), then L[:, after] += L[:, chunk] * D[chunk][after].
 // Row i stays zero left of column i, so chunk kk only touches rows above
 // (kk + 1) * 128.
-int left_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* l, int bs, float* lt, int kk,
-                    cudaStream_t st) {
+int left_chunk_step(lp_ctx* c, const float* d, int lda, float* l, int bs, float* lt, int kk, cudaStream_t st) {
     const int ib = 128;
     const float* dkk = d + (size_t)kk * ib * lda + (size_t)kk * ib;
     float* lk = l + (size_t)kk * ib;
     float* ltk = lt + (size_t)kk * ib * bs;
     const int rows = (kk + 1) * ib;
-    LP_CHECK(launch_tl(dkk, lda, inv + (size_t)kk * kInvFloats, nullptr, 4, ib, nullptr, 4, 0, lk, bs, rows, ltk, bs,
+    LP_CHECK(launch_tl(dkk, lda, nullptr, 4, ib, nullptr, 4, 0, lk, bs, rows, ltk, bs,
                        c->num_sms, st));
     const int m2 = bs - (kk + 1) * ib;
     if (m2 <= 0) return LP_OK;
@@ -251,9 +248,8 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
     float* d = dA + (size_t)k0 * lda + k0;
     const int kb = std::min(bs, n - k0);
     const double b = kb;
-    float* inv = block_inv(c, k0);
     int e = prof_begin(c, st);
-    LP_CHECK(lu_stage(c, d, lda, kb, inv, st));
+    LP_CHECK(lu_stage(c, d, lda, kb, st));
     LP_CHECK(prof_end(c, st, LP_STAGE_LU, e, lu_flops(b), 8.0 * b * b));
     const int rest = n - k0 - kb;
     if (rest <= 0) return LP_OK;
@@ -261,7 +257,7 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
     const double r = rest, w = below;
     if (column_ready != nullptr) LP_CUDA(cudaStreamWaitEvent(st, column_ready, 0));
     e = prof_begin(c, st);
-    LP_CHECK(launch_tl(d, lda, inv, static_cast<const float*>(c->dt.ptr), kb, kb, d + kb, lda, rest,
+    LP_CHECK(launch_tl(d, lda, static_cast<const float*>(c->dt.ptr), kb, kb, d + kb, lda, rest,
                        d + (size_t)kb * lda, lda, below, lt, std::max(4, below), c->num_sms, st));
     return prof_end(c, st, LP_STAGE_TOP, e, trsm_flops(b, r + w), 8.0 * b * r + 12.0 * b * w);
 }
@@ -279,12 +275,8 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
 //   n = 4096: 1747 / 1752 / 1962      n = 16384: 54642 / 51983 / 51272
 static int f32_block(int n) { return n <= 512 ? 512 : n < 4096 ? 128 : n < 9216 ? 256 : 512; }
 
-// Workspaces of the FP32 panel: the inverses of every 128-wide diagonal block
-// and the transposed lower triangle of the current block.
-int panel_ensure(lp_ctx* c, int n, int bs) {
-    LP_CHECK(c->dinv.ensure(sizeof(float) * kInvFloats * (size_t)((n + 127) / 128)));
-    return c->dt.ensure(sizeof(float) * (size_t)bs * bs);
-}
+// Workspace of the FP32 panel: the transposed lower triangle of the current block.
+int panel_ensure(lp_ctx* c, int bs) { return c->dt.ensure(sizeof(float) * (size_t)bs * bs); }
 
 // Blocked right-looking LU without pivoting (the block-row loop of
 // execution_pcie.hpp:177-641, on one GPU) with one step of look-ahead.
@@ -314,7 +306,7 @@ int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st)
         if (lt_bytes(bs) > free_bytes / 8) bs = std::max(128, user_bs);
     }
     LP_CHECK(c->lt.ensure(lt_bytes(bs)));
-    LP_CHECK(panel_ensure(c, n, 512));
+    LP_CHECK(panel_ensure(c, 512));
     float* ltbuf[2] = {static_cast<float*>(c->lt.ptr), static_cast<float*>(c->lt.ptr) + (size_t)bs * n};
     const double b = bs;
     if (n <= bs) return panel_f32(c, dA, n, lda, bs, 0, ltbuf[0], st);
@@ -389,7 +381,7 @@ static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r
     if (k0 > 0) {
         LP_CUDA(cudaStreamWaitEvent(st, panel_done[0], 0));
         int e = prof_begin(c, st);
-        LP_CHECK(launch_tl(dA, lda, block_inv(c, 0), nullptr, 4, bs, nullptr, 4, 0, slab, lda, rows, ln.lt[0], rows,
+        LP_CHECK(launch_tl(dA, lda, nullptr, 4, bs, nullptr, 4, 0, slab, lda, rows, ln.lt[0], rows,
                            c->num_sms, st));
         LP_CHECK(prof_end(c, st, LP_STAGE_LEFT, e, trsm_flops(b, m), 12.0 * b * m));
         for (int K = 0; K < k0; K++) {
@@ -408,7 +400,7 @@ static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r
                 LP_CUDA(cudaStreamWaitEvent(aux, ln.fork, 0));
                 LP_CUDA(cudaStreamWaitEvent(aux, panel_done[K + 1], 0));
                 e = prof_begin(c, aux);
-                LP_CHECK(launch_tl(dA + (size_t)c1 * lda + c1, lda, block_inv(c, c1), nullptr, 4, bs, nullptr, 4, 0, cs,
+                LP_CHECK(launch_tl(dA + (size_t)c1 * lda + c1, lda, nullptr, 4, bs, nullptr, 4, 0, cs,
                                    lda, rows, ln.lt[(K + 1) & 1], rows, c->num_sms, aux));
                 LP_CHECK(prof_end(c, aux, LP_STAGE_LEFT, e, trsm_flops(b, m), 12.0 * b * m));
                 LP_CUDA(cudaEventRecord(ln.join, aux));
@@ -499,7 +491,7 @@ int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, cud
     for (int s = 0; s < ns; s++) hmax = std::max(hmax, cuts[s + 1] - cuts[s]);
     const size_t ltf = (size_t)bs * hmax;
     LP_CHECK(c->lt.ensure(4 * sizeof(float) * ltf));
-    LP_CHECK(panel_ensure(c, n, 512));
+    LP_CHECK(panel_ensure(c, 512));
     if (c->copy_in == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
     if (host_out != nullptr && c->copy == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
     float* lt = static_cast<float*>(c->lt.ptr);
@@ -801,8 +793,8 @@ int lp_lu_block_dev(lp_ctx* c, float* dA, int lda, int bs) {
     LP_CUDA(cudaSetDevice(c->device));
     if (bs <= 128) return launch_lu_small(dA, lda, bs, c->stream);
     if (!aligned16(dA)) return fail(LP_E_INVALID, "lp_lu_block_dev: blocks above 128 must be 16-byte aligned");
-    LP_CHECK(panel_ensure(c, bs, bs));
-    return lu_stage(c, dA, lda, bs, block_inv(c, 0), c->stream);
+    LP_CHECK(panel_ensure(c, bs));
+    return lu_stage(c, dA, lda, bs, c->stream);
 }
 
 int lp_top_update_dev(lp_ctx* c, const float* dLU, int ldlu, float* dT, int ldt, int bs, int ncols) {

@@ -40,15 +40,13 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cuda
 // row_end (-1: n).
 int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, cudaStream_t st, int row_end = -1,
               cudaEvent_t column_ready = nullptr);
-// Workspaces of the panel stages for order n and (inner) block bs.
-int panel_ensure(lp_ctx* c, int n, int bs);
-// k_panel.cu: LU of a 128 x 128 diagonal block, its 32 x 32 inverses into inv
-// (kInvFloats floats) and its lower triangle transposed into dt; top and left
-// beside a factored block of 128 .. 512.
-constexpr size_t kInvFloats = 8 * 1024;
+// Workspace of the panel stages for (inner) block bs.
+int panel_ensure(lp_ctx* c, int bs);
+// k_panel.cu: LU of a 128 x 128 diagonal block, its lower triangle transposed
+// into dt; top and left beside a factored block of 128 .. 512.
 int panel_init_attrs();
-int launch_lu128(float* a, int lda, float* inv, float* dt, int lddt, cudaStream_t st);
-int launch_tl(const float* d, int ldd, const float* inv, const float* dt, int lddt, int bs, float* t, int ldt,
+int launch_lu128(float* a, int lda, float* dt, int lddt, cudaStream_t st);
+int launch_tl(const float* d, int ldd, const float* dt, int lddt, int bs, float* t, int ldt,
               int ncols, float* l, int ldl, int nrows, float* lt, int ldlt, int sms, cudaStream_t st);
 // E4M3: one absmax scale per 512 x 512 block (512 rows of L / columns of T by
 // a 512-wide K segment); sc holds 6 arrays of kseg(k) * nblk floats.
@@ -63,15 +61,14 @@ struct TriInverses {
     float* vinv;
     float* vlt;
 };
-// lu stage (lp_abi.cu) of a bs x bs diagonal block; inv: kInvFloats floats per
-// 128 rows.  With tri (bs > 128), chunk kk of both identity recurrences runs
+// lu stage (lp_abi.cu) of a bs x bs diagonal block.  With tri (bs > 128), chunk kk of both identity recurrences runs
 // on the context's inv_top / inv_left streams as soon as step kk of the lu
 // stage has made block row and column kk of d final; st waits for both at the
 // end.
-int lu_stage(lp_ctx* c, float* d, int lda, int bs, float* inv, cudaStream_t st, const TriInverses* tri = nullptr);
+int lu_stage(lp_ctx* c, float* d, int lda, int bs, cudaStream_t st, const TriInverses* tri = nullptr);
 // Step kk (128-wide chunk) of the identity recurrences, for bs > 128.
-int top_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* t, int bs, int kk, cudaStream_t st);
-int left_chunk_step(lp_ctx* c, const float* d, int lda, const float* inv, float* l, int bs, float* lt, int kk,
+int top_chunk_step(lp_ctx* c, const float* d, int lda, float* t, int bs, int kk, cudaStream_t st);
+int left_chunk_step(lp_ctx* c, const float* d, int lda, float* l, int bs, float* lt, int kk,
                     cudaStream_t st);
 // E4M3 scales: scale_x[seg * sstride + block] per 512-wide K segment and
 // 512-row (A) / 512-column (B) block (k_umma.cu).
@@ -173,7 +170,6 @@ struct lp_ctx {
     cudaEvent_t ev_inv_top = nullptr, ev_inv_left = nullptr;
     lp::Workspace lt;    // transposed left panels (2 x bs x n, alternating by block step)
     lp::Workspace dt;    // transposed lower triangle of the current diagonal block (bs x bs)
-    lp::Workspace dinv;  // 32 x 32 inverses of every 128-wide diagonal block (kInvFloats floats each)
     lp::Workspace q;     // tensor-core operands: 2 x (Lq, Tq), BF16 or E4M3, n x bs each
     lp::Workspace qs;    // E4M3 block scales (absmax, scale, 1/scale for L and T), 2 buffers
     lp::Workspace err;   // device error word of the tensor-core update (bounded waits)
@@ -217,7 +213,7 @@ struct lp_ctx {
     double prof_s[LP_NSTAGES] = {0}, prof_flops[LP_NSTAGES] = {0}, prof_bytes[LP_NSTAGES] = {0};
     long long prof_calls[LP_NSTAGES] = {0};
     void release_all() {
-        lp::Workspace* all[] = {&lt, &dt, &dinv, &q, &qs, &err, &tri, &tq, &gw, &gerr, &dA, &dA0, &dB, &dB64, &dX, &dR, &dCol,
+        lp::Workspace* all[] = {&lt, &dt, &q, &qs, &err, &tri, &tq, &gw, &gerr, &dA, &dA0, &dB, &dB64, &dX, &dR, &dCol,
                                 &dnorm, &gmw, &f64a, &f64b, &f64lt, &f64w, &psync, &pat, &pdesc, &pw, &pipvt, &bsys, &bnext, &tA, &tB, &bA0, &bB32, &bout, &bsys_ir, &hA, &hB, &hX};
         for (auto* w : all) w->release();
         if (bgraph != nullptr) cudaGraphExecDestroy(bgraph);
@@ -240,10 +236,3 @@ struct lp_ctx {
         f64stat = nullptr;
     }
 };
-
-namespace lp {
-// The inverses of the diagonal block that starts at row k0 (a multiple of 128).
-inline float* block_inv(lp_ctx* c, int k0) {
-    return static_cast<float*>(c->dinv.ptr) + kInvFloats * (size_t)(k0 / 128);
-}
-}  // namespace lp

@@ -135,3 +135,41 @@ def test_fp64_substitution_wait_that_runs_out_reports_timeout(ctx, dev, lp, api,
         run()
     assert e.value.status == lp.LP_E_TIMEOUT and "bounded wait" in str(e.value)
     assert np.abs(run() - 1.0).max() < 1e-9
+
+
+def whole_number_factors(n, w, e, seed):
+    """(L, U) with small whole numbers: unit diagonals, -e throughout the strict triangles of the w-wide diagonal
+    blocks, some +-1 outside them.  L U is a matrix of small whole numbers, and so is every intermediate value of the
+    recurrences, which therefore give the factors exactly; the inverses of the blocks' triangles grow like (1 + e)^w."""
+    rng = np.random.default_rng(seed)
+    inside = (np.arange(n)[:, None] // w) == (np.arange(n)[None, :] // w)
+    some = np.where(rng.random((n, n)) < 0.02, rng.choice([-1.0, 1.0], (n, n)), 0.0)
+    F = np.where(inside, -float(e), some)
+    return np.tril(F, -1) + np.eye(n), np.triu(F, 1) + np.eye(n)
+
+
+def encoded(L, U):
+    """The reference's storage (transposed, multipliers negated, -1/u_kk on the diagonal)."""
+    return np.triu(-L.T, 1) + np.tril(U.T, -1) - np.diag(1.0 / np.diag(U))
+
+
+@pytest.mark.parametrize("api,n,bs", [("gefa", 128, 16), ("gefa", 512, 128), ("gefa", 1280, 256), ("gefa", 720, 16),
+                                      ("lu_block", 256, 256), ("lu_block", 512, 512), ("calculate", 1280, 64)])
+def test_factors_of_whole_numbers_are_exact(ctx, dev, lp, api, n, bs):
+    """Top and left lose nothing that the recurrences keep, whatever the condition of the diagonal blocks' triangles."""
+    L, U = whole_number_factors(n, 32, 1, n)
+    S = np.ascontiguousarray((L @ U).T).astype(np.float32)
+    assert np.array_equal(S.astype(np.float64), (L @ U).T)
+    if api == "calculate":
+        pa, pb = lp.Pinned((n, n)), lp.Pinned((n,))
+        pa.array[...], pb.array[...] = S, S.sum(0)
+        ctx.calculate(pa.array, pb.array, bs)
+        got = pa.array
+    else:
+        d = dev.put(S)
+        if api == "gefa":
+            ctx.gefa(d.data_ptr(), n, n, bs)
+        else:
+            ctx.lu_block(d.data_ptr(), n, bs)
+        got = dev.get(d)
+    assert np.array_equal(got, encoded(L, U).astype(np.float32))
