@@ -6,8 +6,8 @@
 // lu, top and left are the float kernels instantiated for double
 // (k_lu.cu, k_trsm.cu: reference operation order, bit-identical on one
 // block); inner is k_dgemm_update.  The substitution below is blocked by 64
-// unknowns, one launch for both sweeps: every CTA forms a block's values with
-// the inverse of its diagonal block, then updates its share of the other
+// unknowns, one launch for both sweeps: every CTA runs a block's recurrence
+// itself, then updates its share of the other
 // unknowns with the block's rows (a GEMV over contiguous rows, each factor
 // element read once per sweep).
 #include <string>
@@ -24,79 +24,46 @@ constexpr int NW = GT / 32;  // warps; in the updates each takes SB / NW rows of
 constexpr int RPW = SB / NW;
 constexpr unsigned kSpinLimit64 = 1u << 22;
 
-// The inverses of both triangles of every SB x SB diagonal block D (encoded
-// factors, read as double; a ragged last block padded with the identity):
-// op[2j] = (I - strict-upper(D))^-1, op[2j + 1] = (diag(D_kk)^-1 -
-// strict-lower(D))^-1, so that the block's 64 dependent steps become one
-// product.  One CTA per block: the four 32 x 32 triangles by one warp each
-// (lane = column), then the 32 x 32 blocks joining them.
-template <typename FT>
-__global__ void __launch_bounds__(128) k_inv64(const FT* __restrict__ a, int lda, int n, double* __restrict__ op) {
-    extern __shared__ __align__(16) double ism[];
-    double(*D)[SB + 1] = reinterpret_cast<double(*)[SB + 1]>(ism);
-    double(*T)[33] = reinterpret_cast<double(*)[33]>(ism + SB * (SB + 1));  // two 32 x 32 products
-    const int j = blockIdx.x, k0 = j * SB, kb = min(SB, n - k0);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int idx = tid; idx < SB * SB; idx += 128) {
-        const int r = idx / SB, c = idx % SB;
-        D[r][c] = r < kb && c < kb ? (double)a[(size_t)(k0 + r) * lda + k0 + c] : (r == c ? 1.0 : 0.0);
-    }
-    __syncthreads();
-    double* Y = op + (size_t)(2 * j) * SB * SB;
-    double* X = Y + SB * SB;
-    const int o = 32 * (warp & 1);  // warps 0, 1: Y's diagonal blocks, 2, 3: X's
-    double x[32];
+// The dependent steps of one block for Q right-hand sides, one warp; lane holds
+// the unknowns lane and lane + 32 (v[q][0], v[q][1]); D: the kb x kb diagonal
+// block (FP32 factors, for the GMRES refinement, widened exactly as they are
+// read).  Forward: v_i += v_k D_ki (i > k).  Backward: s = v_k D_kk, v_i += s D_ki
+// (i < k); v_k = s.
+template <int Q, typename FT>
+__device__ __forceinline__ void block_forward(double (&v)[Q][2], const FT* D, int kb, int lane) {
 #pragma unroll
-    for (int r = 0; r < 32; r++) x[r] = r == lane ? 1.0 : 0.0;
-    if (warp < 2) {
+    for (int h = 0; h < 2; h++)
+#pragma unroll 8
+        for (int kk = 0; kk < min(32, kb - 32 * h); kk++) {
+            const FT* row = D + (32 * h + kk) * SB + lane;
+            const double d0 = (double)row[0], d1 = (double)row[32];
 #pragma unroll
-        for (int k = 31; k > 0; k--)
-#pragma unroll
-            for (int r = 0; r < k; r++) x[r] = fma(D[o + r][o + k], x[k], x[r]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 32; k++) {
-            x[k] *= D[o + k][o + k];
-#pragma unroll
-            for (int r = k + 1; r < 32; r++) x[r] = fma(D[o + r][o + k], x[k], x[r]);
+            for (int q = 0; q < Q; q++) {
+                const double y = __shfl_sync(0xffffffffu, v[q][h], kk);
+                if (lane > kk) v[q][h] = fma(y, h == 0 ? d0 : d1, v[q][h]);
+                if (h == 0) v[q][1] = fma(y, d1, v[q][1]);
+            }
         }
-    }
-    double* out = warp < 2 ? Y : X;
-#pragma unroll
-    for (int r = 0; r < 32; r++) out[(o + r) * SB + o + lane] = x[r];
-    // the blocks beside them: Y01 = Y00 U01 Y11 and X10 = X11 L10 X00, Y10 = X01 = 0; both read back (this CTA's
-    // writes) after the barrier, 64 threads each, 16 outputs per thread
-    __syncthreads();
-    const bool up = tid < 64;
-    const int t = tid & 63, c = t & 31, r0 = 16 * (t >> 5);
-    const int lo = up ? 0 : 32, hi = up ? 32 : 0;  // block (lo, hi) of D and of the inverse
-    const double* in = up ? Y : X;
-    double s[16];
-#pragma unroll
-    for (int q = 0; q < 16; q++) s[q] = 0.0;
-    for (int k = 0; k < 32; k++) {
-        const double v = in[(hi + k) * SB + hi + c];
-#pragma unroll
-        for (int q = 0; q < 16; q++) s[q] = fma(D[lo + r0 + q][hi + k], v, s[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) T[(up ? 0 : 32) + r0 + q][c] = s[q];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 16; q++) s[q] = 0.0;
-    for (int k = 0; k < 32; k++) {
-        const double v = T[(up ? 0 : 32) + k][c];
-#pragma unroll
-        for (int q = 0; q < 16; q++) s[q] = fma(in[(lo + r0 + q) * SB + lo + k], v, s[q]);
-    }
-    double* w = up ? Y : X;
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-        w[(lo + r0 + q) * SB + hi + c] = s[q];
-        w[(hi + r0 + q) * SB + lo + c] = 0.0;
-    }
 }
-constexpr size_t kInv64Smem = sizeof(double) * (SB * (SB + 1) + 64 * 33);
+template <int Q, typename FT>
+__device__ __forceinline__ void block_backward(double (&v)[Q][2], const FT* D, int kb, int lane) {
+#pragma unroll
+    for (int h = 1; h >= 0; h--)
+#pragma unroll 8
+        for (int kk = min(32, kb - 32 * h) - 1; kk >= 0; kk--) {
+            const FT* row = D + (32 * h + kk) * SB;
+            const double d = (double)row[32 * h + kk], d0 = (double)row[lane], d1 = (double)row[lane + 32];
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const double s = __shfl_sync(0xffffffffu, v[q][h], kk) * d;
+                if (lane < kk)
+                    v[q][h] = fma(s, h == 0 ? d0 : d1, v[q][h]);
+                else if (lane == kk)
+                    v[q][h] = s;
+                if (h == 1) v[q][0] = fma(s, d0, v[q][0]);
+            }
+        }
+}
 
 // Bounded grid barrier of a cooperative launch; the counter only grows.
 // absent (tests): this CTA does not arrive.
@@ -126,24 +93,25 @@ __device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, unsi
 
 // Forward and back substitution of one group of right-hand sides (rows of b,
 // overwritten by the solutions), one cooperative launch.  Per block of SB
-// unknowns every CTA forms the block's values itself (one product with the
-// block's inverse, copied in before the barrier), then updates its share of
-// the unknowns after (forward) or before (backward) it with rows loaded before
-// the barrier; one barrier per block.  w1, w2: n x nrhs accumulating values of
-// the two sweeps (the forward sweep's results are the second's input).  A
-// chain of 2 n / 64 short steps, where one launch per block and direction took
-// 15 us each (n = 6144: 192 launches, 2.9 ms).  A barrier that gives up leaves
+// unknowns every CTA runs the block's own recurrence (one warp per right-hand
+// side, two above eight; the diagonal block was copied in before the barrier),
+// then updates its share of the unknowns after (forward) or before (backward)
+// it with rows loaded before the barrier; one barrier per block.  w1, w2: n x
+// nrhs accumulating values of the two sweeps (the forward sweep's results are
+// the second's input).  A chain of 2 n / 64 short steps, where one launch per block and direction took
+// 15 us each (n = 6144: 192 launches, 2.9 ms; now 1.1).  Products with the blocks'
+// inverses in place of the recurrences took 0.27 ms less, but lost what the
+// condition of a block's triangles allows.  A barrier that gives up leaves
 // NaN in the solutions and sets *gave_up, a word in page-locked host memory.
 // stall (tests): CTA 0 never arrives at the first barrier.
 template <typename FT>
 __global__ void __launch_bounds__(GT, 1)
-    k_gesl64(const FT* __restrict__ a, int lda, int n, const double* __restrict__ op, double* w1, double* w2, double* b,
-             int ldb, int nrhs, unsigned* sync, int* gave_up, int stall) {
+    k_gesl64(const FT* __restrict__ a, int lda, int n, double* w1, double* w2, double* b, int ldb, int nrhs,
+             unsigned* sync, int* gave_up, int stall) {
     extern __shared__ __align__(16) double sm[];
-    double* Ob = sm;                          // 2 x SB x SB: the block's inverse, alternating
-    double* in = Ob + 2 * SB * SB;            // RMAX x SB: the block's accumulated values
-    double* ys = in + RMAX * SB;              // RMAX x SB: its solved values
+    double* ys = sm;                          // RMAX x SB: the block's solved values
     double* part = ys + RMAX * SB;            // NW x 32 x RMAX partial sums
+    FT* Db = reinterpret_cast<FT*>(part + NW * 32 * RMAX);  // 2 x SB x SB: the diagonal block, alternating
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, g = blockIdx.x;
     int* err = reinterpret_cast<int*>(sync + 1);
     const int nblk = (n + SB - 1) / SB, steps = 2 * nblk;
@@ -156,9 +124,11 @@ __global__ void __launch_bounds__(GT, 1)
         i1 = min(hi, i0 + ch);
     };
     auto stage = [&](int s) {
-        const double* src = op + (size_t)(2 * block_of(s) + (s < nblk ? 0 : 1)) * SB * SB;
-        double* dst = Ob + (s & 1) * SB * SB;
-        for (int idx = tid * 2; idx < SB * SB; idx += GT * 2) cp_async_vec16(dst + idx, src + idx);
+        const int k0 = block_of(s) * SB, kb = min(SB, n - k0);
+        for (int idx = tid; idx < SB * SB; idx += GT) {
+            const int r = idx / SB, c = idx % SB;
+            if (r < kb && c < kb) cp_async_elem(Db + (s & 1) * SB * SB + idx, a + (size_t)(k0 + r) * lda + k0 + c);
+        }
     };
     double v[RPW];
     auto load_rows = [&](int s, int i, bool ok) {
@@ -174,39 +144,43 @@ __global__ void __launch_bounds__(GT, 1)
         const bool fwd = s < nblk;
         const int k0 = block_of(s) * SB, kb = min(SB, n - k0);
         double* w = fwd ? w1 : w2;
-        for (int idx = tid; idx < nrhs * SB; idx += GT) {
-            const int r = idx / SB, i = idx % SB;
-            in[idx] = i < kb ? __ldcg(w + (size_t)r * n + k0 + i) : 0.0;
-        }
+        double y[2][2];  // this warp's right-hand sides: warp and warp + NW
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = warp + NW * q, i = lane + 32 * h;
+                y[q][h] = r < nrhs && i < kb ? __ldcg(w + (size_t)r * n + k0 + i) : 0.0;
+            }
         cp_async_wait_all();
         __syncthreads();
         if (s + 1 < steps) stage(s + 1);
-        {  // y_i = sum_k op[k][i] in_k: column i by a quarter of the threads per quarter of k
-            const double* o = Ob + (s & 1) * SB * SB;
-            const int i = tid & (SB - 1), kq = (tid >> 6) * (SB / 4);
-            for (int r = 0; r < nrhs; r++) {
-                double y0 = 0.0, y1 = 0.0;
+        if (warp < nrhs) {
+            const FT* D = Db + (s & 1) * SB * SB;
+            if (nrhs <= NW) {
+                double(&y1)[1][2] = reinterpret_cast<double(&)[1][2]>(y);
+                if (fwd) block_forward<1>(y1, D, kb, lane);
+                else block_backward<1>(y1, D, kb, lane);
+            } else if (fwd) {
+                block_forward<2>(y, D, kb, lane);
+            } else {
+                block_backward<2>(y, D, kb, lane);
+            }
+        }
 #pragma unroll
-                for (int k = 0; k < SB / 4; k += 2) {
-                    y0 = fma(o[(kq + k) * SB + i], in[r * SB + kq + k], y0);
-                    y1 = fma(o[(kq + k + 1) * SB + i], in[r * SB + kq + k + 1], y1);
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = warp + NW * q, i = lane + 32 * h;
+                if (r >= nrhs) continue;
+                ys[r * SB + i] = i < kb ? y[q][h] : 0.0;
+                if (g == 0 && i < kb) {
+                    if (fwd)
+                        w2[(size_t)r * n + k0 + i] = y[q][h];  // (w1's block is still being read by other CTAs)
+                    else
+                        b[(size_t)r * ldb + k0 + i] = -y[q][h];
                 }
-                part[(r * 4 + (tid >> 6)) * SB + i] = y0 + y1;
             }
-        }
-        __syncthreads();
-        for (int idx = tid; idx < nrhs * SB; idx += GT) {
-            const int r = idx / SB, i = idx % SB;
-            const double* q = part + r * 4 * SB + i;
-            const double y = (q[0] + q[SB]) + (q[2 * SB] + q[3 * SB]);
-            ys[idx] = y;
-            if (g == 0 && i < kb) {
-                if (fwd)
-                    w2[(size_t)r * n + k0 + i] = y;  // (w1's block is still being read by other CTAs)
-                else
-                    b[(size_t)r * ldb + k0 + i] = -y;
-            }
-        }
         __syncthreads();
         // unknowns after (forward) or before (backward) the block: += y^T S[block][i]
         for (int ib = i0; ib < i1; ib += 32) {
@@ -247,8 +221,8 @@ __global__ void __launch_bounds__(GT, 1)
         }
     }
 }
-constexpr size_t kGesl64Smem = sizeof(double) * (2 * SB * SB + 2 * RMAX * SB + (size_t)NW * 32 * RMAX);
-static_assert(4 * SB <= NW * 32, "the block's partial sums share the updates' space");
+constexpr size_t kGesl64Smem = sizeof(double) * (2 * SB * SB + RMAX * SB + (size_t)NW * 32 * RMAX);
+static_assert(RMAX <= 2 * NW, "a warp takes two right-hand sides");
 
 double event_s64(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0.0f;
@@ -390,17 +364,12 @@ int gefa_f64(lp_ctx* c, double* a, int n, int lda, int bs, cudaStream_t st) {
 template <typename FT>
 static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrhs, int ldb, int* gave_up,
                       cudaStream_t st) {
-    const int g0 = nrhs < RMAX ? nrhs : RMAX, nblk = (n + SB - 1) / SB;
-    const size_t ops = 2 * (size_t)nblk * SB * SB;
-    LP_CHECK(c->f64w.ensure(sizeof(double) * (2 * (size_t)n * g0 + ops + 2)));
-    double* op = static_cast<double*>(c->f64w.ptr);
-    unsigned* sync = reinterpret_cast<unsigned*>(op + ops);  // barrier counter, error word
-    double* w1 = op + ops + 2;
+    const int g0 = nrhs < RMAX ? nrhs : RMAX;
+    LP_CHECK(c->f64w.ensure(sizeof(double) * (2 * (size_t)n * g0 + 2)));
+    unsigned* sync = static_cast<unsigned*>(c->f64w.ptr);  // barrier counter, error word
+    double* w1 = static_cast<double*>(c->f64w.ptr) + 2;
     double* w2 = w1 + (size_t)n * g0;
     const int e = prof_begin(c, st);
-    k_inv64<FT><<<nblk, 128, kInv64Smem, st>>>(a, lda, n, op);
-    LP_CUDA(cudaGetLastError());
-    count_launch();
     int stall = c->stall_site == LP_STALL_GESL64;  // (failure-path tests: the first group)
     if (stall) c->stall_site = LP_STALL_NONE;
     // enough CTAs that a step's products are one pass of 32 unknowns each, at most one per SM
@@ -411,7 +380,7 @@ static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrh
         LP_CUDA(cudaMemcpy2DAsync(w1, sizeof(double) * n, bb, sizeof(double) * ldb, sizeof(double) * n, g,
                                   cudaMemcpyDeviceToDevice, st));
         LP_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st));
-        void* args[] = {&a, &lda, &n, &op, &w1, &w2, &bb, &ldb, &g, &sync, &gave_up, &stall};
+        void* args[] = {&a, &lda, &n, &w1, &w2, &bb, &ldb, &g, &sync, &gave_up, &stall};
         LP_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_gesl64<FT>), dim3(grid), dim3(GT), args,
                                             kGesl64Smem, st));
         count_launch();
@@ -422,8 +391,6 @@ static int gesl64_any(lp_ctx* c, const FT* a, int n, int lda, double* b, int nrh
 }
 
 int gesl64_init_attrs() {
-    LP_CUDA(cudaFuncSetAttribute(k_inv64<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInv64Smem));
-    LP_CUDA(cudaFuncSetAttribute(k_inv64<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInv64Smem));
     LP_CUDA(cudaFuncSetAttribute(k_gesl64<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGesl64Smem));
     LP_CUDA(cudaFuncSetAttribute(k_gesl64<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGesl64Smem));
     return LP_OK;

@@ -173,3 +173,16 @@ def test_factors_of_whole_numbers_are_exact(ctx, dev, lp, api, n, bs):
             ctx.lu_block(d.data_ptr(), n, bs)
         got = dev.get(d)
     assert np.array_equal(got, encoded(L, U).astype(np.float32))
+
+
+@pytest.mark.parametrize("n,nrhs,pad", [(64, 1, 0), (100, 9, 1), (200, 2, 0), (1000, 17, 0)])
+def test_fp64_solution_of_whole_numbers_is_exact(ctx, dev, n, nrhs, pad):
+    """The FP64 substitution loses nothing that the recurrences keep: factors of whole numbers whose diagonal blocks'
+    triangles have inverses up to 3^63, beyond what a double holds exactly."""
+    L, U = whole_number_factors(n, 64, 2, n)
+    want = np.random.default_rng(1).integers(-4, 5, (nrhs, n)).astype(np.float64)
+    store = np.full((n, n + pad), 7.0)
+    store[:, :n] = encoded(L, U)
+    d, b = dev.put(store), dev.put(want @ U.T @ L.T)
+    ctx.gesl_f64(d.data_ptr(), n, n + pad, b.data_ptr(), nrhs)
+    assert np.array_equal(dev.get(b), want)
