@@ -431,9 +431,9 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
 //   emulated FP32 n = 3072 2.35 / 1.68 / 1.51   n = 8192 8.67 / 5.91 / 5.70   n = 32768 276 / 144 / 136
 constexpr int kMixedBlock = 1024;
 
-// Workspaces for blocks of up to bs.  With *grow, only what they need beyond
-// their present sizes is added up.
-static int mixed_ensure(lp_ctx* c, int precision, int n, int bs, int nseg, size_t* grow) {
+// Workspaces for blocks of up to bs; where one of them cannot be allocated, all
+// of them are given back.
+static int mixed_ensure(lp_ctx* c, int precision, int n, int bs, int nseg) {
     const size_t esz = precision == LP_FP8_IR ? 1 : 2, kq = precision == LP_F32_BF16X6 ? 6 * (size_t)bs : bs;
     const size_t nblk = (n + 511) / 512, b = bs;
     const struct { Workspace* w; size_t bytes; } need[] = {
@@ -444,10 +444,10 @@ static int mixed_ensure(lp_ctx* c, int precision, int n, int bs, int nseg, size_
         {&c->tri, 3 * sizeof(float) * b * b},
         {&c->tq, 2 * sizeof(__nv_bfloat16) * (size_t)nseg * b * (b + n)}};
     for (const auto& x : need) {
-        if (grow == nullptr)
-            LP_CHECK(x.w->ensure(x.bytes));
-        else if (x.bytes > x.w->cap)
-            *grow += x.bytes;
+        const int status = x.w->ensure(x.bytes);
+        if (status == LP_OK) continue;
+        for (const auto& y : need) y.w->release();
+        return status;
     }
     return LP_OK;
 }
@@ -464,13 +464,15 @@ int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int user_bs,
     // 2048: 582 -> 638 TFLOP/s, one refinement either way; n = 32768, block 1024: no
     // gain, the plainer factors needing a second refinement.
     const int nseg = x6 ? 6 : user_bs >= 2048 ? 1 : 3;
-    // the wide block's workspaces where device memory has ample room for them, else the caller's
+    // the wide block; only where its workspaces cannot be allocated, the caller's
     int bs = x6 || (!fp8 && n >= 4096) ? std::max(kMixedBlock, user_bs) : user_bs;
-    size_t grow = 0, free_bytes = 0, total_bytes = 0;
-    LP_CHECK(mixed_ensure(c, precision, n, bs, nseg, &grow));
-    if (grow > 0 && bs > user_bs) LP_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-    if (bs > user_bs && grow > free_bytes / 8) bs = user_bs;
-    LP_CHECK(mixed_ensure(c, precision, n, bs, nseg, nullptr));
+    int status = mixed_ensure(c, precision, n, bs, nseg);
+    if (status == LP_E_NOMEM && bs > user_bs) {
+        cudaGetLastError();
+        bs = user_bs;
+        status = mixed_ensure(c, precision, n, bs, nseg);
+    }
+    if (status != LP_OK) return status;
     const size_t esz = fp8 ? 1 : 2;
     const int kq = x6 ? 6 * bs : bs;    // K of the tensor-core update
     const size_t pan = (size_t)kq * n;  // one tensor-core operand

@@ -278,6 +278,43 @@ static int f32_block(int n) { return n <= 512 ? 512 : n < 4096 ? 128 : n < 9216 
 // Workspace of the FP32 panel: the transposed lower triangle of the current block.
 int panel_ensure(lp_ctx* c, int bs) { return c->dt.ensure(sizeof(float) * (size_t)bs * bs); }
 
+// Row-slab boundaries of the streamed factorization: heights 1024, 2048, then
+// 4096 rows (multiples of bs, at least bs), so the first slab's copy is short.
+static std::vector<int> slab_cuts(int n, int bs) {
+    std::vector<int> cuts{0};
+    const int cap = std::max(bs, 4096 / bs * bs);
+    int h = std::max(bs, 1024 / bs * bs);
+    while (cuts.back() < n) {
+        cuts.push_back(std::min(n, cuts.back() + h));
+        h = std::min(cap, 2 * h);
+    }
+    return cuts;
+}
+
+// The FP32 schedule's inner block, with its workspaces: f32_block(n), so that a
+// call's results never depend on what else is in device memory; only where the
+// operands of that block cannot be allocated, the caller's own block.
+int f32_prepare(lp_ctx* c, int n, int user_bs, bool streamed, int* bs) {
+    // L transposed: two panels of n rows (never less than for one block of 512, so that a context warmed at one
+    // order has room for every smaller one), or two of a slab's rows for each lane of the streamed form
+    auto lt_bytes = [&](int b) {
+        if (!streamed) return 2 * sizeof(float) * std::max((size_t)b * n, (size_t)512 * 512);
+        const std::vector<int> cuts = slab_cuts(n, b);
+        int h = 0;
+        for (size_t s = 1; s < cuts.size(); s++) h = std::max(h, cuts[s] - cuts[s - 1]);
+        return 4 * sizeof(float) * (size_t)b * h;
+    };
+    *bs = f32_block(n);
+    LP_CHECK(panel_ensure(c, 512));
+    int status = c->lt.ensure(lt_bytes(*bs));
+    if (status == LP_E_NOMEM && *bs > std::max(128, user_bs)) {
+        cudaGetLastError();
+        *bs = std::max(128, user_bs);
+        status = c->lt.ensure(lt_bytes(*bs));
+    }
+    return status;
+}
+
 // Blocked right-looking LU without pivoting (the block-row loop of
 // execution_pcie.hpp:177-641, on one GPU) with one step of look-ahead.
 // Step K's trailing update C += L_K * T_K is split: first the next block row
@@ -296,17 +333,8 @@ int panel_ensure(lp_ctx* c, int bs) { return c->dt.ensure(sizeof(float) * (size_
 // The stages give the reference recurrences' values up to rounding; the exact
 // recurrences are lp_lu_block_dev, lp_top_update_dev, lp_left_update_dev.
 int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
-    // the order's block where device memory has ample room for its operands, else the caller's
-    int bs = f32_block(n);
-    // (never less than for one block of 512, so that a context warmed at one order has room for every smaller one)
-    auto lt_bytes = [&](int b) { return 2 * sizeof(float) * std::max((size_t)b * n, (size_t)512 * 512); };
-    if (bs > std::max(128, user_bs) && lt_bytes(bs) > c->lt.cap) {
-        size_t free_bytes = 0, total_bytes = 0;
-        LP_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-        if (lt_bytes(bs) > free_bytes / 8) bs = std::max(128, user_bs);
-    }
-    LP_CHECK(c->lt.ensure(lt_bytes(bs)));
-    LP_CHECK(panel_ensure(c, 512));
+    int bs = 0;
+    LP_CHECK(f32_prepare(c, n, user_bs, false, &bs));
     float* ltbuf[2] = {static_cast<float*>(c->lt.ptr), static_cast<float*>(c->lt.ptr) + (size_t)bs * n};
     const double b = bs;
     if (n <= bs) return panel_f32(c, dA, n, lda, bs, 0, ltbuf[0], st);
@@ -370,7 +398,7 @@ struct Lane {
 // < r1, recording panel_done[K] (by band(K, stream)) when block row K is
 // final.  Every element receives the operations of gefa_f32 in the same order
 // (the stages are row- or column-independent, the update adds a k-ordered
-// product per element), so the factors equal gefa_f32's.
+// product per element), so the factors equal gefa_f32's with the same block.
 template <class Band>
 static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r1, const Lane& ln,
                      const cudaEvent_t* panel_done, Band band) {
@@ -451,23 +479,9 @@ static int gefa_rows(lp_ctx* c, float* dA, int n, int lda, int bs, int r0, int r
     return LP_OK;
 }
 
-// Row-slab boundaries of the streamed factorization: heights 1024, 2048, then
-// 4096 rows (multiples of bs, at least bs), so the first slab's copy is short.
-static std::vector<int> slab_cuts(int n, int bs) {
-    std::vector<int> cuts{0};
-    const int cap = std::max(bs, 4096 / bs * bs);
-    int h = std::max(bs, 1024 / bs * bs);
-    while (cuts.back() < n) {
-        cuts.push_back(std::min(n, cuts.back() + h));
-        h = std::min(cap, 2 * h);
-    }
-    return cuts;
-}
-
 // Events of the streamed form: one per block row, one per slab (no more than
 // block rows), the start and the second lane's end.
-size_t streamed_events(int n) {
-    const int bs = f32_block(n);
+size_t streamed_events(int n, int bs) {
     return 2 * (size_t)((n + bs - 1) / bs) + 2;
 }
 
@@ -480,18 +494,15 @@ size_t streamed_events(int n) {
 // lanes at once (a slab's own steps start after the other lane's last panel),
 // so the panel's scratch is shared.  With host_out, every block row goes back
 // to host_out (leading dimension lda) on the copy stream as soon as it is
-// final.  ev: streamed_events(n) events.
-int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, cudaStream_t st, float* host_out,
+// final.  bs: from f32_prepare.  ev: streamed_events(n, bs) events.
+int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int bs, cudaStream_t st, float* host_out,
                       const std::vector<cudaEvent_t>& ev) {
-    const int bs = f32_block(n);
     const std::vector<int> cuts = slab_cuts(n, bs);
     const int ns = (int)cuts.size() - 1, nb = (n + bs - 1) / bs;
     if ((int)ev.size() < nb + ns + 2) return fail(LP_E_INVALID, "streamed factorization: too few events");
     int hmax = 0;
     for (int s = 0; s < ns; s++) hmax = std::max(hmax, cuts[s + 1] - cuts[s]);
     const size_t ltf = (size_t)bs * hmax;
-    LP_CHECK(c->lt.ensure(4 * sizeof(float) * ltf));
-    LP_CHECK(panel_ensure(c, 512));
     if (c->copy_in == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
     if (host_out != nullptr && c->copy == nullptr) LP_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
     float* lt = static_cast<float*>(c->lt.ptr);
@@ -942,9 +953,11 @@ int lp_calculate(lp_ctx* c, int n, int lda, int bs, int repetitions, float* A, f
                 if (e != nullptr) cudaEventDestroy(e);
         }
     } evs;
+    int block = 0;
     if (pinned) {
+        LP_CHECK(f32_prepare(c, n, bs, true, &block));
         evs.c = c;
-        evs.v.resize(streamed_events(n), nullptr);
+        evs.v.resize(streamed_events(n, block), nullptr);
         for (auto& e : evs.v) LP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     int status = LP_OK;
@@ -953,7 +966,7 @@ int lp_calculate(lp_ctx* c, int n, int lda, int bs, int repetitions, float* A, f
         LP_CUDA(cudaMemcpyAsync(dB, b, sizeof(float) * n, cudaMemcpyHostToDevice, st));
         if (pinned) {
             LP_CUDA(cudaEventRecord(c->ev[0], st));
-            status = gefa_f32_streamed(c, A, dA, n, lda, st, last ? A : nullptr, evs.v);
+            status = gefa_f32_streamed(c, A, dA, n, lda, block, st, last ? A : nullptr, evs.v);
         } else {
             LP_CUDA(cudaMemcpyAsync(dA, A, abytes, cudaMemcpyHostToDevice, st));
             LP_CUDA(cudaEventRecord(c->ev[0], st));

@@ -30,10 +30,10 @@ int validate_matrix(const void* a, int n, int lda, int bs, const char* who, int 
 int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int bs, cudaStream_t st);
 // gefa_f32 on a matrix still in page-locked host memory hA, copied in row slabs
 // while the factorization runs; block rows return to host_out (if not null)
-// as they become final.  ev: streamed_events(n) events.
-int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, cudaStream_t st, float* host_out,
+// as they become final.  bs: from f32_prepare; ev: streamed_events(n, bs) events.
+int gefa_f32_streamed(lp_ctx* c, const float* hA, float* dA, int n, int lda, int bs, cudaStream_t st, float* host_out,
                       const std::vector<cudaEvent_t>& ev);
-size_t streamed_events(int n);
+size_t streamed_events(int n, int bs);
 int gefa_mixed(lp_ctx* c, int precision, float* dA, int n, int lda, int bs, cudaStream_t st);
 // Panel work of the block step at row k0 (lu, top, left; Lt into lt), on
 // stream st; the left stage covers the rows below the diagonal block up to

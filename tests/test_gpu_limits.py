@@ -186,3 +186,47 @@ def test_fp64_solution_of_whole_numbers_is_exact(ctx, dev, n, nrhs, pad):
     d, b = dev.put(store), dev.put(want @ U.T @ L.T)
     ctx.gesl_f64(d.data_ptr(), n, n + pad, b.data_ptr(), nrhs)
     assert np.array_equal(dev.get(b), want)
+
+
+@pytest.mark.parametrize("kind,n,need_mb", [("f32", 9216, 38), ("calculate", 9216, 34), ("bf16", 4096, 114)])
+def test_factors_do_not_depend_on_free_memory(lp, dev, torch_cuda, kind, n, need_mb):
+    """The inner block follows from the order and the precision: with little memory left beside what it takes (its
+    operands: need_mb), a context that has allocated nothing yet gives the bits of one with room.  With less than that,
+    the call still succeeds, in the caller's block: the factors agree to the operands' rounding."""
+    torch = torch_cuda
+    bs, mb = 128, 1 << 20
+    g = torch.Generator(device="cuda").manual_seed(n)
+    S = torch.rand(n, n, generator=g, device="cuda").sub_(0.5)
+    S.diagonal().copy_(S.abs().sum(1) + 1.0)
+    torch.cuda.synchronize()
+    host = lp.Pinned((n, n)) if kind == "calculate" else None
+
+    def factors(c, M):
+        if host is not None:
+            host.array[...] = M.cpu().numpy()
+            b = lp.Pinned((n,))
+            b.array[...] = 1.0
+            c.calculate(host.array, b.array, bs)
+            return host.array.copy()
+        c.gefa_prec(kind, M.data_ptr(), n, n, bs)
+        c.sync()
+        return M
+
+    with lp.Context(0) as c:
+        want = factors(c, S.clone())
+    matrix_mb = n * n * 4 // mb + 4 if host is not None else 0  # lp_calculate's own copy
+    for work, left_mb in zip((S.clone(), S.clone()), (2 * need_mb, need_mb // 2)):
+        with lp.Context(0) as c:
+            torch.cuda.empty_cache()
+            hog = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb + matrix_mb) * mb, dtype=torch.uint8, device="cuda")
+            try:
+                got = factors(c, work)
+            finally:
+                del hog
+                torch.cuda.empty_cache()
+        same = np.array_equal(got, want) if host is not None else torch.equal(got, want)
+        if left_mb >= need_mb:
+            assert same
+        else:
+            a, b = (torch.as_tensor(x).cuda().double() for x in (got, want))
+            assert float((a - b).abs().max() / b.abs().max()) < (2e-3 if kind == "bf16" else 256 * FLT_EPS)
