@@ -118,22 +118,46 @@ int prof_end(lp_ctx* c, cudaStream_t st, int kind, int e0, double flops, double 
     return LP_OK;
 }
 
+int prof_end_tl(lp_ctx* c, cudaStream_t st, int e0, double top_flops, double top_bytes, double left_flops,
+                double left_bytes) {
+    if (e0 < 0 || left_flops <= 0.0) return prof_end(c, st, LP_STAGE_TOP, e0, top_flops, top_bytes);
+    LP_CHECK(prof_end(c, st, LP_STAGE_TOP, e0, top_flops, top_bytes));
+    StageMark left = c->marks.back();
+    c->marks.back().f1 = left.f0 = top_flops / (top_flops + left_flops);
+    left.kind = LP_STAGE_LEFT;
+    left.flops = left_flops;
+    left.bytes = left_bytes;
+    c->marks.push_back(left);
+    return LP_OK;
+}
+
 // Folds the recorded marks into the per-stage sums (waits for the stream).
+// Launches of one stage that run beside each other (parts of a trailing update)
+// count once: the sum is over the union of their intervals.
 static int prof_collect(lp_ctx* c) {
     if (c->marks.empty()) return LP_OK;
     LP_CUDA(cudaStreamSynchronize(c->stream));
     LP_CUDA(cudaStreamSynchronize(c->aux));
     LP_CUDA(cudaStreamSynchronize(c->aux2));
+    std::vector<std::pair<double, double>> spans[LP_NSTAGES];
     for (const auto& m : c->marks) {
-        float ms = 0.0f, a = 0.0f, b = 0.0f;
+        float ms = 0.0f, a = 0.0f;
         LP_CUDA(cudaEventElapsedTime(&ms, c->prof_ev[m.e0], c->prof_ev[m.e1]));
         LP_CUDA(cudaEventElapsedTime(&a, c->prof_base, c->prof_ev[m.e0]));
-        LP_CUDA(cudaEventElapsedTime(&b, c->prof_base, c->prof_ev[m.e1]));
-        c->timeline.push_back(lp_stage_event{m.kind, m.stream, a * 1e-3, b * 1e-3});
-        c->prof_s[m.kind] += ms * 1e-3;
+        const double t0 = (a + m.f0 * ms) * 1e-3, t1 = (a + m.f1 * ms) * 1e-3;
+        c->timeline.push_back(lp_stage_event{m.kind, m.stream, t0, t1});
+        spans[m.kind].emplace_back(t0, t1);
         c->prof_flops[m.kind] += m.flops;
         c->prof_bytes[m.kind] += m.bytes;
         c->prof_calls[m.kind] += 1;
+    }
+    for (int k = 0; k < LP_NSTAGES; k++) {
+        std::sort(spans[k].begin(), spans[k].end());
+        double end = -INFINITY;
+        for (const auto& s : spans[k]) {
+            c->prof_s[k] += std::max(0.0, s.second - std::max(s.first, end));
+            end = std::max(end, s.second);
+        }
     }
     c->marks.clear();
     c->prof_used = 0;
@@ -259,7 +283,7 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
     e = prof_begin(c, st);
     LP_CHECK(launch_tl(d, lda, static_cast<const float*>(c->dt.ptr), kb, kb, d + kb, lda, rest,
                        d + (size_t)kb * lda, lda, below, lt, std::max(4, below), c->num_sms, st));
-    return prof_end(c, st, LP_STAGE_TOP, e, trsm_flops(b, r + w), 8.0 * b * r + 12.0 * b * w);
+    return prof_end_tl(c, st, e, trsm_flops(b, r), 8.0 * b * r, trsm_flops(b, w), 12.0 * b * w);
 }
 
 // Inner block of the FP32 schedule, from the order alone whatever block the

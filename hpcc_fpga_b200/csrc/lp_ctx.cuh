@@ -7,12 +7,15 @@
 
 namespace lp {
 
-// One profiled stage launch: events e0/e1 of the context's pool bracket it.
+// One profiled stage launch: events e0/e1 of the context's pool bracket it.  A
+// launch that does the work of two stages has a mark for each, with the part
+// [f0, f1] of the time between the events.
 struct StageMark {
     int kind;
     int stream;  // 0: the context's main stream, 1: its auxiliary stream
     int e0, e1;
     double flops, bytes;
+    double f0 = 0.0, f1 = 1.0;
 };
 
 // A device allocation that only grows (freed on growth and at destroy).
@@ -143,6 +146,9 @@ constexpr int kSolveMaxRefinements = 50;
 // is off); prof_end records the closing event and the stage's work.
 int prof_begin(lp_ctx* c, cudaStream_t st);
 int prof_end(lp_ctx* c, cudaStream_t st, int kind, int e0, double flops, double bytes);
+// The same for a launch that does top and left; its time is divided as the flops are.
+int prof_end_tl(lp_ctx* c, cudaStream_t st, int e0, double top_flops, double top_bytes, double left_flops,
+                double left_bytes);
 
 }  // namespace lp
 

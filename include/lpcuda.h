@@ -112,7 +112,8 @@ int lp_host_free(void* p);
 #define LP_STAGE_OTHER 5
 #define LP_NSTAGES 6
 typedef struct {
-    double stage_s[LP_NSTAGES];      /* summed device time per stage */
+    double stage_s[LP_NSTAGES];      /* device time per stage (launches of a stage beside each other count once;
+                                        a launch of top and left is divided between them by its flops) */
     double stage_flops[LP_NSTAGES];  /* algorithmic flops of those launches */
     double stage_bytes[LP_NSTAGES];  /* algorithmic HBM bytes of those launches */
     long long stage_calls[LP_NSTAGES];

@@ -230,3 +230,27 @@ def test_factors_do_not_depend_on_free_memory(lp, dev, torch_cuda, kind, n, need
         else:
             a, b = (torch.as_tensor(x).cuda().double() for x in (got, want))
             assert float((a - b).abs().max() / b.abs().max()) < (2e-3 if kind == "bf16" else 256 * FLT_EPS)
+
+
+def test_stage_profile_of_the_fp32_schedule(ctx, dev):
+    """Every stage of the factorization is booked, with its share of the work: top and left (one launch) each b^2 r
+    flops per block step, all stages together the 2 n^3 / 3 of the factorization to its lower-order terms; a stage's
+    time is at most the span of its launches, which parts running beside each other do not add to."""
+    n = 2048
+    d = dev.put(oracle.gen_baseline(n, seed=1, margin=1.0)[0])
+    ctx.set_profiling(True)
+    try:
+        ctx.read_profile(reset=True)
+        ctx.gefa(d.data_ptr(), n, n, 128)
+        p = ctx.read_profile(reset=False)
+        events = ctx.read_timeline()
+        ctx.read_profile(reset=True)
+    finally:
+        ctx.set_profiling(False)
+    assert p["left"]["s"] > 0.0 and p["top"]["s"] > 0.0
+    assert p["left"]["flops"] == p["top"]["flops"] == sum(128.0 ** 2 * r for r in range(128, n, 128))
+    total = sum(p[s]["flops"] for s in ("lu", "top", "left", "inner"))
+    assert abs(total - 2 * n ** 3 / 3) < 0.01 * total
+    for s in ("lu", "top", "left", "inner"):
+        t = [(e[2], e[3]) for e in events if e[0] == s]
+        assert len(t) == p[s]["calls"] and 0.0 < p[s]["s"] <= (max(b for _, b in t) - min(a for a, _ in t)) * (1 + 1e-6)
