@@ -668,7 +668,7 @@ template <int NR>
 constexpr size_t sweep_smem() {
     return sizeof(float) * ((size_t)kOpFloats + (size_t)stages<NR>() * STAGE_FLOATS + 2 * (size_t)NR * SB);
 }
-// the pieces fit in the ring; the tile's sums fit in two slots beside the last source's four
+// the pieces fit in the ring; the tile's sums fit in five slots beside the last source's four
 static_assert(kScrFloats <= 9 * STAGE_FLOATS && 64 * L64 <= kMidOff, "scratch");
 static_assert(NWARP * 16 * SB <= SPT * STAGE_FLOATS && 16 * SB <= STAGE_FLOATS && stages<1>() >= 2 * SPT + 1, "ring");
 static_assert(RS % NWARP == 0 && (GT & 31) == 0, "rows per warp");

@@ -427,8 +427,11 @@ static int panel_tc(lp_ctx* c, float* dA, int n, int lda, int bs, int K, int nse
 // operands moves their factors by more than FP32 accuracy (E4M3, n = 12288:
 // 6e-5 relative to the factors' norm; BF16 2e-5 at n = 2048, 1e-5 at 4096, 5e-6 at 12288).
 // Measured on one B200, factorization alone in ms, blocks of 128 / 512 / 1024:
-//   BF16          n = 4096 2.89 / 1.95 / 1.84   n = 8192 7.55 / 4.70 / 4.35   n = 32768 217 / 66.0 / 47.8
-//   emulated FP32 n = 3072 2.35 / 1.68 / 1.51   n = 8192 8.67 / 5.91 / 5.70   n = 32768 276 / 144 / 136
+//   BF16          n = 4096 2.36 / 1.60 / 1.55   n = 8192 6.05 / 3.72 / 3.59   n = 32768 217 / 63.2 / 43.2
+//   emulated FP32 n = 3072 2.18 / 1.37 / 1.29   n = 8192 6.80 / 4.63 / 4.70   n = 32768 270 / 145 / 141
+// (Between 6144 and 16384 a block of 512 would be 1 to 5 % faster for the emulated
+// form, n = 16384 19.8 against 20.7: one line for all its orders was drawn when
+// the chain was longer.)
 constexpr int kMixedBlock = 1024;
 
 // Workspaces for blocks of up to bs; where one of them cannot be allocated, all

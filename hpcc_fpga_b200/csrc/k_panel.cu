@@ -3,8 +3,9 @@
 // beside it.  They compute the recurrences of k_lu.cu / k_trsm.cu (gefa's lu,
 // top and left, LINPACK/src/host/linpack_data.cpp:166-196) with fused
 // multiply-adds and sums in another order, so their results agree with those to
-// rounding; the stage entry points that promise the reference's exact
-// operation order keep the other kernels.
+// rounding; the entry points that promise the reference's exact operation order
+// (lp_lu_block_dev up to 128, lp_top_update_dev, lp_left_update_dev) keep the
+// other kernels.
 //
 // k_lu128 is a chain of 128 dependent pivots on one SM, so what counts is the
 // latency per pivot.  Eight worker warps hold the block in registers (8 x 8

@@ -292,11 +292,11 @@ int panel_f32(lp_ctx* c, float* dA, int n, int lda, int bs, int k0, float* lt, c
 // the chain of a step (what bounds small orders) and large blocks read and
 // write the trailing matrix less often (what bounds large ones).  Measured on
 // one B200, factorization alone in us with blocks of 128 / 256 / 512:
-//   n =  512: 139 / 146 / 129         n =  6144: 4112 / 3949 / 4260
-//   n = 1024: 290 / 319 / 342         n =  8192: 8183 / 7806 / 8019
-//   n = 2048: 618 / 696 / 788         n =  9216: 11091 / 10585 / 10767
-//   n = 3968: 1673 / 1670 / 1901      n = 12288: 24273 / 23099 / 23044
-//   n = 4096: 1747 / 1752 / 1962      n = 16384: 54642 / 51983 / 51272
+//   n =  512: 135 / 140 / 125         n =  6144: 4098 / 3959 / 4275
+//   n = 1024: 285 / 313 / 332         n =  8192: 8224 / 7834 / 8095
+//   n = 2048: 607 / 687 / 770         n =  9216: 11125 / 10626 / 10807
+//   n = 3968: 1643 / 1659 / 1886      n = 12288: 24336 / 23213 / 23225
+//   n = 4096: 1731 / 1728 / 1963      n = 16384: 54802 / 52226 / 51533
 static int f32_block(int n) { return n <= 512 ? 512 : n < 4096 ? 128 : n < 9216 ? 256 : 512; }
 
 // Workspace of the FP32 panel: the transposed lower triangle of the current block.
@@ -355,7 +355,7 @@ int f32_prepare(lp_ctx* c, int n, int user_bs, bool streamed, int* bs) {
 // U_b's CTAs fill the SMs.  With the event on the panel's side (U_a on the main
 // stream) n = 2048 took 773 us for 717, n = 4096 2245 for 2182.
 // The stages give the reference recurrences' values up to rounding; the exact
-// recurrences are lp_lu_block_dev, lp_top_update_dev, lp_left_update_dev.
+// recurrences are lp_lu_block_dev (up to 128), lp_top_update_dev, lp_left_update_dev.
 int gefa_f32(lp_ctx* c, float* dA, int n, int lda, int user_bs, cudaStream_t st) {
     int bs = 0;
     LP_CHECK(f32_prepare(c, n, user_bs, false, &bs));

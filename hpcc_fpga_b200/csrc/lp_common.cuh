@@ -126,7 +126,7 @@ int launch_trsm_left(const float* lu, int ldlu, float* l, int ldl, int bs, int n
 // FP32 SIMT trailing update C(m x n) += Lt^T (bs x m) * T (bs x n).
 int launch_sgemm_update(float* c, int ldc, const float* lt, int ldlt, const float* t, int ldt, int m, int n,
                         int k, cudaStream_t s);
-// FP64 SIMT trailing update, the same operand layout (k_dgemm.cu).
+// FP64 trailing update (warp-level FP64 MMA), the same operand layout (k_dgemm.cu).
 int launch_dgemm_update(double* c, int ldc, const double* lt, int ldlt, const double* t, int ldt, int m, int n, int k,
                         cudaStream_t s);
 int dgemm_init_attrs();

@@ -159,7 +159,7 @@ struct lp_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t aux = nullptr;               // second (high-priority) stream for concurrent panel work
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaStream_t aux2 = nullptr;              // third stream: the left update runs here beside the top update
+    cudaStream_t aux2 = nullptr;              // third: the block column's update, the tensor-core panel's operands, FP64 left
     cudaStream_t copy = nullptr;              // device-to-host copies of finished factor bands (lp_calculate)
     cudaStream_t copy_in = nullptr;           // host-to-device copies of the matrix's row slabs (lp_calculate)
     cudaStream_t lane_st = nullptr, lane_aux = nullptr;  // second lane of the row-slab schedule

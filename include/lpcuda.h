@@ -82,6 +82,8 @@ int lp_version(void);
  * (shared/include/hpcc_benchmark.hpp:560-575, shared/setup/fpga_setup.cpp)
  * with one CUDA device, stream and workspace. */
 int lp_device_count(int* count);
+/* A call that waits for the device polls (2 ms without pause, giving up its time
+ * slice, then every 50 us); the serving loop's workers block instead. */
 int lp_ctx_create(int device, lp_ctx** out);
 int lp_ctx_destroy(lp_ctx* ctx);
 /* The cudaStream_t the *_dev calls are ordered on (as void*). */
@@ -193,13 +195,23 @@ int lp_inner_update_tc_dev(lp_ctx* ctx, int precision, float* dC, int ldc, const
 /* Blocked right-looking LU without pivoting of the n x n matrix at dA, in
  * place, in the reference encoding.  Replaces the block-row loop of
  * execution::pcie::calculate (execution_types/execution_pcie.hpp:177-641).
- * n must be a multiple of bs. */
+ * n must be a multiple of bs (16..512).  The schedule's own inner block follows
+ * from n alone, so bs does not change the factors (only where device memory
+ * cannot hold that block's operands, 2 * 512 floats per row at most, bs takes
+ * its place).  Its products and sums are ordered for the GPU: the factors agree
+ * with the reference's to rounding. */
 int lp_gefa_dev(lp_ctx* ctx, float* dA, int n, int lda, int bs);
 /* The same factorization with the trailing updates in the chosen precision
  * (LP_F32: identical to lp_gefa_dev, bs 16..512; LP_BF16_IR / LP_FP8_IR /
  * LP_F32_BF16X6: tensor-core trailing updates and top/left products, bs a
- * power of two in 128..2048 — a wider block cuts the FP32 traffic of the
- * trailing updates; the factors stay FP32). */
+ * power of two in 128..2048; the factors stay FP32).  A wider block cuts the
+ * FP32 traffic of the trailing updates: LP_F32_BF16X6, and LP_BF16_IR from
+ * n = 4096 on, take at least 1024 whatever bs says (unless those operands cannot
+ * be allocated), the other forms take bs.  The context keeps the operands: for
+ * blocks of 1024 some 20 KB (LP_BF16_IR) or 72 KB (LP_F32_BF16X6) per row.  The
+ * top/left products use the explicit inverses of the diagonal block's triangles:
+ * for matrices that are not diagonally dominant their error grows with the
+ * triangles' condition. */
 int lp_gefa_prec_dev(lp_ctx* ctx, int precision, float* dA, int n, int lda, int bs);
 /* x = LU \ b followed by FP64 iterative refinement: r = b - M x with the
  * original FP32 matrix dA0 widened to FP64, d = LU \ r, x += d, until the
@@ -432,7 +444,8 @@ int lp_batch_autotune(lp_ctx* ctx, int count, const lp_system* systems, const fl
 #define LP_SERVE_PER_REQUEST 1
 typedef struct lp_server lp_server;
 typedef struct {
-    long long hbm_budget_bytes; /* device memory for resident factors + in-flight work (default 80e9) */
+    long long hbm_budget_bytes; /* device memory for resident factors + in-flight work (default 80e9); every
+                                   worker's own workspaces (see lp_gefa_prec_dev) come on top */
     int mode;                   /* LP_SERVE_CONTINUOUS or LP_SERVE_PER_REQUEST */
     int precision;              /* LP_F32, LP_BF16_IR or LP_FP8_IR */
     int slots;                  /* concurrent large-system streams (1..16; 1 in per-request mode) */
