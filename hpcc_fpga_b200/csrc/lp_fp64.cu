@@ -28,41 +28,74 @@ constexpr unsigned kSpinLimit64 = 1u << 22;
 // the unknowns lane and lane + 32 (v[q][0], v[q][1]); D: the kb x kb diagonal
 // block (FP32 factors, for the GMRES refinement, widened exactly as they are
 // read).  Forward: v_i += v_k D_ki (i > k).  Backward: s = v_k D_kk, v_i += s D_ki
-// (i < k); v_k = s.
+// (i < k); v_k = s.  Four steps at a time: one exchange brings their values to
+// every lane, which forms the four results itself (the operations of the
+// unknowns' own lanes, in the same order), so a step costs a quarter of an
+// exchange's latency (n = 6144: 0.07 ms); G = 1 is the plain step of a ragged
+// block's end.
+template <int G, int Q, typename FT>
+__device__ __forceinline__ void steps_forward(double (&v)[Q][2], const FT* D, int h, int kk, int lane) {
+    const FT* row = D + (32 * h + kk) * SB;  // row of the first step
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        double y[G];
+#pragma unroll
+        for (int j = 0; j < G; j++) y[j] = __shfl_sync(0xffffffffu, v[q][h], kk + j);
+#pragma unroll
+        for (int j = 1; j < G; j++)
+#pragma unroll
+            for (int i = 0; i < j; i++) y[j] = fma(y[i], (double)row[i * SB + 32 * h + kk + j], y[j]);
+#pragma unroll
+        for (int j = 0; j < G; j++) {
+            if (lane > kk + j) v[q][h] = fma(y[j], (double)row[j * SB + 32 * h + lane], v[q][h]);
+            if (h == 0) v[q][1] = fma(y[j], (double)row[j * SB + 32 + lane], v[q][1]);
+        }
+    }
+}
+template <int G, int Q, typename FT>
+__device__ __forceinline__ void steps_backward(double (&v)[Q][2], const FT* D, int h, int kk, int lane) {
+    const FT* row = D + (32 * h + kk) * SB;  // row of the last step (the lowest unknown)
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+        double s[G];
+#pragma unroll
+        for (int j = 0; j < G; j++) s[j] = __shfl_sync(0xffffffffu, v[q][h], kk + j);
+#pragma unroll
+        for (int j = G - 1; j >= 0; j--) {
+#pragma unroll
+            for (int i = G - 1; i > j; i--) s[j] = fma(s[i], (double)row[i * SB + 32 * h + kk + j], s[j]);
+            s[j] *= (double)row[j * SB + 32 * h + kk + j];
+        }
+#pragma unroll
+        for (int j = G - 1; j >= 0; j--) {
+            if (lane < kk + j)
+                v[q][h] = fma(s[j], (double)row[j * SB + 32 * h + lane], v[q][h]);
+            else if (lane == kk + j)
+                v[q][h] = s[j];
+            if (h == 1) v[q][0] = fma(s[j], (double)row[j * SB + lane], v[q][0]);
+        }
+    }
+}
 template <int Q, typename FT>
 __device__ __forceinline__ void block_forward(double (&v)[Q][2], const FT* D, int kb, int lane) {
 #pragma unroll
-    for (int h = 0; h < 2; h++)
-#pragma unroll 8
-        for (int kk = 0; kk < min(32, kb - 32 * h); kk++) {
-            const FT* row = D + (32 * h + kk) * SB + lane;
-            const double d0 = (double)row[0], d1 = (double)row[32];
-#pragma unroll
-            for (int q = 0; q < Q; q++) {
-                const double y = __shfl_sync(0xffffffffu, v[q][h], kk);
-                if (lane > kk) v[q][h] = fma(y, h == 0 ? d0 : d1, v[q][h]);
-                if (h == 0) v[q][1] = fma(y, d1, v[q][1]);
-            }
-        }
+    for (int h = 0; h < 2; h++) {
+        const int m = min(32, kb - 32 * h);
+        int kk = 0;
+#pragma unroll 2
+        for (; kk + 4 <= m; kk += 4) steps_forward<4>(v, D, h, kk, lane);
+        for (; kk < m; kk++) steps_forward<1>(v, D, h, kk, lane);
+    }
 }
 template <int Q, typename FT>
 __device__ __forceinline__ void block_backward(double (&v)[Q][2], const FT* D, int kb, int lane) {
 #pragma unroll
-    for (int h = 1; h >= 0; h--)
-#pragma unroll 8
-        for (int kk = min(32, kb - 32 * h) - 1; kk >= 0; kk--) {
-            const FT* row = D + (32 * h + kk) * SB;
-            const double d = (double)row[32 * h + kk], d0 = (double)row[lane], d1 = (double)row[lane + 32];
-#pragma unroll
-            for (int q = 0; q < Q; q++) {
-                const double s = __shfl_sync(0xffffffffu, v[q][h], kk) * d;
-                if (lane < kk)
-                    v[q][h] = fma(s, h == 0 ? d0 : d1, v[q][h]);
-                else if (lane == kk)
-                    v[q][h] = s;
-                if (h == 1) v[q][0] = fma(s, d0, v[q][0]);
-            }
-        }
+    for (int h = 1; h >= 0; h--) {
+        int kk = min(32, kb - 32 * h);
+        while (kk > 0 && (kk & 3) != 0) steps_backward<1>(v, D, h, --kk, lane);
+#pragma unroll 2
+        for (kk -= 4; kk >= 0; kk -= 4) steps_backward<4>(v, D, h, kk, lane);
+    }
 }
 
 // Bounded grid barrier of a cooperative launch; the counter only grows.
@@ -99,8 +132,8 @@ __device__ __forceinline__ bool grid_sync64(unsigned* bar, unsigned target, unsi
 // it with rows loaded before the barrier; one barrier per block.  w1, w2: n x
 // nrhs accumulating values of the two sweeps (the forward sweep's results are
 // the second's input).  A chain of 2 n / 64 short steps, where one launch per block and direction took
-// 15 us each (n = 6144: 192 launches, 2.9 ms; now 1.1).  Products with the blocks'
-// inverses in place of the recurrences took 0.27 ms less, but lost what the
+// 15 us each (n = 6144: 192 launches, 2.9 ms; now 1.0).  Products with the blocks'
+// inverses in place of the recurrences took 0.20 ms less, but lost what the
 // condition of a block's triangles allows.  A barrier that gives up leaves
 // NaN in the solutions and sets *gave_up, a word in page-locked host memory.
 // stall (tests): CTA 0 never arrives at the first barrier.
